@@ -9,9 +9,9 @@
 //    near-singular rule of boundaryelementsolver.cpp:1387-1514. FP64: the
 //    labels must resolve 1e-7.
 //  * mlp_*: FP32 training of the 24-64-64-5 ReLU network (forward + softmax
-//    cross-entropy + backward per sample, parameter gradients one thread per
-//    parameter with the samples summed in order, so the result is bitwise
-//    reproducible; Adam).
+//    cross-entropy + backward and the parameter gradient per tile of samples
+//    in one CTA's shared memory, partial gradients summed in a fixed order, so
+//    the result is bitwise reproducible; Adam).
 //  * sel_infer / sel_near_classes: BF16 inference on the tensor cores, one warp
 //    per 32 pairs (two m16 row tiles sharing the weight fragments), mma.sync
 //    m16n8k16 with FP32 accumulation; low-confidence pairs get the highest
@@ -21,6 +21,7 @@
 //    highest order and keeps that value when the two disagree.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -376,105 +377,238 @@ __global__ void __launch_bounds__(128) sel_label_kernel(const Elem* __restrict__
 // ---------------- FP32 training ----------------
 constexpr int TB = 128;
 
-// forward, softmax cross-entropy and the per-sample deltas
-__global__ void __launch_bounds__(TB) mlp_fwd_bwd_kernel(const float* __restrict__ prm,
-                                                         const float* __restrict__ X,
-                                                         const uint8_t* __restrict__ y, int64_t B,
-                                                         float* __restrict__ work) {
-  __shared__ float W[SEL_NPARAM];
-  for (int i = threadIdx.x; i < SEL_NPARAM; i += TB) W[i] = prm[i];
-  __syncthreads();
-  const int64_t s = (int64_t)blockIdx.x * TB + threadIdx.x;
-  if (s >= B) return;
-  float* H1 = work;
-  float* H2 = H1 + B * SEL_H;
-  float* D1 = H2 + B * SEL_H;
-  float* D2 = D1 + B * SEL_H;
-  float* D3 = D2 + B * SEL_H;
-  float* LS = D3 + B * 8;
-  float x[SEL_NF], h1[SEL_H], h2[SEL_H], z[SEL_C];
-  for (int i = 0; i < SEL_NF; i++) x[i] = X[s * SEL_NF + i];
-  for (int j = 0; j < SEL_H; j++) {
-    float a = W[SEL_OB1 + j];
-    for (int i = 0; i < SEL_NF; i++) a += x[i] * W[SEL_OW1 + i * SEL_H + j];
-    h1[j] = fmaxf(a, 0.0f);
+// Training step. One CTA runs forward, softmax cross-entropy and backward for
+// tiles of TS samples entirely in shared memory and keeps its share of the
+// parameter gradient in registers over its tiles, so no activation goes to
+// memory: what leaves is one partial gradient per CTA (plus its loss), which
+// the second kernel adds in a fixed order (bitwise reproducible).
+// Bound: issue of the FP32 products and their shared-memory operands. Every
+// thread owns register tiles (1 hidden unit x 8 samples forward and backward,
+// 4 x 4 of dW2, 2 x 4 of dW1), so a product costs about half a load; the
+// samples of a group of 64 threads are read as broadcasts, W2 rows are padded
+// to 65 words for the transposed read of the backward pass. At B = 4,096 a
+// step with Adam takes 25.6 us; with per-sample activations in memory and one
+// thread per parameter summing over all samples it took 381 us.
+constexpr int TT = 256;      // threads of a training CTA
+constexpr int TS = 32;       // samples per tile
+constexpr int TLD = SEL_H + 4;   // row stride of the hidden tiles (16-byte rows)
+constexpr int TW2 = SEL_H + 1;   // row stride of W2
+constexpr int TRAIN_MAX_CTAS = 304;  // partial gradients of one step: two per SM
+
+struct TrainSmem {
+  float x[TS * SEL_NF];
+  float a[TS * TLD];  // h1, then its deltas
+  float b[TS * TLD];  // h2, then its deltas
+  float d3[TS * 8];
+  float w1[SEL_NF * SEL_H];
+  float w2[SEL_H * TW2];
+  float w3[SEL_H * SEL_C];
+  float b1[SEL_H], b2[SEL_H], b3[8];
+  float ls[TS];
+};
+
+// out[s][j] = relu(b[j] + sum_i in[s][i] w[i * ldw + j]) for the thread's unit
+// j and 8 samples s0 .. s0 + 7
+template <int K, int LDI, int LDW>
+__device__ __forceinline__ void train_layer(const float* in, const float* w, float bias, int j,
+                                            int s0, float* out) {
+  float acc[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) acc[q] = bias;
+#pragma unroll 4
+  for (int i = 0; i < K; i += 4) {
+    const float w0 = w[i * LDW + j], w1 = w[(i + 1) * LDW + j], w2 = w[(i + 2) * LDW + j],
+                w3 = w[(i + 3) * LDW + j];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const float4 v = *reinterpret_cast<const float4*>(in + (s0 + q) * LDI + i);
+      acc[q] = fmaf(v.x, w0, acc[q]);
+      acc[q] = fmaf(v.y, w1, acc[q]);
+      acc[q] = fmaf(v.z, w2, acc[q]);
+      acc[q] = fmaf(v.w, w3, acc[q]);
+    }
   }
-  for (int j = 0; j < SEL_H; j++) {
-    float a = W[SEL_OB2 + j];
-    for (int i = 0; i < SEL_H; i++) a += h1[i] * W[SEL_OW2 + i * SEL_H + j];
-    h2[j] = fmaxf(a, 0.0f);
+#pragma unroll
+  for (int q = 0; q < 8; q++) out[(s0 + q) * TLD + j] = fmaxf(acc[q], 0.0f);
+}
+
+// part + blockIdx.x * stride: the CTA's gradient sums, then its loss sum
+// (scaled by 1 / B when it is the only CTA: part is then the gradient itself)
+__global__ void __launch_bounds__(TT) mlp_train_kernel(const float* __restrict__ prm,
+                                                       const float* __restrict__ X,
+                                                       const uint8_t* __restrict__ y, int64_t B,
+                                                       float* __restrict__ part,
+                                                       float* __restrict__ loss, int64_t stride) {
+  __shared__ __align__(16) TrainSmem S;
+  const int t = threadIdx.x;
+  for (int i = t; i < SEL_NF * SEL_H; i += TT) S.w1[i] = prm[SEL_OW1 + i];
+  for (int i = t; i < SEL_H * SEL_H; i += TT)
+    S.w2[(i >> 6) * TW2 + (i & 63)] = prm[SEL_OW2 + i];
+  for (int i = t; i < SEL_H * SEL_C; i += TT) S.w3[i] = prm[SEL_OW3 + i];
+  if (t < SEL_H) {
+    S.b1[t] = prm[SEL_OB1 + t];
+    S.b2[t] = prm[SEL_OB2 + t];
   }
-  float zm = -1e30f;
-  for (int j = 0; j < SEL_C; j++) {
-    float a = W[SEL_OB3 + j];
-    for (int i = 0; i < SEL_H; i++) a += h2[i] * W[SEL_OW3 + i * SEL_C + j];
-    z[j] = a;
-    zm = fmaxf(zm, a);
-  }
-  float se = 0;
-  for (int j = 0; j < SEL_C; j++) se += expf(z[j] - zm);
-  const int lab = y[s];
-  LS[s] = -(z[lab] - zm - logf(se));
-  float d3[SEL_C];
+  if (t < SEL_C) S.b3[t] = prm[SEL_OB3 + t];
   const float inv_b = 1.0f / (float)B;
-  for (int j = 0; j < SEL_C; j++) {
-    d3[j] = (expf(z[j] - zm) / se - (j == lab ? 1.0f : 0.0f)) * inv_b;
-    D3[s * 8 + j] = d3[j];
+  const int j = t & 63, s0 = (t >> 6) * 8;       // forward / backward tile
+  const int gi = (t >> 4) * 4, gj = (t & 15) * 4;  // dW2 tile
+  const int fi = (t >> 4) * 2;                   // dW1 tile (threads below 192)
+  float g2[4][4] = {}, g1[2][4] = {}, g3[2] = {}, gb1 = 0, gb2 = 0, gb3 = 0, lsum = 0;
+  const int64_t tiles = (B + TS - 1) / TS;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t base = tile * TS;
+    const int ns = (int)min((int64_t)TS, B - base);
+    __syncthreads();
+    for (int i = t; i < TS * SEL_NF; i += TT)
+      S.x[i] = i < ns * SEL_NF ? X[base * SEL_NF + i] : 0.0f;
+    __syncthreads();
+    train_layer<SEL_NF, SEL_NF, SEL_H>(S.x, S.w1, S.b1[j], j, s0, S.a);
+    __syncthreads();
+    train_layer<SEL_H, TLD, TW2>(S.a, S.w2, S.b2[j], j, s0, S.b);
+    __syncthreads();
+    {  // logits, loss and d3: 8 lanes per sample
+      const int s = t >> 3, c = t & 7;
+      float z = -1e30f;
+      if (c < SEL_C) {
+        z = S.b3[c];
+        for (int i = 0; i < SEL_H; i++) z = fmaf(S.b[s * TLD + i], S.w3[i * SEL_C + c], z);
+      }
+      float zm = z;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) zm = fmaxf(zm, __shfl_xor_sync(0xffffffffu, zm, o));
+      const float e = c < SEL_C ? expf(z - zm) : 0.0f;
+      float se = e;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+      const bool on = s < ns;
+      const int lab = on ? y[base + s] : -1;
+      S.d3[s * 8 + c] = on && c < SEL_C ? (e / se - (c == lab ? 1.0f : 0.0f)) * inv_b : 0.0f;
+      float zl = c == lab ? z : 0.0f;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) zl += __shfl_xor_sync(0xffffffffu, zl, o);
+      if (c == 0) S.ls[s] = on ? -(zl - zm - logf(se)) : 0.0f;
+    }
+    __syncthreads();
+    // dW3 and db3 from h2; the loss
+    if (t < SEL_C) {
+      for (int s = 0; s < TS; s++) gb3 += S.d3[s * 8 + t];
+    } else if (t == 32) {
+      for (int s = 0; s < TS; s++) lsum += S.ls[s];
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int p = t + q * TT;
+      if (p < SEL_H * SEL_C) {
+        const int i = p / SEL_C, c = p - i * SEL_C;
+        for (int s = 0; s < TS; s++) g3[q] = fmaf(S.b[s * TLD + i], S.d3[s * 8 + c], g3[q]);
+      }
+    }
+    __syncthreads();
+    // d2 in place of h2
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      float v = 0;
+#pragma unroll
+      for (int c = 0; c < SEL_C; c++) v = fmaf(S.w3[j * SEL_C + c], S.d3[(s0 + q) * 8 + c], v);
+      float& h = S.b[(s0 + q) * TLD + j];
+      h = h > 0.0f ? v : 0.0f;
+    }
+    __syncthreads();
+    // dW2 and db2 from h1 and d2
+    for (int s = 0; s < TS; s++) {
+      const float4 u = *reinterpret_cast<const float4*>(S.a + s * TLD + gi);
+      const float4 v = *reinterpret_cast<const float4*>(S.b + s * TLD + gj);
+      const float uu[4] = {u.x, u.y, u.z, u.w}, vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int p = 0; p < 4; p++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) g2[p][q] = fmaf(uu[p], vv[q], g2[p][q]);
+    }
+    if (t < SEL_H)
+      for (int s = 0; s < TS; s++) gb2 += S.b[s * TLD + t];
+    // d1: sums over the row of W2 of unit j, kept until every h1 has been read
+    float d[8] = {};
+#pragma unroll 4
+    for (int i = 0; i < SEL_H; i += 4) {
+      const float w0 = S.w2[j * TW2 + i], w1 = S.w2[j * TW2 + i + 1], w2 = S.w2[j * TW2 + i + 2],
+                  w3 = S.w2[j * TW2 + i + 3];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const float4 v = *reinterpret_cast<const float4*>(S.b + (s0 + q) * TLD + i);
+        d[q] = fmaf(v.x, w0, d[q]);
+        d[q] = fmaf(v.y, w1, d[q]);
+        d[q] = fmaf(v.z, w2, d[q]);
+        d[q] = fmaf(v.w, w3, d[q]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      float& h = S.a[(s0 + q) * TLD + j];
+      h = h > 0.0f ? d[q] : 0.0f;
+    }
+    __syncthreads();
+    if (t < 192) {
+      for (int s = 0; s < TS; s++) {
+        const float2 u = *reinterpret_cast<const float2*>(S.x + s * SEL_NF + fi);
+        const float4 v = *reinterpret_cast<const float4*>(S.a + s * TLD + gj);
+        const float vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          g1[0][q] = fmaf(u.x, vv[q], g1[0][q]);
+          g1[1][q] = fmaf(u.y, vv[q], g1[1][q]);
+        }
+      }
+    } else {
+      for (int s = 0; s < TS; s++) gb1 += S.a[s * TLD + (t - 192)];
+    }
   }
-  float d2[SEL_H];
-  for (int i = 0; i < SEL_H; i++) {
-    float a = 0;
-    for (int j = 0; j < SEL_C; j++) a += W[SEL_OW3 + i * SEL_C + j] * d3[j];
-    d2[i] = h2[i] > 0.0f ? a : 0.0f;
-    D2[s * SEL_H + i] = d2[i];
-    H2[s * SEL_H + i] = h2[i];
+  float* g = part + blockIdx.x * stride;
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) g[SEL_OW2 + (gi + p) * SEL_H + gj + q] = g2[p][q];
+  if (t < 192) {
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) g[SEL_OW1 + (fi + p) * SEL_H + gj + q] = g1[p][q];
+  } else {
+    g[SEL_OB1 + t - 192] = gb1;
   }
-  for (int i = 0; i < SEL_H; i++) {
-    float a = 0;
-    for (int j = 0; j < SEL_H; j++) a += W[SEL_OW2 + i * SEL_H + j] * d2[j];
-    D1[s * SEL_H + i] = h1[i] > 0.0f ? a : 0.0f;
-    H1[s * SEL_H + i] = h1[i];
+  if (t < SEL_H) g[SEL_OB2 + t] = gb2;
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+    if (t + q * TT < SEL_H * SEL_C) g[SEL_OW3 + t + q * TT] = g3[q];
+  if (t < SEL_C) g[SEL_OB3 + t] = gb3;
+  if (t == 32) {
+    if (gridDim.x == 1) *loss = lsum * inv_b;
+    else g[SEL_NPARAM] = lsum;
   }
 }
 
-// one thread per parameter (+1 for the mean loss); samples summed in order
-__global__ void mlp_param_grad_kernel(const float* __restrict__ X, int64_t B,
-                                      const float* __restrict__ work, float* __restrict__ grad,
-                                      float* __restrict__ loss) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p > SEL_NPARAM) return;
-  const float* H1 = work;
-  const float* H2 = H1 + B * SEL_H;
-  const float* D1 = H2 + B * SEL_H;
-  const float* D2 = D1 + B * SEL_H;
-  const float* D3 = D2 + B * SEL_H;
-  const float* LS = D3 + B * 8;
+// Sum of the nct partial gradients: 8 threads per parameter, each its
+// interleaved share in order, then their sums in order.
+__global__ void __launch_bounds__(256) mlp_grad_sum_kernel(const float* __restrict__ part, int nct,
+                                                           int64_t stride, float inv_b,
+                                                           float* __restrict__ grad,
+                                                           float* __restrict__ loss) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int p = blockIdx.x * 32 + lane;
   float a = 0;
-  if (p == SEL_NPARAM) {
-    for (int64_t s = 0; s < B; s++) a += LS[s];
-    *loss = a / (float)B;
-    return;
+  if (p <= SEL_NPARAM) {
+#pragma unroll 8
+    for (int c = w; c < nct; c += 8) a += part[c * stride + p];
   }
-  if (p < SEL_OB1) {
-    const int i = p / SEL_H, j = p % SEL_H;
-    for (int64_t s = 0; s < B; s++) a += X[s * SEL_NF + i] * D1[s * SEL_H + j];
-  } else if (p < SEL_OW2) {
-    const int j = p - SEL_OB1;
-    for (int64_t s = 0; s < B; s++) a += D1[s * SEL_H + j];
-  } else if (p < SEL_OB2) {
-    const int i = (p - SEL_OW2) / SEL_H, j = (p - SEL_OW2) % SEL_H;
-    for (int64_t s = 0; s < B; s++) a += H1[s * SEL_H + i] * D2[s * SEL_H + j];
-  } else if (p < SEL_OW3) {
-    const int j = p - SEL_OB2;
-    for (int64_t s = 0; s < B; s++) a += D2[s * SEL_H + j];
-  } else if (p < SEL_OB3) {
-    const int i = (p - SEL_OW3) / SEL_C, j = (p - SEL_OW3) % SEL_C;
-    for (int64_t s = 0; s < B; s++) a += H2[s * SEL_H + i] * D3[s * 8 + j];
-  } else {
-    const int j = p - SEL_OB3;
-    for (int64_t s = 0; s < B; s++) a += D3[s * 8 + j];
-  }
-  grad[p] = a;
+  red[w][lane] = a;
+  __syncthreads();
+  if (w != 0 || p > SEL_NPARAM) return;
+#pragma unroll
+  for (int q = 1; q < 8; q++) a += red[q][lane];
+  if (p < SEL_NPARAM) grad[p] = a;
+  else *loss = a * inv_b;
 }
 
 __global__ void mlp_adam_kernel(float* __restrict__ prm, const float* __restrict__ g,
@@ -873,8 +1007,22 @@ void launch_sel_label(const Elem* P, const Elem* Q, const double* k, int64_t n, 
 void launch_mlp_grad(const float* params, const float* X, const uint8_t* y, int64_t B,
                      float* grad, float* loss, float* work, cudaStream_t s) {
   if (B <= 0) return;
-  mlp_fwd_bwd_kernel<<<(unsigned)((B + TB - 1) / TB), TB, 0, s>>>(params, X, y, B, work);
-  mlp_param_grad_kernel<<<(SEL_NPARAM + 1 + 127) / 128, 128, 0, s>>>(X, B, work, grad, loss);
+  // CTAs: as many as tiles, two per SM at most, and as many partial gradients
+  // as the work area of B samples holds (B = 4,096: 128 CTAs of one tile);
+  // below two partials a single CTA writes the gradient itself. A tile count
+  // just above the limit would leave a few CTAs with one tile more than the
+  // rest, so the tiles are dealt evenly.
+  const int64_t stride = SEL_NPARAM + 1;
+  const int64_t tiles = (B + TS - 1) / TS;
+  const int64_t room = B * SEL_WORK_PER_SAMPLE / stride;
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>({tiles, room, TRAIN_MAX_CTAS}));
+  const int64_t per = (tiles + most - 1) / most;
+  const int64_t ncta = (tiles + per - 1) / per;
+  mlp_train_kernel<<<(unsigned)ncta, TT, 0, s>>>(params, X, y, B, ncta > 1 ? work : grad, loss,
+                                                 stride);
+  if (ncta > 1)
+    mlp_grad_sum_kernel<<<(unsigned)((stride + 31) / 32), 256, 0, s>>>(
+        work, (int)ncta, stride, 1.0f / (float)B, grad, loss);
 }
 
 void launch_mlp_adam(float* params, const float* grad, float* m, float* v, int64_t step,

@@ -43,7 +43,7 @@ struct SelBlob {
   float mu[SEL_NF], inv_sigma[SEL_NF];
 };
 
-// FP32 training work area per sample: H1, H2, D1, D2 (64 each), P/D3 (8), loss (1)
+// FP32 training work area per sample (the partial gradients of the step's CTAs)
 constexpr int SEL_WORK_PER_SAMPLE = 4 * SEL_H + 8 + 1;
 
 // Host-built rule tables (classes 0-4, plain 16-point, 64-point reference).
@@ -61,8 +61,8 @@ void launch_sel_label(const Elem* P, const Elem* Q, const double* k, int64_t n, 
                       float* err, cudaStream_t s);
 
 // FP32 training: forward + softmax cross-entropy, backward, parameter
-// gradients (deterministic: one thread per parameter, samples in order) and
-// the mean loss. work: B * SEL_WORK_PER_SAMPLE floats.
+// gradients (deterministic: per-CTA partials summed in a fixed order) and the
+// mean loss. work: B * SEL_WORK_PER_SAMPLE floats.
 void launch_mlp_grad(const float* params, const float* X, const uint8_t* y, int64_t B,
                      float* grad, float* loss, float* work, cudaStream_t s);
 void launch_mlp_adam(float* params, const float* grad, float* m, float* v, int64_t step,
