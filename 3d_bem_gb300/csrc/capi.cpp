@@ -248,10 +248,10 @@ struct bem_handle {
   std::vector<Elem> Er;
   DBuf<Elem> dEr;
   DBuf<ElemF> dEFr;
-  DBuf<FieldElemF> dFeR;
+  DBuf<unsigned char> dFeR;
   // field evaluation (bem_field): element records, coefficients, partial
   // sums, copies of the caller's points / boundary data / sources
-  DBuf<FieldElemF> dFe;
+  DBuf<unsigned char> dFe;
   DBuf<unsigned char> dFcoef;
   DBuf<double2> dFpart, dFphi, dFdphi, dFout1, dFout2;
   DBuf<double> dFpts, dFsrc;
@@ -2789,13 +2789,19 @@ namespace {
 
 // ---- field evaluation ----
 
-// Element chunks of the field sum: enough CTAs for about eight per SM, chunks
-// of at least 512 elements.
-int field_split(const bem_handle* h, int64_t M) {
-  const int64_t bx = (M + FIELD_PTS - 1) / FIELD_PTS;
-  const int64_t want = (8LL * h->nsm + bx - 1) / bx;
-  const int64_t most = std::max<int64_t>(1, h->N / 512);
-  return (int)std::max<int64_t>(1, std::min<int64_t>({want, most, 256}));
+// Element chunks of the field sum: CTAs for 2,048 points per SM (about eight
+// CTAs of 256), in chunks of at least 16 elements -- few points need many
+// chunks: 997 points x 5,123 elements in chunks of 512 elements kept 40 of the
+// 152 SMs busy (FP64 19.0 ms) -- and at most 32 MiB of partial sums beyond what
+// chunks of 512 elements need.
+int field_split(const bem_handle* h, int64_t M, int64_t R) {
+  const int64_t pts = field_points(M);
+  const int64_t bx = (M + pts - 1) / pts;
+  const int64_t want = (2048LL / pts * h->nsm + bx - 1) / bx;
+  const int64_t coarse = std::max<int64_t>(1, h->N / 512);
+  const int64_t room = std::max<int64_t>(coarse, (32LL << 20) / (int64_t)sizeof(double2) / (M * R));
+  const int64_t most = std::min(std::max<int64_t>(1, h->N / 16), room);
+  return (int)std::max<int64_t>(1, std::min<int64_t>({want, most, 1024}));
 }
 
 // calculateFieldSolution (boundaryelementsolver.cpp:2192-2249) on device
@@ -2822,24 +2828,23 @@ void field_dev(bem_handle* h, double freq, const double* pts, int64_t M, const d
     h->field_src.assign(src, src + 5 * nsrc);
     h->dFsrc.upload(h->field_src, s);
   }
-  if (prec == 1) h->dFe.ensure((size_t)N);
+  const size_t fes = prec == 1 ? sizeof(FieldElemF) : sizeof(FieldElem);
+  h->dFe.ensure((size_t)N * fes);
   h->dFcoef.ensure((size_t)N * R * (prec == 1 ? sizeof(FieldCoefF) : sizeof(FieldCoef)));
-  const int S = field_split(h, M);
+  const int S = field_split(h, M, R);
   // with an impedance plane the reflected elements add a second set of S
   // partial sums with the same coefficients (:2305-2311)
   const int passes = h->have_plane ? 2 : 1;
   h->dFpart.ensure((size_t)passes * S * R * M);
   h->launches += launch_field_prep(h->dE.p, h->dPerm.p, N, phi, dphi, (int)R, prec, h->dFe.p,
                                    h->dFcoef.p, s);
-  h->launches += launch_field_sum(h->dE.p, h->dFe.p, h->dFcoef.p, N, (int)R, pts, M, k, prec, S,
+  h->launches += launch_field_sum(h->dFe.p, h->dFcoef.p, N, (int)R, pts, M, k, prec, S,
                                   h->dFpart.p, s);
   if (h->have_plane) {
-    if (prec == 1) {
-      h->dFeR.ensure((size_t)N);
-      h->launches += launch_field_prep(h->dEr.p, nullptr, N, nullptr, nullptr, 0, prec,
-                                       h->dFeR.p, nullptr, s);
-    }
-    h->launches += launch_field_sum(h->dEr.p, h->dFeR.p, h->dFcoef.p, N, (int)R, pts, M, k, prec,
+    h->dFeR.ensure((size_t)N * fes);
+    h->launches += launch_field_prep(h->dEr.p, nullptr, N, nullptr, nullptr, 0, prec, h->dFeR.p,
+                                     nullptr, s);
+    h->launches += launch_field_sum(h->dFeR.p, h->dFcoef.p, N, (int)R, pts, M, k, prec,
                                     S, h->dFpart.p + (size_t)S * R * M, s);
   }
   h->launches += launch_field_finish(h->dFpart.p, passes * S, M, (int)R, pts,

@@ -52,7 +52,7 @@ __constant__ float cR7gf[7] = {
 __global__ void field_prep_kernel(const Elem* __restrict__ E, const int64_t* __restrict__ perm,
                                   int64_t N, const double2* __restrict__ phi,
                                   const double2* __restrict__ dphi, int R, int precision,
-                                  FieldElemF* __restrict__ fe, void* __restrict__ coef) {
+                                  void* __restrict__ fe, void* __restrict__ coef) {
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= N) return;
   const Elem& e = E[j];
@@ -78,7 +78,29 @@ __global__ void field_prep_kernel(const Elem* __restrict__ E, const int64_t* __r
       f.qn[i] = (float)on;
     }
     f.pad[0] = f.pad[1] = f.pad[2] = 0.0f;
-    fe[j] = f;
+    static_cast<FieldElemF*>(fe)[j] = f;
+  } else {
+    FieldElem f;
+    double rho = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      f.c[d] = e.c[d];
+      f.nrm[d] = e.nrm[d];
+    }
+#pragma unroll
+    for (int i = 0; i < 7; i++) {
+      const double a1 = cR7x1[i], a2 = cR7x2[i], a3 = 1.0 - a2 - a1;
+      double o2 = 0.0;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const double q = (a1 * e.n1[d] + a2 * e.n2[d]) + a3 * e.n3[d];
+        f.q[3 * i + d] = q;
+        o2 += (q - e.c[d]) * (q - e.c[d]);
+      }
+      rho = fmax(rho, o2);
+    }
+    f.rho = sqrt(rho);
+    static_cast<FieldElem*>(fe)[j] = f;
   }
   if (R == 0) return;  // element records only (the reflected elements)
   const int64_t cj = perm[j];
@@ -100,11 +122,12 @@ __global__ void field_prep_kernel(const Elem* __restrict__ E, const int64_t* __r
 }
 
 // Columns r0 .. r0 + RB - 1, element chunk blockIdx.y.
-template <int RB>
+template <int RB, int FIELD_PTS>
 __global__ void __launch_bounds__(FIELD_PTS)
     field_sum32_kernel(const FieldElemF* __restrict__ fe, const FieldCoefF* __restrict__ coef,
                        int64_t N, int64_t chunk, const double* __restrict__ pts, int64_t M,
                        float k, float kc, int r0, int R, double2* __restrict__ partial) {
+  constexpr int FIELD_TILE = FIELD_PTS / 2;
   __shared__ FieldElemF se[FIELD_TILE];
   __shared__ FieldCoefF sc[RB][FIELD_TILE];
   const int64_t ip = (int64_t)blockIdx.x * FIELD_PTS + threadIdx.x;
@@ -185,12 +208,81 @@ __global__ void __launch_bounds__(FIELD_PTS)
   }
 }
 
-template <int RB>
+// sin and cos of x, |x| <= X, by their Taylor series to x^(2 NS + 1) and
+// x^(2 NC): for X = 0.35 (6, 6) the first terms left out are below 3e-19 and
+// 5e-18 of the functions, for X = 1 (8, 9) below 9e-18 and 5e-19.
+template <int NS, int NC>
+__device__ __forceinline__ void sincos_taylor(double x, double& sn, double& cs) {
+  constexpr double is[9] = {1.0,
+                            -1.0 / 6,
+                            1.0 / 120,
+                            -1.0 / 5040,
+                            1.0 / 362880,
+                            -1.0 / 39916800,
+                            1.0 / 6227020800.0,
+                            -1.0 / 1307674368000.0,
+                            1.0 / 355687428096000.0};
+  constexpr double ic[10] = {1.0,
+                             -1.0 / 2,
+                             1.0 / 24,
+                             -1.0 / 720,
+                             1.0 / 40320,
+                             -1.0 / 3628800,
+                             1.0 / 479001600.0,
+                             -1.0 / 87178291200.0,
+                             1.0 / 20922789888000.0,
+                             -1.0 / 6402373705728000.0};
+  const double t = x * x;
+  double ps = is[NS], pc = ic[NC];
+#pragma unroll
+  for (int q = NS - 1; q >= 1; q--) ps = fma(ps, t, is[q]);
+#pragma unroll
+  for (int q = NC - 1; q >= 0; q--) pc = fma(pc, t, ic[q]);
+  sn = fma(x * t, ps, x);
+  cs = pc;
+}
+
+// Sums over the 7 rule points of w G / (4 pi r) and of its radial part
+// w (1 - ikr) G / (4 pi r^3), both times exp(-ik r_c) unless FULL (NS, NC:
+// terms of the series of the phase differences k (r - r_c)).
+template <bool FULL, int NS, int NC>
+__device__ __forceinline__ void field_points64(const FieldElem& e, double px, double py, double pz,
+                                               double k, double krc, double& Lx, double& Ly,
+                                               double& Mx, double& My) {
+  for (int i = 0; i < 7; i++) {
+    const double rx = px - e.q[3 * i], ry = py - e.q[3 * i + 1], rz = pz - e.q[3 * i + 2];
+    const double rr = fma(rx, rx, fma(ry, ry, rz * rz));
+    const double ir = rsqrt(rr);
+    double r = rr * ir;
+    r = fma(0.5 * ir, fma(-r, r, rr), r);  // one correction: r to half an ulp
+    double sn, cs;
+    if constexpr (FULL) sincos(k * r, &sn, &cs);
+    else sincos_taylor<NS, NC>(fma(k, r, -krc), sn, cs);
+    const double g0 = ir * cR7g[i];
+    Lx = fma(g0, cs, Lx);
+    Ly = fma(g0, sn, Ly);
+    const double h = g0 * (ir * ir), kr = k * r;
+    Mx = fma(h, fma(kr, sn, cs), Mx);
+    My = fma(h, fma(-kr, cs, sn), My);
+  }
+}
+
+// FP64: bound by the FP64 pipe (2 FMA per clock and SM on this GPU), so the
+// kernel is laid out for few FP64 instructions per rule point (about 55; a
+// sincos, a square root and a division each took ~80 with the rule points
+// recomputed): rule points come ready from the element records, 1 / r from one
+// rsqrt, (p - q) . n is the same for all points of the plane, and exp(ikr) =
+// exp(ik r_c) exp(ik (r - r_c)) takes one sincos per element at its centroid
+// and a short Taylor series per point (|k (r - r_c)| <= k rho; elements with
+// k rho > 1 take the full sincos). 5,123 elements x 997 points, 3 columns:
+// 3.70 ms; 18.99 ms before, with 40 CTAs on 152 SMs (see field_split).
+template <int RB, int FIELD_PTS>
 __global__ void __launch_bounds__(FIELD_PTS)
-    field_sum64_kernel(const Elem* __restrict__ E, const FieldCoef* __restrict__ coef, int64_t N,
-                       int64_t chunk, const double* __restrict__ pts, int64_t M, double k,
-                       int r0, int R, double2* __restrict__ partial) {
-  __shared__ Elem se[FIELD_TILE];
+    field_sum64_kernel(const FieldElem* __restrict__ fe, const FieldCoef* __restrict__ coef,
+                       int64_t N, int64_t chunk, const double* __restrict__ pts, int64_t M,
+                       double k, int r0, int R, double2* __restrict__ partial) {
+  constexpr int FIELD_TILE = FIELD_PTS / 4;
+  __shared__ FieldElem se[FIELD_TILE];
   __shared__ FieldCoef sc[RB][FIELD_TILE];
   const int64_t ip = (int64_t)blockIdx.x * FIELD_PTS + threadIdx.x;
   const int64_t e0 = (int64_t)blockIdx.y * chunk;
@@ -206,35 +298,38 @@ __global__ void __launch_bounds__(FIELD_PTS)
   for (int64_t t0 = e0; t0 < e1; t0 += FIELD_TILE) {
     const int nt = (int)min((int64_t)FIELD_TILE, e1 - t0);
     __syncthreads();
-    const double2* src = reinterpret_cast<const double2*>(E + t0);
+    const double2* src = reinterpret_cast<const double2*>(fe + t0);
     double2* dst = reinterpret_cast<double2*>(se);
-    for (int i = threadIdx.x; i < nt * 8; i += FIELD_PTS) dst[i] = src[i];
+    constexpr int PIECES = (int)(sizeof(FieldElem) / sizeof(double2));
+    for (int i = threadIdx.x; i < nt * PIECES; i += FIELD_PTS) dst[i] = src[i];
     for (int i = threadIdx.x; i < RB * nt; i += FIELD_PTS) {
       const int r = i / nt, j = i - r * nt;
       sc[r][j] = coef[(int64_t)(r0 + r) * N + t0 + j];
     }
     __syncthreads();
     for (int j = 0; j < nt; j++) {
-      const Elem& e = se[j];
+      const FieldElem& e = se[j];
+      const double dx = p[0] - e.c[0], dy = p[1] - e.c[1], dz = p[2] - e.c[2];
+      const double dn = fma(dx, e.nrm[0], fma(dy, e.nrm[1], dz * e.nrm[2]));
+      const double krho = k * e.rho;
       double Lx = 0.0, Ly = 0.0, Mx = 0.0, My = 0.0;
-      for (int i = 0; i < 7; i++) {
-        const double a1 = cR7x1[i], a2 = cR7x2[i], a3 = 1.0 - a2 - a1;
-        const double rx = p[0] - ((a1 * e.n1[0] + a2 * e.n2[0]) + a3 * e.n3[0]);
-        const double ry = p[1] - ((a1 * e.n1[1] + a2 * e.n2[1]) + a3 * e.n3[1]);
-        const double rz = p[2] - ((a1 * e.n1[2] + a2 * e.n2[2]) + a3 * e.n3[2]);
-        const double r = sqrt(rx * rx + ry * ry + rz * rz);
-        const double ir = 1.0 / r;
-        const double kr = k * r;
-        double sn, cs;
-        sincos(kr, &sn, &cs);
-        const double g0 = ir * cR7g[i];
-        const double Gx = cs * g0, Gy = sn * g0;
-        const double t = -(rx * e.nrm[0] + ry * e.nrm[1] + rz * e.nrm[2]) * (ir * ir);
-        Lx += Gx;
-        Ly += Gy;
-        Mx += t * (-Gx - kr * Gy);
-        My += t * (kr * Gx - Gy);
+      if (krho <= 1.0) {  // the same for every thread: an element's property
+        const double krc = k * sqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+        double s0, c0, ax0 = 0.0, ay0 = 0.0, bx0 = 0.0, by0 = 0.0;
+        if (krho <= 0.35)
+          field_points64<false, 6, 6>(e, p[0], p[1], p[2], k, krc, ax0, ay0, bx0, by0);
+        else
+          field_points64<false, 8, 9>(e, p[0], p[1], p[2], k, krc, ax0, ay0, bx0, by0);
+        sincos(krc, &s0, &c0);
+        Lx = ax0 * c0 - ay0 * s0;
+        Ly = ax0 * s0 + ay0 * c0;
+        Mx = bx0 * c0 - by0 * s0;
+        My = bx0 * s0 + by0 * c0;
+      } else {
+        field_points64<true, 1, 1>(e, p[0], p[1], p[2], k, 0.0, Lx, Ly, Mx, My);
       }
+      Mx *= dn;
+      My *= dn;
 #pragma unroll
       for (int r = 0; r < RB; r++) {
         const FieldCoef c = sc[r][j];
@@ -250,19 +345,36 @@ __global__ void __launch_bounds__(FIELD_PTS)
   }
 }
 
-__global__ void field_finish_kernel(const double2* __restrict__ partial, int S, int64_t M, int R,
-                                    const double* __restrict__ pts, const double* __restrict__ src,
-                                    int nsrc, double k, double2 pfac, double2* __restrict__ phi_f,
-                                    double2* __restrict__ p_f) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M * R) return;
-  const int64_t r = i / M, ip = i - r * M;
+// Eight threads per value add its S partial sums, each an interleaved share in
+// order, then their sums in order (with one thread per value and S up to 300
+// chunks this kernel was a chain of 300 additions on a dozen CTAs).
+__global__ void __launch_bounds__(256)
+    field_finish_kernel(const double2* __restrict__ partial, int S, int64_t M, int R,
+                        const double* __restrict__ pts, const double* __restrict__ src, int nsrc,
+                        double k, double2 pfac, double2* __restrict__ phi_f,
+                        double2* __restrict__ p_f) {
+  __shared__ double2 red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+  const bool on = i < M * R;
   double ax = 0.0, ay = 0.0;
-  for (int s = 0; s < S; s++) {
-    const double2 v = partial[((int64_t)s * R + r) * M + ip];
-    ax += v.x;
-    ay += v.y;
+  if (on) {
+#pragma unroll 4
+    for (int s = w; s < S; s += 8) {
+      const double2 v = partial[(int64_t)s * R * M + i];
+      ax += v.x;
+      ay += v.y;
+    }
   }
+  red[w][lane] = make_double2(ax, ay);
+  __syncthreads();
+  if (w != 0 || !on) return;
+#pragma unroll
+  for (int q = 1; q < 8; q++) {
+    ax += red[q][lane].x;
+    ay += red[q][lane].y;
+  }
+  const int64_t ip = i % M;
   if (nsrc > 0) {  // sourcePhiTerm: w exp(ikr) / (4 pi r)
     const double px = pts[3 * ip], py = pts[3 * ip + 1], pz = pts[3 * ip + 2];
     for (int q = 0; q < nsrc; q++) {
@@ -281,26 +393,42 @@ __global__ void field_finish_kernel(const double2* __restrict__ partial, int S, 
   if (p_f) p_f[i] = make_double2(pfac.x * ax - pfac.y * ay, pfac.x * ay + pfac.y * ax);
 }
 
-template <int RB>
-void sum_pass(const Elem* E, const FieldElemF* fe, const void* coef, int64_t N, int R,
-              const double* pts, int64_t M, double k, int precision, int S, int64_t chunk,
-              int r0, double2* partial, cudaStream_t s) {
-  const dim3 grid((unsigned)((M + FIELD_PTS - 1) / FIELD_PTS), (unsigned)S);
+template <int RB, int PTS>
+void sum_pass(const void* fe, const void* coef, int64_t N, int R, const double* pts, int64_t M,
+              double k, int precision, int S, int64_t chunk, int r0, double2* partial,
+              cudaStream_t s) {
+  const dim3 grid((unsigned)((M + PTS - 1) / PTS), (unsigned)S);
   if (precision == 1) {
     const double kc = k / (2.0 * 3.14159265358979323846);
-    field_sum32_kernel<RB><<<grid, FIELD_PTS, 0, s>>>(fe, static_cast<const FieldCoefF*>(coef), N,
-                                                      chunk, pts, M, (float)k, (float)kc, r0, R,
-                                                      partial);
+    field_sum32_kernel<RB, PTS><<<grid, PTS, 0, s>>>(
+        static_cast<const FieldElemF*>(fe), static_cast<const FieldCoefF*>(coef), N, chunk, pts, M,
+        (float)k, (float)kc, r0, R, partial);
   } else {
-    field_sum64_kernel<RB><<<grid, FIELD_PTS, 0, s>>>(E, static_cast<const FieldCoef*>(coef), N,
-                                                      chunk, pts, M, k, r0, R, partial);
+    field_sum64_kernel<RB, PTS><<<grid, PTS, 0, s>>>(static_cast<const FieldElem*>(fe),
+                                                     static_cast<const FieldCoef*>(coef), N, chunk,
+                                                     pts, M, k, r0, R, partial);
   }
+}
+
+template <int PTS>
+int sum_passes(const void* fe, const void* coef, int64_t N, int R, const double* pts, int64_t M,
+               double k, int prec, int S, int64_t chunk, double2* partial, cudaStream_t s) {
+  int n = 0;
+  for (int r0 = 0; r0 < R; r0 += FIELD_RB, n++) {
+    switch (R - r0 >= FIELD_RB ? FIELD_RB : R - r0) {
+      case 1: sum_pass<1, PTS>(fe, coef, N, R, pts, M, k, prec, S, chunk, r0, partial, s); break;
+      case 2: sum_pass<2, PTS>(fe, coef, N, R, pts, M, k, prec, S, chunk, r0, partial, s); break;
+      case 3: sum_pass<3, PTS>(fe, coef, N, R, pts, M, k, prec, S, chunk, r0, partial, s); break;
+      default: sum_pass<4, PTS>(fe, coef, N, R, pts, M, k, prec, S, chunk, r0, partial, s); break;
+    }
+  }
+  return n;
 }
 
 }  // namespace
 
 int launch_field_prep(const Elem* E, const int64_t* perm, int64_t N, const double2* phi,
-                      const double2* dphi, int R, int precision, FieldElemF* fe, void* coef,
+                      const double2* dphi, int R, int precision, void* fe, void* coef,
                       cudaStream_t s) {
   if (N <= 0) return 0;
   field_prep_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(E, perm, N, phi, dphi, R,
@@ -308,21 +436,14 @@ int launch_field_prep(const Elem* E, const int64_t* perm, int64_t N, const doubl
   return 1;
 }
 
-int launch_field_sum(const Elem* E, const FieldElemF* fe, const void* coef, int64_t N, int R,
-                     const double* pts, int64_t M, double k, int precision, int S,
-                     double2* partial, cudaStream_t s) {
+int launch_field_sum(const void* fe, const void* coef, int64_t N, int R, const double* pts,
+                     int64_t M, double k, int precision, int S, double2* partial,
+                     cudaStream_t s) {
   if (M <= 0 || R <= 0 || S <= 0) return 0;
   const int64_t chunk = (N + S - 1) / S;
-  int n = 0;
-  for (int r0 = 0; r0 < R; r0 += FIELD_RB, n++) {
-    switch (R - r0 >= FIELD_RB ? FIELD_RB : R - r0) {
-      case 1: sum_pass<1>(E, fe, coef, N, R, pts, M, k, precision, S, chunk, r0, partial, s); break;
-      case 2: sum_pass<2>(E, fe, coef, N, R, pts, M, k, precision, S, chunk, r0, partial, s); break;
-      case 3: sum_pass<3>(E, fe, coef, N, R, pts, M, k, precision, S, chunk, r0, partial, s); break;
-      default: sum_pass<4>(E, fe, coef, N, R, pts, M, k, precision, S, chunk, r0, partial, s); break;
-    }
-  }
-  return n;
+  return field_points(M) == FIELD_PTS_SMALL
+             ? sum_passes<FIELD_PTS_SMALL>(fe, coef, N, R, pts, M, k, precision, S, chunk, partial, s)
+             : sum_passes<FIELD_PTS_LARGE>(fe, coef, N, R, pts, M, k, precision, S, chunk, partial, s);
 }
 
 int launch_field_finish(const double2* partial, int S, int64_t M, int R, const double* pts,
@@ -330,8 +451,8 @@ int launch_field_finish(const double2* partial, int S, int64_t M, int R, const d
                         double2* p_f, cudaStream_t s) {
   const int64_t cnt = M * R;
   if (cnt <= 0) return 0;
-  field_finish_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(partial, S, M, R, pts, src,
-                                                                    nsrc, k, pfac, phi_f, p_f);
+  field_finish_kernel<<<(unsigned)((cnt + 31) / 32), 256, 0, s>>>(partial, S, M, R, pts, src, nsrc,
+                                                                  k, pfac, phi_f, p_f);
   return 1;
 }
 

@@ -33,24 +33,38 @@ struct FieldCoef {
   double2 a, b;
 };
 
-constexpr int FIELD_PTS = 256;  // observation points (threads) per CTA
-constexpr int FIELD_TILE = 128; // elements per shared-memory tile
+// FP64 element record (224 bytes): centroid, unit normal, the 7 rule points
+// and the largest distance of a rule point from the centroid.
+struct __align__(16) FieldElem {
+  double c[3], nrm[3], q[21], rho;
+};
+static_assert(sizeof(FieldElem) == 224, "FieldElem is fourteen 16-byte pieces");
+
+// Observation points (threads) per CTA, and elements per shared-memory tile:
+// below 4,096 points CTAs of 64, so that a ragged last CTA idles at most 63
+// threads and there are enough CTAs to even out the SMs; above, 256 points
+// share one staging of the elements.
+constexpr int FIELD_PTS_SMALL = 64, FIELD_PTS_LARGE = 256;
+constexpr int64_t FIELD_SMALL_POINTS = 4096;
+inline int field_points(int64_t M) {
+  return M < FIELD_SMALL_POINTS ? FIELD_PTS_SMALL : FIELD_PTS_LARGE;
+}
 constexpr int FIELD_RB = 4;     // right-hand sides per pass
 
-// Element records (precision 1 only) and the coefficients of R columns:
-// phi, dphi are N x R complex FP64 in the caller's order, perm[j] the caller
-// index of cluster-order element j. coef: R x N FieldCoefF (precision 1) or
-// FieldCoef (precision 0). R = 0: the records only (perm, phi, dphi, coef
-// unused).
+// Element records and the coefficients of R columns: phi, dphi are N x R
+// complex FP64 in the caller's order, perm[j] the caller index of cluster-order
+// element j. fe: N FieldElemF (precision 1) or FieldElem (precision 0); coef:
+// R x N FieldCoefF or FieldCoef. R = 0: the records only (perm, phi, dphi,
+// coef unused).
 int launch_field_prep(const Elem* E, const int64_t* perm, int64_t N, const double2* phi,
-                      const double2* dphi, int R, int precision, FieldElemF* fe, void* coef,
+                      const double2* dphi, int R, int precision, void* fe, void* coef,
                       cudaStream_t s);
 
 // Partial sums over S element chunks: partial[(s R + r) M + i] for the M
 // points pts (M x 3, FP64) and all R columns. k is the wavenumber.
-int launch_field_sum(const Elem* E, const FieldElemF* fe, const void* coef, int64_t N, int R,
-                     const double* pts, int64_t M, double k, int precision, int S,
-                     double2* partial, cudaStream_t s);
+int launch_field_sum(const void* fe, const void* coef, int64_t N, int R, const double* pts,
+                     int64_t M, double k, int precision, int S, double2* partial,
+                     cudaStream_t s);
 
 // phi_f = sum over the S partials + point sources (src: nsrc x 5 doubles x, y,
 // z, Re w, Im w; sourcePhiTerm, boundaryelementsolver.cpp:3443-3450), added to

@@ -38,3 +38,27 @@ def test_training_gradient_at_tile_edges(bem, B):
     ref = mlp.grad(p.astype(np.float64), X.astype(np.float64), y.astype(int))
     assert np.linalg.norm(got[0] - ref) < 1e-5 * np.linalg.norm(ref)
     assert abs(float(loss.item()) - mlp.loss(p.astype(np.float64), X, y.astype(int))) < 1e-5
+
+
+@pytest.mark.parametrize("M", [1, 63, 65, 997, 4095, 4097])
+@pytest.mark.parametrize("freq", [300.0, 2500.0, 9000.0])
+def test_field_at_tile_edges(bem, meshes, orc, M, freq):
+    """Point tiles of 64 and 256, short element chunks, and the three forms of
+    the FP64 phase (k rho below 0.35, below 1 and above, rho ~ 0.02 m). FP64
+    differs from the oracle by the rounding of k r (about 200 at most): 1e-11
+    norm-wise; FP32 integrand 2e-5."""
+    tri = meshes.box(n_target=1200, seed=7)[:-3]
+    n = tri.shape[0]
+    rng = np.random.default_rng(M)
+    phi = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    dphi = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    pts = rng.uniform(-0.4, 0.8, (M, 3))
+    some = np.unique(np.r_[0, M - 1, rng.integers(0, M, 40)])  # points the oracle evaluates
+    ref, _ = orc.field(tri, freq, pts[some], phi, dphi, c=343.0, rho=1.2)
+    for precision, tol in ((0, 1e-11), (1, 2e-5)):
+        s = bem.Solver(precision=precision, wave_speed=343.0, density=1.2)
+        s.set_mesh(tri)
+        pf, _ = s.field(freq, pts, phi, dphi)
+        assert rel(pf[some], ref) < tol
+        assert np.isfinite(pf).all()
+        s.close()
