@@ -116,6 +116,14 @@ __device__ __forceinline__ bool gate_closed(const HmvGate& g) {
 }
 #endif
 
+// A piece of pass V of the H-matvec: `rows` rows of one block, from V + voff
+// (row stride n) and s + soff, times x[c0 .. c0 + n).
+struct __align__(16) HmvVRec {
+  int64_t voff, soff;
+  int32_t c0, n, rows, pad;
+};
+constexpr int HMV_VROWS = 16, HMV_VLROWS = 4, HMV_VLONG = 256;
+
 struct HmvArgs {
   int precision;  // 0: double2 storage, 1: float2 storage
   int fp32_math;  // float2 storage only: 0 FP64 arithmetic, 1 FP32 products with
@@ -142,10 +150,11 @@ struct HmvArgs {
   int accumulate;
   float2* xf;  // FP32 scratch copies of x (ldx x nrhs) and t (ldt x nrhs)
   float2* tf;  // for the FP32-arithmetic variant
-  // optional pass-V work list: items (far block, first row), 16 rows each,
-  // built from the block ranks; null = one CTA per far block
-  const int2* vwork;
-  int64_t nvwork;
+  // pass-V records, longest rows first; the first nlong are those of HMV_VLROWS
+  // rows of the blocks with more than HMV_VLONG columns (launch_vrec)
+  const HmvVRec* vrec;
+  int64_t nlong, nvwork;
+  const int2* vwork;  // launch_vrec only: (far block, first row) of every record
   HmvGate gate;  // null f: always run
   // two-float products only: remainders of the near-field entries (F + Flo
   // = the FP64 entries), null when the pool holds FP32-computed entries
@@ -165,6 +174,8 @@ void launch_points_nearfield(const NearBlock* blocks, int64_t nblocks, const Nea
 int launch_aca(const AcaArgs& a, int threads, cudaStream_t s);
 constexpr int ACA_BIG_MN = 512;  // blocks with m + n >= this get 512-thread CTAs
 int launch_hmatvec(const HmvArgs& a, cudaStream_t s);  // returns kernels launched
+// pass-V records of the work list a.vwork (nlong, nvwork, far, rank set)
+void launch_vrec(const HmvArgs& a, HmvVRec* rec, cudaStream_t s);
 
 // Fixed device scratch of the allocation-free H-matvec (complex FP64 entries,
 // 32 MiB): holds ldt x nrhs projections of one pass.

@@ -113,8 +113,9 @@ struct DevHM {
   bool has_lo = false;
   DBuf<int32_t> rank, flags;
   std::vector<int32_t> h_rank, h_flags;
-  DBuf<int2> vwork;  // H-matvec pass-V work items (block, first row)
-  int64_t nvwork = 0;
+  DBuf<int2> vwork;  // H-matvec pass-V work items (block, first row) and their records
+  DBuf<HmvVRec> vrec;
+  int64_t nlong = 0, nvwork = 0;
   int prec = 0;
   bool assembled = false;
 };
@@ -445,24 +446,42 @@ void fetch_ranks(bem_handle* h, DevHM& m) {
   const size_t nf = h->L.far.size();
   m.h_rank.resize(nf);
   m.h_flags.resize(nf);
+  m.nlong = 0;
   if (nf) {
     CK(cudaMemcpyAsync(m.h_rank.data(), m.rank.p, nf * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaMemcpyAsync(m.h_flags.data(), m.flags.p, nf * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   }
   sync(h);
-  // pass-V work items of the H-matvec: 16 rows of one block each, so the
-  // largest blocks spread over many CTAs. The buffer holds the most items the
-  // rank reservations allow, so it is allocated once per layout: growing it
-  // with the ranks of a frequency would free the old one, and cudaFree waits
-  // for every stream of the device (all sweep workers' queued kernels).
+  // pass-V work items of the H-matvec, longest rows first: HMV_VLROWS rows of
+  // the blocks with more than HMV_VLONG columns (a CTA each), then HMV_VROWS
+  // rows of the others (a warp each). The buffer holds the most items the rank
+  // reservations allow, so it is allocated once per layout: growing it with the
+  // ranks of a frequency would free the old one, and cudaFree waits for every
+  // stream of the device (all sweep workers' queued kernels).
   int64_t most = 0;
-  for (const FarBlock& f : h->L.far) most += ((int64_t)f.kcap + 15) / 16;
+  for (const FarBlock& f : h->L.far) {
+    const int step = f.n > HMV_VLONG ? HMV_VLROWS : HMV_VROWS;
+    most += ((int64_t)f.kcap + step - 1) / step;
+  }
   m.vwork.ensure((size_t)std::max<int64_t>(most, 1));
+  m.vrec.ensure((size_t)std::max<int64_t>(most, 1));
   std::vector<int2> vw;
-  for (size_t i = 0; i < nf; i++)
-    for (int32_t l0 = 0; l0 < m.h_rank[i]; l0 += 16) vw.push_back(make_int2((int)i, l0));
+  vw.reserve(nf + nf / 2);
+  for (int32_t i : h->L.v_order) {
+    const int step = h->L.far[i].n > HMV_VLONG ? HMV_VLROWS : HMV_VROWS;
+    for (int32_t l0 = 0; l0 < m.h_rank[i]; l0 += step) vw.push_back(make_int2(i, l0));
+    if (step == HMV_VLROWS) m.nlong = (int64_t)vw.size();
+  }
   m.vwork.upload(vw, h->stream);
   m.nvwork = (int64_t)vw.size();
+  HmvArgs ra{};
+  ra.vwork = m.vwork.p;
+  ra.nlong = m.nlong;
+  ra.nvwork = m.nvwork;
+  ra.far = h->dFar.p;
+  ra.rank = m.rank.p;
+  launch_vrec(ra, m.vrec.p, h->stream);
+  h->launches += m.nvwork > 0;
   sync(h);
   m.assembled = true;
   // factors of the previous matrix: dropped, unless they are kept as the
@@ -755,7 +774,8 @@ void hmatvec_dev(bem_handle* h, int which, const double2* x, double2* y, int64_t
     a.accumulate = acc;
     a.xf = h->dXf.p;
     a.tf = h->dTf.p;
-    a.vwork = m.vwork.p;
+    a.vrec = m.vrec.p;
+    a.nlong = m.nlong;
     a.nvwork = m.nvwork;
     a.Flo = (arith == ARITH_TWOFLOAT && m.has_lo) ? m.Flo.p : nullptr;
     if (gate_flags) a.gate = HmvGate{gate_flags + r0 * GATE_STRIDE, GATE_STRIDE, (int)a.nrhs};
@@ -2693,7 +2713,8 @@ bem_status bem_hmatvec_noalloc(bem_handle* h, int32_t which, const void* x, void
       a.V = m.V.p;
       a.S = m.S.p;
       a.F = m.F.p;
-      a.vwork = m.vwork.p;  // (block, 16-row) work items of pass V: handle-owned, no allocation
+      a.vrec = m.vrec.p;  // pass-V records: handle-owned, no allocation
+      a.nlong = m.nlong;
       a.nvwork = m.nvwork;
       a.x = xd + r0 * ncols;
       a.ldx = ncols;

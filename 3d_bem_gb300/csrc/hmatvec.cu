@@ -4,17 +4,24 @@
 // and scatters each block's U(s o (V^T x)) or F x into y under an omp critical.
 // Here the product runs in two passes with no atomics and a fixed summation
 // order:
-//   pass V: t_b = s_b o (V_b x_C) for every admissible block (one CTA each);
-//   pass U: one CTA per leaf row cluster sums, for its rows, every block whose
-//           row range contains them (U_b rows . t_b and dense F_b rows . x_C).
+//   pass V: t_b = s_b o (V_b x_C) for every admissible block, one warp per 16
+//           rows of V;
+//   pass U: one CTA (or cluster of CTAs) per leaf row cluster sums, for its
+//           rows, every block whose row range contains them (U_b rows . t_b
+//           and dense F_b rows . x_C).
 // Every stored matrix entry is read once per call for all R vectors.
 //
 // Arithmetic variants (GB300's FP64 rate is far below what HBM can feed):
 //   double2 storage, FP64 math  -- the plain complex-FP64 method;
-//   float2 storage,  FP64 math  -- exact products of the stored operator, used
-//                                  for the iterative-refinement residual;
-//   float2 storage,  FP32 math  -- FP32 products inside a block, FP64 sums
-//                                  across blocks; the inner GMRES operator.
+//   float2 storage,  FP64 math  -- exact products of the stored operator;
+//   float2 storage,  FP32 math  -- FP32 products inside a block, compensated
+//                                  FP32 sums across blocks; the inner GMRES
+//                                  operator;
+//   float2 storage,  two-float  -- FP64-accurate products on the FP32 units;
+//                                  the iterative-refinement residual.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <mutex>
 
 #include "bem_kernels.h"
@@ -23,470 +30,88 @@
 namespace bemgpu {
 namespace {
 
-constexpr int VT = 128;  // threads of a pass-V CTA
-constexpr int UT = 512;  // threads of a pass-U CTA (16 warps split a leaf's block list)
-// The FP32 U pass has two launch shapes. With many leaves (at least 4 per SM)
-// 256-thread CTAs capped at 40 registers (6 per SM, 48 warps) stream faster:
-// 20,480 elements 0.241 -> 0.222 ms per product against 512-thread CTAs with 60
-// registers (2 per SM); 128-thread CTAs (0.291 ms) and a 32-register cap
-// (0.226 ms, more spills) were slower. With few leaves the 512-thread CTAs
-// keep more warps busy: 5,120 elements 0.074 against 0.107 ms, 1,280 elements
-// 0.030 against 0.038 ms.
-constexpr int UT32_NARROW = 256, UT32_NARROW_MIN_CTAS = 6;
-constexpr int UT32_NARROW_LEAVES_PER_SM = 4;
-constexpr int UT32_WIDE_R = 256, UT32_WIDE_R_MIN_CTAS = 2;  // R >= 4: up to 128 registers
-constexpr int VROWS = 16;  // rows of V per pass-V work item (4 warps x 4 rows)
+namespace cg = cooperative_groups;
 
-template <typename T, bool F32> struct Acc;
-// FP64 accumulation
-template <typename T> struct Acc<T, false> {
-  double x = 0, y = 0;
-  __device__ __forceinline__ void fma(double2 a, double2 b) {
-    x += a.x * b.x - a.y * b.y;
-    y += a.x * b.y + a.y * b.x;
-  }
-};
-// FP32 accumulation
-template <typename T> struct Acc<T, true> {
-  float x = 0, y = 0;
-  __device__ __forceinline__ void fma(float2 a, float2 b) {
-    x += a.x * b.x - a.y * b.y;
-    y += a.x * b.y + a.y * b.x;
-  }
-};
+constexpr int VT = 128;          // threads of a pass-V CTA
+constexpr int VCTAS_PER_SM = 64;  // pass-V CTAs beyond the long rows (16 or 64: the same)
+constexpr int UT = 128;          // threads of a pass-U CTA
 
-__device__ __forceinline__ float2 ld32(const float2* p) { return __ldg(p); }
-
-// The block and row range of a pass-V CTA: with a work list, item
-// (block, first row) covers up to VROWS rows of V, so the largest blocks are
-// spread over many CTAs; without one, a CTA takes a whole block.
-__device__ __forceinline__ void vrange(const int2* __restrict__ vwork,
-                                       const int32_t* __restrict__ rank, int& b, int& lbeg,
-                                       int& lend) {
-  if (vwork) {
-    const int2 wi = vwork[blockIdx.x];
-    b = wi.x;
-    lbeg = wi.y;
-    lend = min(wi.y + VROWS, rank[b]);
-  } else {
-    b = blockIdx.x;
-    lbeg = 0;
-    lend = rank[b];
-  }
+// Launch shapes, measured per product (V + U pass, us). Pass V: 4 columns ahead
+// for one vector (20,480 sphere: 72 us; 2: 75, 1: 120), no unrolling for more
+// (20,480 pencil, 8 vectors: 104 us; 2: 150, 4: 130 -- fewer warps fit).
+// Pass U: 16 columns in flight and 6 CTAs of 128 per SM for one vector (20,480
+// sphere 68 us; 8 columns and 8 CTAs 81, 32 and 4: 83, CTAs of 64: 120, of 256:
+// 86), 8 columns for more (pencil, 8 vectors 107 us; 4 columns 121). Two-float
+// sums spill beyond 4 columns.
+__host__ __device__ constexpr int vunroll(int R) { return R == 1 ? 4 : 1; }
+template <class A>
+__host__ __device__ constexpr int ucolumns(int R) {
+  return A::kLo ? 4 : (R == 1 ? 16 : 8);
 }
-__device__ __forceinline__ float2 tof(double2 v) { return make_float2((float)v.x, (float)v.y); }
+__host__ __device__ constexpr int uctas(int R) { return R == 1 ? 6 : (R <= 3 ? 5 : 4); }
 
-// t[r][soff + l] = s_l * sum_j V[l, j] x[c0 + j, r]
-template <typename T, bool F32, int R>
-__global__ void __launch_bounds__(VT) hmv_vpass(const FarBlock* __restrict__ far,
-                                                const int32_t* __restrict__ rank,
-                                                const T* __restrict__ Vp,
-                                                const T* __restrict__ Sp,
-                                                const double2* __restrict__ x, int64_t ldx,
-                                                double2* __restrict__ t, int64_t ldt,
-                                                const int2* __restrict__ vwork, HmvGate gate) {
-  int bi, lbeg, lend;
-  vrange(vwork, rank, bi, lbeg, lend);
-  if (gate_closed(gate)) lend = lbeg;  // an empty range, not an early return: the
-                                       // kernel keeps its load scheduling
-  const FarBlock fb = far[bi];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int l = lbeg + w; l < lend; l += VT / 32) {
-    const T* Vl = Vp + fb.voff + (int64_t)l * fb.n;
-    double ax[R], ay[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) ax[r] = ay[r] = 0.0;
-    if constexpr (F32) {
-      float fx[R], fy[R];
-#pragma unroll
-      for (int r = 0; r < R; r++) fx[r] = fy[r] = 0.0f;
-#pragma unroll 4
-      for (int j = lane; j < fb.n; j += 32) {
-        const float2 v = ld32((const float2*)(Vl + j));
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          const float2 xv = tof(x[r * ldx + fb.c0 + j]);
-          fx[r] += v.x * xv.x - v.y * xv.y;
-          fy[r] += v.x * xv.y + v.y * xv.x;
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        ax[r] = fx[r];
-        ay[r] = fy[r];
-      }
-    } else {
-#pragma unroll 4
-      for (int j = lane; j < fb.n; j += 32) {
-        const double2 v = load_c(Vl + j);
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          const double2 xv = x[r * ldx + fb.c0 + j];
-          ax[r] += v.x * xv.x - v.y * xv.y;
-          ay[r] += v.x * xv.y + v.y * xv.x;
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        ax[r] += __shfl_xor_sync(0xffffffffu, ax[r], o);
-        ay[r] += __shfl_xor_sync(0xffffffffu, ay[r], o);
-      }
-    }
-    if (lane == 0) {
-      const double2 s = load_c(Sp + fb.soff + l);
-#pragma unroll
-      for (int r = 0; r < R; r++) t[r * ldt + fb.soff + l] = cmul(s, make_double2(ax[r], ay[r]));
-    }
+// ----- arithmetic policies: storage S, vector value X, accumulator Acc -----
+
+// FP64 products of either storage; vectors in the caller's columns
+template <typename T>
+struct ArF64 {
+  using S = T;
+  using X = double2;
+  using Acc = double2;
+  static constexpr bool kInterleaved = false;
+  static constexpr int kWords = 4;  // 32-bit registers of an accumulator
+  static constexpr bool kLo = false;  // dense blocks may have a low part (near_fp64)
+  static __device__ __forceinline__ Acc zero() { return make_double2(0.0, 0.0); }
+  static __device__ __forceinline__ void fma(Acc& a, S v, X x) {
+    double2 w;
+    if constexpr (sizeof(T) == sizeof(float2)) w = make_double2((double)v.x, (double)v.y);
+    else w = v;
+    a.x += w.x * x.x - w.y * x.y;
+    a.y += w.x * x.y + w.y * x.x;
   }
-}
-
-// One CTA per leaf row cluster; warps split the leaf's block list, lanes own
-// rows (32 rows per pass).
-template <typename T, bool F32, int R>
-__global__ void __launch_bounds__(UT) hmv_upass(
-    const LeafRows* __restrict__ leaves, const int32_t* __restrict__ list_off,
-    const int32_t* __restrict__ list, const FarBlock* __restrict__ far,
-    const int32_t* __restrict__ rank, const NearBlock* __restrict__ nearb,
-    const T* __restrict__ Up, const T* __restrict__ F, const double2* __restrict__ x,
-    int64_t ldx, const double2* __restrict__ t, int64_t ldt, double2* __restrict__ y,
-    int64_t ldy, int accumulate, HmvGate gate) {
-  __shared__ double2 part[UT / 32][32];
-  LeafRows lf = leaves[blockIdx.x];
-  if (gate_closed(gate)) lf.size = 0;  // no rows (see the V pass)
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int beg = list_off[blockIdx.x], end = list_off[blockIdx.x + 1];
-  for (int base = 0; base < lf.size; base += 32) {
-    const int ri = base + lane;  // row inside the leaf
-    const bool active = ri < lf.size;
-    const int64_t grow = lf.start + ri;
-    double ax[R], ay[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) ax[r] = ay[r] = 0.0;
-    for (int e = beg + w; e < end; e += UT / 32) {
-      const int32_t code = list[e];
-      Acc<T, F32> acc[R];
-      if (code >= 0) {  // admissible block: U rows . t
-        const FarBlock fb = far[code];
-        const int k = rank[code];
-        const T* U = Up + fb.uoff + (grow - fb.r0);
-        if (active) {
-#pragma unroll 4
-          for (int l = 0; l < k; l++) {
-            if constexpr (F32) {
-              const float2 u = ld32((const float2*)(U + (int64_t)l * fb.m));
-#pragma unroll
-              for (int r = 0; r < R; r++)
-                acc[r].fma(u, tof(t[r * ldt + fb.soff + l]));
-            } else {
-              const double2 u = load_c(U + (int64_t)l * fb.m);
-#pragma unroll
-              for (int r = 0; r < R; r++)
-                acc[r].fma(u, t[r * ldt + fb.soff + l]);
-            }
-          }
-        }
-      } else {  // dense near-field block: F rows . x
-        const NearBlock nb = nearb[-code - 1];
-        const T* Fb = F + nb.off + (grow - nb.r0);
-        if (active) {
-#pragma unroll 4
-          for (int j = 0; j < nb.n; j++) {
-            if constexpr (F32) {
-              const float2 f = ld32((const float2*)(Fb + (int64_t)j * nb.m));
-#pragma unroll
-              for (int r = 0; r < R; r++)
-                acc[r].fma(f, tof(x[r * ldx + nb.c0 + j]));
-            } else {
-              const double2 f = load_c(Fb + (int64_t)j * nb.m);
-#pragma unroll
-              for (int r = 0; r < R; r++)
-                acc[r].fma(f, x[r * ldx + nb.c0 + j]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < R; r++) {  // block partial into the FP64 row sum
-        ax[r] += (double)acc[r].x;
-        ay[r] += (double)acc[r].y;
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      part[w][lane] = make_double2(ax[r], ay[r]);
-      __syncthreads();
-      if (w == 0 && active) {
-        double2 s = part[0][lane];
-#pragma unroll
-        for (int q = 1; q < UT / 32; q++) s = cadd(s, part[q][lane]);
-        double2* yp = y + r * ldy + grow;
-        *yp = accumulate ? cadd(*yp, s) : s;
-      }
-      __syncthreads();
-    }
+  static __device__ __forceinline__ void add(Acc& a, Acc b) {
+    a.x += b.x;
+    a.y += b.y;
   }
-}
-
-// ---------------------------------------------------------------------------
-// FP32-arithmetic variant (complex-FP32 storage): x and t travel as FP32, the
-// block partials are added across blocks with a compensated (two-sum) FP32
-// accumulator, so no instruction of the inner loops touches the FP64 pipe.
-// ---------------------------------------------------------------------------
-struct TwoSum {
-  float hi = 0, lo = 0;
-  __device__ __forceinline__ void add(float v) {
-    const float s = hi + v;
-    const float bp = s - hi;
-    lo += (hi - (s - bp)) + (v - bp);
-    hi = s;
+  static __device__ __forceinline__ Acc shfl(Acc a, int o) {
+    return make_double2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
+  }
+  static __device__ __forceinline__ X scaled(S s, Acc a) {  // s * a as a vector value
+    double2 w;
+    if constexpr (sizeof(T) == sizeof(float2)) w = make_double2((double)s.x, (double)s.y);
+    else w = s;
+    return cmul(w, a);
   }
 };
 
-template <int R>
-__global__ void __launch_bounds__(VT) hmv32_vpass(const FarBlock* __restrict__ far,
-                                                  const int32_t* __restrict__ rank,
-                                                  const float2* __restrict__ Vp,
-                                                  const float2* __restrict__ Sp,
-                                                  const float2* __restrict__ x, int64_t ldx,
-                                                  float2* __restrict__ t, int64_t ldt,
-                                                  const int2* __restrict__ vwork, HmvGate gate) {
-  int bi, lbeg, lend;
-  vrange(vwork, rank, bi, lbeg, lend);
-  if (gate_closed(gate)) lend = lbeg;  // an empty range, not an early return: the
-                                       // kernel keeps its load scheduling
-  const FarBlock fb = far[bi];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // each warp streams G rows of V at once (G independent loads in flight per
-  // lane; short rows would otherwise leave one load per reduction chain)
-  constexpr int G = 4;
-  for (int l0 = lbeg + w * G; l0 < lend; l0 += (VT / 32) * G) {
-    const int ng = min(G, lend - l0);
-    const float2* V0 = Vp + fb.voff + (int64_t)l0 * fb.n;
-    float fx[G][R], fy[G][R];
-#pragma unroll
-    for (int g = 0; g < G; g++)
-#pragma unroll
-      for (int r = 0; r < R; r++) fx[g][r] = fy[g][r] = 0.0f;
-    for (int j = lane; j < fb.n; j += 32) {
-      float2 v[G];
-#pragma unroll
-      for (int g = 0; g < G; g++) v[g] = g < ng ? __ldg(V0 + (int64_t)g * fb.n + j) : make_float2(0, 0);
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        const float2 xv = __ldg(x + r * ldx + fb.c0 + j);
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-          fx[g][r] += v[g].x * xv.x - v[g].y * xv.y;
-          fy[g][r] += v[g].x * xv.y + v[g].y * xv.x;
-        }
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < G; g++)
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          fx[g][r] += __shfl_xor_sync(0xffffffffu, fx[g][r], o);
-          fy[g][r] += __shfl_xor_sync(0xffffffffu, fy[g][r], o);
-        }
-      }
-    if (lane < ng) {
-#pragma unroll
-      for (int g = 0; g < G; g++) {
-        if (g != lane) continue;  // lane g writes row l0 + g
-        const float2 s = __ldg(Sp + fb.soff + l0 + g);
-#pragma unroll
-        for (int r = 0; r < R; r++)
-          t[r * ldt + fb.soff + l0 + g] = fmul(s, make_float2(fx[g][r], fy[g][r]));
-      }
-    }
+// FP32 products and sums; vectors as FP32, the R values of an index together
+struct ArF32 {
+  using S = float2;
+  using X = float2;
+  using Acc = float2;
+  static constexpr bool kInterleaved = true;
+  static constexpr int kWords = 2;
+  static constexpr bool kLo = false;
+  static __device__ __forceinline__ Acc zero() { return make_float2(0.0f, 0.0f); }
+  static __device__ __forceinline__ void fma(Acc& a, S v, X x) {
+    a.x += v.x * x.x - v.y * x.y;
+    a.y += v.x * x.y + v.y * x.x;
   }
-}
-
-template <int R, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) hmv32_upass(
-    const LeafRows* __restrict__ leaves, const int32_t* __restrict__ list_off,
-    const int32_t* __restrict__ list, const FarBlock* __restrict__ far,
-    const int32_t* __restrict__ rank, const NearBlock* __restrict__ nearb,
-    const float2* __restrict__ Up, const float2* __restrict__ F, const float2* __restrict__ x,
-    int64_t ldx, const float2* __restrict__ t, int64_t ldt, double2* __restrict__ y,
-    int64_t ldy, int accumulate, HmvGate gate) {
-  __shared__ float4 part[NT / 32][32];
-  LeafRows lf = leaves[blockIdx.x];
-  if (gate_closed(gate)) lf.size = 0;  // no rows (see the V pass)
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int beg = list_off[blockIdx.x], end = list_off[blockIdx.x + 1];
-  for (int base = 0; base < lf.size; base += 32) {
-    const int ri = base + lane;
-    const bool active = ri < lf.size;
-    const int64_t grow = lf.start + ri;
-    TwoSum sx[R], sy[R];
-    for (int e = beg + w; e < end; e += NT / 32) {
-      const int32_t code = list[e];
-      float ax[R], ay[R];
-#pragma unroll
-      for (int r = 0; r < R; r++) ax[r] = ay[r] = 0.0f;
-      if (code >= 0) {
-        const FarBlock fb = far[code];
-        const int k = rank[code];
-        const float2* U = Up + fb.uoff + (grow - fb.r0);
-        if (active) {
-#pragma unroll 4
-          for (int l = 0; l < k; l++) {
-            const float2 u = __ldg(U + (int64_t)l * fb.m);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-              const float2 tv = __ldg(t + r * ldt + fb.soff + l);
-              ax[r] += u.x * tv.x - u.y * tv.y;
-              ay[r] += u.x * tv.y + u.y * tv.x;
-            }
-          }
-        }
-      } else {
-        const NearBlock nb = nearb[-code - 1];
-        const float2* Fb = F + nb.off + (grow - nb.r0);
-        if (active) {
-#pragma unroll 4
-          for (int j = 0; j < nb.n; j++) {
-            const float2 f = __ldg(Fb + (int64_t)j * nb.m);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-              const float2 xv = __ldg(x + r * ldx + nb.c0 + j);
-              ax[r] += f.x * xv.x - f.y * xv.y;
-              ay[r] += f.x * xv.y + f.y * xv.x;
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        sx[r].add(ax[r]);
-        sy[r].add(ay[r]);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      part[w][lane] = make_float4(sx[r].hi, sx[r].lo, sy[r].hi, sy[r].lo);
-      __syncthreads();
-      if (w == 0 && active) {
-        TwoSum ux, uy;  // combine the warps' partials in FP32, then one FP64 add
-#pragma unroll
-        for (int q = 0; q < NT / 32; q++) {
-          const float4 p = part[q][lane];
-          ux.add(p.x);
-          ux.add(p.y);
-          uy.add(p.z);
-          uy.add(p.w);
-        }
-        const double2 v = make_double2((double)ux.hi + (double)ux.lo, (double)uy.hi + (double)uy.lo);
-        double2* yp = y + r * ldy + grow;
-        *yp = accumulate ? cadd(*yp, v) : v;
-      }
-      __syncthreads();
-    }
+  static __device__ __forceinline__ void add(Acc& a, Acc b) {
+    a.x += b.x;
+    a.y += b.y;
   }
-}
-
-__global__ void to_float_kernel(const double2* __restrict__ x, float2* __restrict__ xf,
-                                int64_t n, HmvGate gate) {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i < n && !gate_closed(gate)) xf[i] = make_float2((float)x[i].x, (float)x[i].y);
-}
-
-// streaming multiprocessors of the current device (cached per device)
-int sm_count() {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      n = 152;
-    cached[dev] = n;
+  static __device__ __forceinline__ Acc shfl(Acc a, int o) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
   }
-  return cached[dev];
-}
+  static __device__ __forceinline__ X scaled(S s, Acc a) { return fmul(s, a); }
+};
 
-template <int R>
-void launch32_r(const HmvArgs& a, cudaStream_t s) {
-  to_float_kernel<<<(unsigned)((a.ldx * R + 255) / 256), 256, 0, s>>>(a.x, a.xf, a.ldx * R,
-                                                                      a.gate);
-  const int64_t nv = a.vwork ? a.nvwork : a.nfar;
-  if (nv > 0)
-    hmv32_vpass<R><<<(unsigned)nv, VT, 0, s>>>(a.far, a.rank, (const float2*)a.V,
-                                               (const float2*)a.S, a.xf, a.ldx, a.tf, a.ldt,
-                                               a.vwork, a.gate);
-  if (a.nleaves > 0) {
-    if (R >= 4)  // many right-hand sides: their accumulators need the registers
-                 // (the 40-register narrow shape spilled ~0.9 KB a thread at R = 8)
-      hmv32_upass<R, UT32_WIDE_R, UT32_WIDE_R_MIN_CTAS><<<(unsigned)a.nleaves, UT32_WIDE_R, 0, s>>>(
-          a.leaves, a.list_off, a.list, a.far, a.rank, a.nearb, (const float2*)a.U,
-          (const float2*)a.F, a.xf, a.ldx, a.tf, a.ldt, a.y, a.ldy, a.accumulate, a.gate);
-    else if (a.nleaves >= (int64_t)UT32_NARROW_LEAVES_PER_SM * sm_count())
-      hmv32_upass<R, UT32_NARROW, UT32_NARROW_MIN_CTAS><<<(unsigned)a.nleaves, UT32_NARROW, 0, s>>>(
-          a.leaves, a.list_off, a.list, a.far, a.rank, a.nearb, (const float2*)a.U,
-          (const float2*)a.F, a.xf, a.ldx, a.tf, a.ldt, a.y, a.ldy, a.accumulate, a.gate);
-    else
-      hmv32_upass<R, UT, 2><<<(unsigned)a.nleaves, UT, 0, s>>>(
-          a.leaves, a.list_off, a.list, a.far, a.rank, a.nearb, (const float2*)a.U,
-          (const float2*)a.F, a.xf, a.ldx, a.tf, a.ldt, a.y, a.ldy, a.accumulate, a.gate);
-  }
-}
-
-void launch32(const HmvArgs& a, cudaStream_t s) {
-  switch (a.nrhs) {
-    case 1: launch32_r<1>(a, s); break;
-    case 2: launch32_r<2>(a, s); break;
-    case 3: launch32_r<3>(a, s); break;
-    case 4: launch32_r<4>(a, s); break;
-    case 5: launch32_r<5>(a, s); break;
-    case 6: launch32_r<6>(a, s); break;
-    case 7: launch32_r<7>(a, s); break;
-    default: launch32_r<8>(a, s); break;
-  }
-}
-
-template <typename T, bool F32, int R>
-void launch_r(const HmvArgs& a, cudaStream_t s) {
-  const int64_t nv = a.vwork ? a.nvwork : a.nfar;
-  if (nv > 0)
-    hmv_vpass<T, F32, R><<<(unsigned)nv, VT, 0, s>>>(a.far, a.rank, (const T*)a.V,
-                                                     (const T*)a.S, a.x, a.ldx, a.t, a.ldt,
-                                                     a.vwork, a.gate);
-  if (a.nleaves > 0)
-    hmv_upass<T, F32, R><<<(unsigned)a.nleaves, UT, 0, s>>>(
-        a.leaves, a.list_off, a.list, a.far, a.rank, a.nearb, (const T*)a.U, (const T*)a.F, a.x,
-        a.ldx, a.t, a.ldt, a.y, a.ldy, a.accumulate, a.gate);
-}
-
-template <typename T, bool F32>
-void launch_t(const HmvArgs& a, cudaStream_t s) {
-  switch (a.nrhs) {
-    case 1: launch_r<T, F32, 1>(a, s); break;
-    case 2: launch_r<T, F32, 2>(a, s); break;
-    case 3: launch_r<T, F32, 3>(a, s); break;
-    case 4: launch_r<T, F32, 4>(a, s); break;
-    case 5: launch_r<T, F32, 5>(a, s); break;
-    case 6: launch_r<T, F32, 6>(a, s); break;
-    case 7: launch_r<T, F32, 7>(a, s); break;
-    default: launch_r<T, F32, 8>(a, s); break;  // the runtime splits R > 8 into chunks of 8
-  }
-}
-}  // namespace
-
-// ---------------------------------------------------------------------------
-// Double-float variant (complex-FP32 storage): FP64-accurate products of the
-// stored operator computed on the FP32 units. x and t are unevaluated sums
-// hi + lo of two floats; each stored entry a (exact in FP32) times hi is
+// Two-float products and sums on complex-FP32 storage. x and t are unevaluated
+// sums hi + lo of two floats; each stored entry a (exact in FP32) times hi is
 // split exactly with an FMA (p + e = a * hi), and sums run in two-float
-// precision (~2^-48). Used for the iterative-refinement residual b - A x,
-// which needs ~1e-14 relative accuracy but would be FP64-pipe-bound in
-// native FP64 on GB300.
-// ---------------------------------------------------------------------------
+// precision (~2^-48). The refinement residual b - A x needs ~1e-14 relative
+// accuracy but would be FP64-pipe-bound in native FP64 on GB300.
 struct DF {
   float hi = 0, lo = 0;
   // this += a * (yh + yl), a exact
@@ -506,17 +131,9 @@ struct DF {
     lo += e + l2;
     hi = s;
   }
-  __device__ __forceinline__ void shfl_reduce() {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float h2 = __shfl_xor_sync(0xffffffffu, hi, o);
-      const float l2 = __shfl_xor_sync(0xffffffffu, lo, o);
-      add(h2, l2);
-    }
-  }
 };
 
-// complex df accumulator: re + i im
+// complex two-float accumulator
 struct CDF {
   DF re, im;
   // += a * y, a = (ax, ay) exact floats, y = (yrh + yrl) + i (yih + yil)
@@ -528,141 +145,661 @@ struct CDF {
   }
 };
 
-__global__ void to_df_kernel(const double2* __restrict__ x, float4* __restrict__ xd, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n) return;
-  const double2 v = x[i];
-  const float rh = (float)v.x, ih = (float)v.y;
-  xd[i] = make_float4(rh, (float)(v.x - (double)rh), ih, (float)(v.y - (double)ih));
+struct ArDF {
+  using S = float2;
+  using X = float4;
+  using Acc = CDF;
+  static constexpr bool kInterleaved = true;
+  static constexpr int kWords = 4;
+  static constexpr bool kLo = true;
+  static __device__ __forceinline__ Acc zero() { return CDF(); }
+  static __device__ __forceinline__ void fma(Acc& a, S v, X x) { a.fma(v, x); }
+  static __device__ __forceinline__ void add(Acc& a, const Acc& b) {
+    a.re.add(b.re.hi, b.re.lo);
+    a.im.add(b.im.hi, b.im.lo);
+  }
+  static __device__ __forceinline__ Acc shfl(const Acc& a, int o) {
+    CDF b;
+    b.re.hi = __shfl_xor_sync(0xffffffffu, a.re.hi, o);
+    b.re.lo = __shfl_xor_sync(0xffffffffu, a.re.lo, o);
+    b.im.hi = __shfl_xor_sync(0xffffffffu, a.im.hi, o);
+    b.im.lo = __shfl_xor_sync(0xffffffffu, a.im.lo, o);
+    return b;
+  }
+  static __device__ __forceinline__ X scaled(S s, const Acc& a) {
+    CDF o;
+    o.fma(s, make_float4(a.re.hi, a.re.lo, a.im.hi, a.im.lo));
+    return make_float4(o.re.hi, o.re.lo, o.im.hi, o.im.lo);
+  }
+};
+
+__device__ __forceinline__ float2 ldg_s(const float2* p) { return __ldg(p); }
+__device__ __forceinline__ double2 ldg_s(const double2* p) { return __ldg(p); }
+
+// The R vector values of index i: FP64 vectors in columns of ld (x, or t with
+// its R values together), FP32 and two-float ones together, read as 16-byte
+// pieces where R makes them aligned.
+template <int R>
+__device__ __forceinline__ void load_vec(const float2* __restrict__ p, int64_t i, float2 (&v)[R]) {
+  if constexpr (R % 2 == 0) {
+    const float4* q = reinterpret_cast<const float4*>(p + i * R);
+#pragma unroll
+    for (int r = 0; r < R; r += 2) {
+      const float4 w = __ldg(q + r / 2);
+      v[r] = make_float2(w.x, w.y);
+      v[r + 1] = make_float2(w.z, w.w);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = __ldg(p + i * R + r);
+  }
+}
+template <int R>
+__device__ __forceinline__ void load_vec(const float4* __restrict__ p, int64_t i, float4 (&v)[R]) {
+#pragma unroll
+  for (int r = 0; r < R; r++) v[r] = __ldg(p + i * R + r);
+}
+template <int R>
+__device__ __forceinline__ void load_vec(const double2* __restrict__ p, int64_t i, double2 (&v)[R]) {
+#pragma unroll
+  for (int r = 0; r < R; r++) v[r] = __ldg(p + i * R + r);
+}
+template <class A, int R>
+__device__ __forceinline__ void load_x(const typename A::X* __restrict__ x, int64_t ldx, int64_t i,
+                                       typename A::X (&v)[R]) {
+  if constexpr (A::kInterleaved) {
+    load_vec<R>(x, i, v);
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = __ldg(x + r * ldx + i);
+  }
+}
+// ---------------------------------------------------------------------------
+// Pass V: t[soff + l][r] = s_l * sum_j V[l, j] x[c0 + j, r].
+// Work items come longest first, in two forms. Rows of more than HMV_VLONG
+// entries: a CTA takes HMV_VLROWS rows, its warps a quarter of the columns each
+// (a warp alone on 16 rows of 2,560 entries was the tail of the whole pass).
+// Shorter ones: a warp takes 16 rows, its four groups of 8 lanes rows l0 + g +
+// 4 i (i < G at a time). Most blocks are small (mean rank 17, mean row 126
+// entries at 20,480 sphere elements), where the reduction over the lanes costs
+// as much as the products: 8 lanes per row and a halving exchange (each step
+// halves what a lane still sums) take 8 shuffles for 16 rows at R = 1; one row
+// per warp step and a full butterfly took 160.
+// ---------------------------------------------------------------------------
+
+// acc[n] summed over the lanes that differ in the bits M, M / 2, .. 1 of their
+// number: each step halves the values a lane keeps while their number is
+// even; returns the index of the first value the lane ends with and clears
+// `mine` where another lane holds the same sums
+template <class A, int N, int M>
+__device__ __forceinline__ int halve(typename A::Acc (&acc)[N], int lane, bool& mine) {
+  if constexpr (M == 0) {
+    return 0;
+  } else if constexpr (N % 2 == 0) {
+    using Acc = typename A::Acc;
+    const bool up = lane & M;
+    Acc half[N / 2];
+#pragma unroll
+    for (int i = 0; i < N / 2; i++) {
+      const Acc send = up ? acc[i] : acc[i + N / 2];
+      const Acc got = A::shfl(send, M);
+      half[i] = up ? acc[i + N / 2] : acc[i];
+      A::add(half[i], got);
+    }
+    const int o = halve<A, N / 2, M / 2>(half, lane, mine) + (up ? N / 2 : 0);
+#pragma unroll
+    for (int i = 0; i < N / 2; i++) acc[i] = half[i];
+    return o;
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i++) A::add(acc[i], A::shfl(acc[i], M));
+    if (lane & M) mine = false;
+    return halve<A, N, M / 2>(acc, lane, mine);
+  }
+}
+// values a lane keeps after halve<A, n, m>
+__host__ __device__ constexpr int kept(int n, int m) {
+  return m == 0 ? n : kept(n % 2 == 0 ? n / 2 : n, m / 2);
 }
 
-// t[r][soff + l] = s_l * sum_j V[l, j] x[c0 + j, r], all in two-float
-template <int R>
-__global__ void __launch_bounds__(VT) hmvdf_vpass(const FarBlock* __restrict__ far,
-                                                  const int32_t* __restrict__ rank,
-                                                  const float2* __restrict__ Vp,
-                                                  const float2* __restrict__ Sp,
-                                                  const float4* __restrict__ x, int64_t ldx,
-                                                  float4* __restrict__ t, int64_t ldt,
-                                                  const int2* __restrict__ vwork) {
-  int bi, lbeg, lend;
-  vrange(vwork, rank, bi, lbeg, lend);
-  const FarBlock fb = far[bi];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int l = lbeg + w; l < lend; l += VT / 32) {
-    const float2* Vl = Vp + fb.voff + (int64_t)l * fb.n;
-    CDF acc[R];
-#pragma unroll 2
-    for (int j = lane; j < fb.n; j += 32) {
-      const float2 v = __ldg(Vl + j);
+// acc[i R + r] += sum over j = j0, j0 + step, .. < j1 of row[i][j] x[j, r]
+template <class A, int R, int G>
+__device__ __forceinline__ void vdots(const typename A::S* const (&row)[G],
+                                      const typename A::X* __restrict__ x, int64_t ldx, int64_t c0,
+                                      int j0, int j1, int step, typename A::Acc (&acc)[G * R]) {
+  constexpr int UN = vunroll(R);
+#pragma unroll UN
+  for (int j = j0; j < j1; j += step) {
+    typename A::S v[G];
 #pragma unroll
-      for (int r = 0; r < R; r++) acc[r].fma(v, __ldg(x + r * ldx + fb.c0 + j));
-    }
-    const float2 s = __ldg(Sp + fb.soff + l);
+    for (int i = 0; i < G; i++) v[i] = ldg_s(row[i] + j);
+    typename A::X xv[R];
+    load_x<A, R>(x, ldx, c0 + j, xv);
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      acc[r].re.shfl_reduce();
-      acc[r].im.shfl_reduce();
-      if (lane == 0) {
-        // (s) * (re + i im): s exact floats
-        CDF o;
-        o.fma(s, make_float4(acc[r].re.hi, acc[r].re.lo, acc[r].im.hi, acc[r].im.lo));
-        t[r * ldt + fb.soff + l] = make_float4(o.re.hi, o.re.lo, o.im.hi, o.im.lo);
-      }
-    }
+    for (int i = 0; i < G; i++)
+#pragma unroll
+      for (int r = 0; r < R; r++) A::fma(acc[i * R + r], v[i], xv[r]);
   }
 }
 
+// Expands the work list into records, so that a warp of pass V reaches its rows
+// after one load instead of three dependent ones.
+__global__ void vrec_kernel(const int2* __restrict__ vwork, int nlong, int64_t nvwork,
+                            const FarBlock* __restrict__ far, const int32_t* __restrict__ rank,
+                            HmvVRec* __restrict__ rec) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= nvwork) return;
+  const int2 w = vwork[i];
+  const FarBlock fb = far[w.x];
+  HmvVRec r;
+  r.voff = fb.voff + (int64_t)w.y * fb.n;
+  r.soff = fb.soff + w.y;
+  r.c0 = (int32_t)fb.c0;
+  r.n = fb.n;
+  r.rows = min(i < nlong ? HMV_VLROWS : HMV_VROWS, rank[w.x] - w.y);
+  r.pad = 0;
+  rec[i] = r;
+}
+
+__device__ __forceinline__ HmvVRec load_rec(const HmvVRec* p) {
+  HmvVRec r;
+  const int4 a = __ldg(reinterpret_cast<const int4*>(p));
+  const int4 b = __ldg(reinterpret_cast<const int4*>(p) + 1);
+  r.voff = (int64_t)(uint32_t)a.x | ((int64_t)a.y << 32);
+  r.soff = (int64_t)(uint32_t)a.z | ((int64_t)a.w << 32);
+  r.c0 = b.x;
+  r.n = b.y;
+  r.rows = b.z;
+  return r;
+}
+
+template <class A, int R, int G>
+__global__ void __launch_bounds__(VT) hmv_vpass(const HmvVRec* __restrict__ rec, int nlong,
+                                                int64_t nrec,
+                                                const typename A::S* __restrict__ Vp,
+                                                const typename A::S* __restrict__ Sp,
+                                                const typename A::X* __restrict__ x, int64_t ldx,
+                                                typename A::X* __restrict__ t, HmvGate gate) {
+  using S = typename A::S;
+  using Acc = typename A::Acc;
+  if (gate_closed(gate)) return;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if ((int)blockIdx.x < nlong) {
+    constexpr int GL = G < HMV_VLROWS ? G : HMV_VLROWS;  // rows at a time
+    constexpr int K = kept(GL * R, 16);
+    __shared__ Acc part[VT / 32][GL][R];
+    const HmvVRec rc = load_rec(rec + blockIdx.x);
+    const int quarter = (rc.n + VT / 32 - 1) / (VT / 32);
+    const int jb = w * quarter, je = min(rc.n, jb + quarter);
+    for (int l0 = 0; l0 < rc.rows; l0 += GL) {
+      const S* row[GL];
+#pragma unroll
+      for (int i = 0; i < GL; i++)  // rows past the end repeat the last one
+        row[i] = Vp + rc.voff + (int64_t)min(l0 + i, rc.rows - 1) * rc.n;
+      Acc acc[GL * R];
+#pragma unroll
+      for (int i = 0; i < GL * R; i++) acc[i] = A::zero();
+      vdots<A, R, GL>(row, x, ldx, rc.c0, jb + lane, je, 32, acc);
+      bool mine = true;
+      const int o = halve<A, GL * R, 16>(acc, lane, mine);
+      if (mine) {
+#pragma unroll
+        for (int i = 0; i < K; i++) part[w][(o + i) / R][(o + i) % R] = acc[i];
+      }
+      __syncthreads();
+      if (threadIdx.x < GL * R) {
+        const int l = threadIdx.x / R, r = threadIdx.x % R;
+        Acc v = part[0][l][r];
+#pragma unroll
+        for (int q = 1; q < VT / 32; q++) A::add(v, part[q][l][r]);
+        if (l0 + l < rc.rows)
+          t[(rc.soff + l0 + l) * R + r] = A::scaled(ldg_s(Sp + rc.soff + l0 + l), v);
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  // the shorter items, dealt to the warps of the grid in turn (longest first);
+  // the next record is loaded while the current one's rows are
+  const int64_t stride = (int64_t)(gridDim.x - nlong) * (VT / 32);
+  int64_t item = nlong + (int64_t)(blockIdx.x - nlong) * (VT / 32) + w;
+  if (item >= nrec) return;
+  const int g = lane >> 3, c = lane & 7;
+  constexpr int K = kept(G * R, 4);
+  HmvVRec rc = load_rec(rec + item);
+  while (true) {
+    const int64_t next = item + stride;
+    const HmvVRec rn = load_rec(rec + (next < nrec ? next : item));
+    const S sl = ldg_s(Sp + rc.soff + min(lane, rc.rows - 1));  // lane l: scale of row l
+    for (int q0 = 0; q0 < rc.rows; q0 += 4 * G) {
+      const S* row[G];
+#pragma unroll
+      for (int i = 0; i < G; i++)  // rows past the end repeat the last one
+        row[i] = Vp + rc.voff + (int64_t)min(q0 + g + 4 * i, rc.rows - 1) * rc.n;
+      Acc acc[G * R];
+#pragma unroll
+      for (int i = 0; i < G * R; i++) acc[i] = A::zero();
+      vdots<A, R, G>(row, x, ldx, rc.c0, c, rc.n, 8, acc);
+      bool mine = true;
+      const int o = halve<A, G * R, 4>(acc, lane, mine);
+#pragma unroll
+      for (int i = 0; i < K; i++) {
+        const int l = q0 + g + 4 * ((o + i) / R);
+        S sc;
+        sc.x = __shfl_sync(0xffffffffu, sl.x, l);
+        sc.y = __shfl_sync(0xffffffffu, sl.y, l);
+        if (mine && l < rc.rows) t[(rc.soff + l) * R + (o + i) % R] = A::scaled(sc, acc[i]);
+      }
+    }
+    if (next >= nrec) break;
+    item = next;
+    rc = rn;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Pass U: y rows of a leaf += U t of its admissible and F x of its dense
+// blocks. The CTAs of a cluster (one, two or four) load the descriptors of the
+// leaf's blocks into shared memory at once, lay all their columns end to end
+// and give every warp the same number of consecutive columns; lanes own rows. A
+// warp takes 32 columns at a time: lane i finds the block and address of the
+// i-th, loads its values of t or x and leaves both in shared memory, where the
+// loop over the columns reads them as broadcasts. So the loads in flight do not
+// stop at the end of a block (mean rank 17), and blocks of rank 5 and 80 do not
+// unbalance the warps. FP32 sums are plain over 32 columns and compensated
+// beyond. The partial sums of the warps and CTAs are added in a fixed order.
+// Bound by the bytes of U and F for one vector (20,480 sphere, 351 MB: 68 us,
+// 5.2 TB/s; one warp per block with 125 us before) and by the shared-memory
+// broadcasts and FMAs for eight (pencil, 20,480: 107 us, before 221 us).
+// ---------------------------------------------------------------------------
+
+// FP32 sums across blocks, compensated
+struct TwoSum {
+  float hi = 0, lo = 0;
+  __device__ __forceinline__ void add(float v) {
+    const float s = hi + v;
+    const float bp = s - hi;
+    lo += (hi - (s - bp)) + (v - bp);
+    hi = s;
+  }
+};
+
+// two FP32 FMAs as one instruction: same FMA rate, half the issue slots
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// Row sums of a warp over its columns: column() per column, flush() after 32 of
+// them; total[r][lane] (shared memory, zero at first) holds what is summed over
+// the warps in the end.
+template <class A, int R>
+struct RowSum {  // FP64, two-float
+  using Out = typename A::Acc;
+  static __device__ __forceinline__ Out none() { return A::zero(); }
+  typename A::Acc acc[R];
+  __device__ __forceinline__ RowSum() {
+#pragma unroll
+    for (int r = 0; r < R; r++) acc[r] = A::zero();
+  }
+  __device__ __forceinline__ void column(typename A::S u, const typename A::X* v) {
+#pragma unroll
+    for (int r = 0; r < R; r++) A::fma(acc[r], u, v[r]);
+  }
+  __device__ __forceinline__ void flush(Out (*total)[32], int lane) {}
+  __device__ __forceinline__ void finish(Out (*total)[32], int lane) {
+#pragma unroll
+    for (int r = 0; r < R; r++) total[r][lane] = acc[r];
+  }
+  static __device__ __forceinline__ void join(Out& a, const Out& b) { A::add(a, b); }
+};
 template <int R>
-__global__ void __launch_bounds__(UT) hmvdf_upass(
+struct RowSum<ArF32, R> {
+  using Out = float4;  // compensated sums (re.hi, re.lo, im.hi, im.lo)
+  static __device__ __forceinline__ Out none() { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+  // partial sums of up to 32 columns; with 4 or more vectors as packed pairs: pa
+  // sums u.x (t.x, t.y) and pb sums u.y (t.x, t.y), re = pa.x - pb.y,
+  // im = pa.y + pb.x
+  static constexpr bool kPacked = R >= 4;
+  uint64_t pa[kPacked ? R : 1], pb[kPacked ? R : 1];
+  float2 acc[kPacked ? 1 : R];
+  __device__ __forceinline__ RowSum() { clear(); }
+  __device__ __forceinline__ void clear() {
+    if constexpr (kPacked) {
+#pragma unroll
+      for (int r = 0; r < R; r++) pa[r] = pb[r] = 0;
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; r++) acc[r] = make_float2(0.0f, 0.0f);
+    }
+  }
+  __device__ __forceinline__ void column(float2 u, const float2* v) {
+    if constexpr (kPacked) {
+      const uint64_t ux = pack2(u.x, u.x), uy = pack2(u.y, u.y);
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const uint64_t w = pack2(v[r].x, v[r].y);
+        pa[r] = ffma2(ux, w, pa[r]);
+        pb[r] = ffma2(uy, w, pb[r]);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; r++) ArF32::fma(acc[r], u, v[r]);
+    }
+  }
+  __device__ __forceinline__ void flush(Out (*total)[32], int lane) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      float2 s;
+      if constexpr (kPacked) {
+        const float2 a = unpack2(pa[r]), b = unpack2(pb[r]);
+        s = make_float2(a.x - b.y, a.y + b.x);
+      } else {
+        s = acc[r];
+      }
+      const Out o = total[r][lane];
+      TwoSum sx{o.x, o.y}, sy{o.z, o.w};
+      sx.add(s.x);
+      sy.add(s.y);
+      total[r][lane] = make_float4(sx.hi, sx.lo, sy.hi, sy.lo);
+    }
+    clear();
+  }
+  __device__ __forceinline__ void finish(Out (*total)[32], int lane) {}
+  static __device__ __forceinline__ void join(Out& a, const Out& b) {
+    TwoSum x{a.x, a.y}, y{a.z, a.w};
+    x.add(b.x);
+    x.add(b.y);
+    y.add(b.z);
+    y.add(b.w);
+    a = make_float4(x.hi, x.lo, y.hi, y.lo);
+  }
+};
+__device__ __forceinline__ double2 out_value(double2 v) { return v; }
+__device__ __forceinline__ double2 out_value(const float4& v) {
+  return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
+}
+__device__ __forceinline__ double2 out_value(const CDF& v) {
+  return make_double2((double)v.re.hi + (double)v.re.lo, (double)v.im.hi + (double)v.im.lo);
+}
+
+// inclusive prefix sums of v over the CTA; total returned in sum
+template <int NW>
+__device__ __forceinline__ int cta_scan(int v, int (&scan)[NW], int& sum) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  if (lane == 31) scan[w] = v;
+  __syncthreads();
+  sum = 0;
+  int before = 0;
+#pragma unroll
+  for (int q = 0; q < NW; q++) {
+    before += q < w ? scan[q] : 0;
+    sum += scan[q];
+  }
+  __syncthreads();
+  return before + v;
+}
+
+template <class A, int R, int MINB, int UN>
+__global__ void __launch_bounds__(UT, MINB) hmv_upass(
     const LeafRows* __restrict__ leaves, const int32_t* __restrict__ list_off,
     const int32_t* __restrict__ list, const FarBlock* __restrict__ far,
     const int32_t* __restrict__ rank, const NearBlock* __restrict__ nearb,
-    const float2* __restrict__ Up, const float2* __restrict__ F, const float2* __restrict__ Flo,
-    const float4* __restrict__ x, int64_t ldx, const float4* __restrict__ t, int64_t ldt,
-    double2* __restrict__ y, int64_t ldy, int accumulate) {
-  __shared__ float4 part[UT / 32][32];
-  const LeafRows lf = leaves[blockIdx.x];
+    const typename A::S* __restrict__ Up, const typename A::S* __restrict__ F,
+    const typename A::S* __restrict__ Flo, const typename A::X* __restrict__ x, int64_t ldx,
+    const typename A::X* __restrict__ t, double2* __restrict__ y, int64_t ldy, int accumulate,
+    int ncta, HmvGate gate) {
+  using S = typename A::S;
+  using X = typename A::X;
+  using Sum = RowSum<A, R>;
+  using Out = typename Sum::Out;
+  constexpr int NW = UT / 32;
+  struct __align__(16) Stage {  // the warp's 32 columns
+    X v[32][R];
+    const S* ptr[32];
+  };
+  __shared__ const S* d_ptr[UT];  // first column at the leaf's row base
+  __shared__ int d_ld[UT];        // column stride
+  __shared__ int d_vec[UT];       // first index into t or x
+  __shared__ int d_end[2][UT];    // columns up to the end of the block: admissible, dense
+  __shared__ int scan[NW];
+  __shared__ __align__(16) unsigned char stage_raw[sizeof(Stage) * NW];
+  __shared__ __align__(16) unsigned char part_raw[sizeof(Out) * NW * R * 32];
+  Out(*part)[R][32] = reinterpret_cast<Out(*)[R][32]>(part_raw);
+  if (gate_closed(gate)) return;  // the same for every CTA of a cluster
+  const int leaf = blockIdx.x / ncta, cta = blockIdx.x - leaf * ncta;
+  const LeafRows lf = leaves[leaf];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int beg = list_off[blockIdx.x], end = list_off[blockIdx.x + 1];
+  Stage& st = reinterpret_cast<Stage*>(stage_raw)[w];
+  const int beg = list_off[leaf], end = list_off[leaf + 1];
+  const int nwarp = ncta * NW, me = cta * NW + w;
   for (int base = 0; base < lf.size; base += 32) {
-    const int ri = base + lane;
-    const bool active = ri < lf.size;
-    const int64_t grow = lf.start + ri;
-    CDF acc[R];
-    for (int e = beg + w; e < end; e += UT / 32) {
-      const int32_t code = list[e];
-      if (!active) continue;
-      if (code >= 0) {
-        const FarBlock fb = far[code];
-        const int k = rank[code];
-        const float2* U = Up + fb.uoff + (grow - fb.r0);
-#pragma unroll 2
-        for (int l = 0; l < k; l++) {
-          const float2 u = __ldg(U + (int64_t)l * fb.m);
+    const bool active = base + lane < lf.size;
+    const int64_t grow = lf.start + base;
+    const int my = active ? lane : 0;  // idle lanes repeat the first row
+    Sum sum;
 #pragma unroll
-          for (int r = 0; r < R; r++) acc[r].fma(u, __ldg(t + r * ldt + fb.soff + l));
+    for (int r = 0; r < R; r++) part[w][r][lane] = Sum::none();
+    for (int e0 = beg; e0 < end; e0 += UT) {
+      const int e = e0 + threadIdx.x, cntb = min(UT, end - e0);
+      int nf = 0, nn = 0;
+      if (e < end) {
+        const int32_t code = list[e];
+        if (code >= 0) {
+          const FarBlock fb = far[code];
+          nf = rank[code];
+          d_ptr[threadIdx.x] = Up + fb.uoff + (grow - fb.r0);
+          d_ld[threadIdx.x] = fb.m;
+          d_vec[threadIdx.x] = (int)fb.soff;
+        } else {
+          const NearBlock nb = nearb[-code - 1];
+          nn = nb.n;
+          d_ptr[threadIdx.x] = F + nb.off + (grow - nb.r0);
+          d_ld[threadIdx.x] = nb.m;
+          d_vec[threadIdx.x] = (int)nb.c0;
         }
-      } else {
-        const NearBlock nb = nearb[-code - 1];
-        const float2* Fb = F + nb.off + (grow - nb.r0);
-        if (Flo) {  // FP64 entries as hi + lo
-          const float2* Lb = Flo + nb.off + (grow - nb.r0);
-          for (int j = 0; j < nb.n; j++) {
-            const float2 f = __ldg(Fb + (int64_t)j * nb.m), fl = __ldg(Lb + (int64_t)j * nb.m);
+      }
+      int total[2];
+      d_end[0][threadIdx.x] = cta_scan<NW>(nf, scan, total[0]);
+      d_end[1][threadIdx.x] = cta_scan<NW>(nn, scan, total[1]);
+      __syncthreads();
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-              const float4 xv = __ldg(x + r * ldx + nb.c0 + j);
-              acc[r].fma(f, xv);
-              acc[r].fma(fl, xv);
+      for (int dense = 0; dense < 2; dense++) {
+        const int* ends = d_end[dense];
+        const int c1 = (int)((int64_t)total[dense] * (me + 1) / nwarp);
+        int c = (int)((int64_t)total[dense] * me / nwarp);
+        // the lane's column of the 32 from c (past the end: the last one)
+        const S* ptr = nullptr;
+        X v[R];
+        const auto find = [&]() {
+          const int col = min(c + lane, c1 - 1);
+          int lo = 0, hi = cntb - 1;  // first block that ends after it
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (ends[mid] > col) hi = mid;
+            else lo = mid + 1;
+          }
+          const int l = col - (lo > 0 ? ends[lo - 1] : 0);
+          ptr = d_ptr[lo] + (int64_t)l * d_ld[lo];
+          if (dense) load_x<A, R>(x, ldx, d_vec[lo] + l, v);
+          else load_vec<R>(t, d_vec[lo] + l, v);
+        };
+        if (c < c1) find();
+        while (c < c1) {
+          const int nb = min(32, c1 - c);
+          __syncwarp();
+          st.ptr[lane] = ptr;
+#pragma unroll
+          for (int r = 0; r < R; r++) st.v[lane][r] = v[r];
+          __syncwarp();
+          c += 32;
+          if (c < c1) find();  // the next 32 load meanwhile
+          for (int i = 0; i < nb; i += UN) {
+            S u[UN];
+#pragma unroll
+            for (int q = 0; q < UN; q++) {
+              u[q] = ldg_s(st.ptr[i + q] + my);
+              if (i + q >= nb) u[q].x = u[q].y = 0;
+            }
+#pragma unroll
+            for (int q = 0; q < UN; q++) sum.column(u[q], st.v[i + q]);
+            if constexpr (A::kLo) {
+              if (dense && Flo) {  // FP64 entries as hi + lo
+#pragma unroll
+                for (int q = 0; q < UN; q++) {
+                  u[q] = ldg_s(Flo + (st.ptr[i + q] - F) + my);
+                  if (i + q >= nb) u[q].x = u[q].y = 0;
+                }
+#pragma unroll
+                for (int q = 0; q < UN; q++) sum.column(u[q], st.v[i + q]);
+              }
             }
           }
-        } else {
-#pragma unroll 2
-          for (int j = 0; j < nb.n; j++) {
-            const float2 f = __ldg(Fb + (int64_t)j * nb.m);
-#pragma unroll
-            for (int r = 0; r < R; r++) acc[r].fma(f, __ldg(x + r * ldx + nb.c0 + j));
-          }
+          sum.flush(part[w], lane);
         }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      part[w][lane] = make_float4(acc[r].re.hi, acc[r].re.lo, acc[r].im.hi, acc[r].im.lo);
-      __syncthreads();
-      if (w == 0 && active) {
-        CDF sum;
-#pragma unroll
-        for (int q = 0; q < UT / 32; q++) {
-          const float4 p = part[q][lane];
-          sum.re.add(p.x, p.y);
-          sum.im.add(p.z, p.w);
-        }
-        const double2 v = make_double2((double)sum.re.hi + (double)sum.re.lo,
-                                       (double)sum.im.hi + (double)sum.im.lo);
-        double2* yp = y + r * ldy + grow;
-        *yp = accumulate ? cadd(*yp, v) : v;
       }
       __syncthreads();
     }
+    sum.finish(part[w], lane);
+    __syncthreads();
+    for (int i = threadIdx.x; i < R * 32; i += UT) {
+      const int r = i >> 5;
+      Out s = part[0][r][lane];
+#pragma unroll
+      for (int q = 1; q < NW; q++) Sum::join(s, part[q][r][lane]);
+      part[0][r][lane] = s;
+    }
+    if (ncta > 1) {
+      cg::cluster_group cl = cg::this_cluster();
+      cl.sync();
+      if (cta == 0)
+        for (int i = threadIdx.x; i < R * 32; i += UT) {
+          const int r = i >> 5;
+          Out s = part[0][r][lane];
+          for (int q = 1; q < ncta; q++) Sum::join(s, *cl.map_shared_rank(&part[0][r][lane], q));
+          part[0][r][lane] = s;
+        }
+      cl.sync();
+    }
+    if (cta == 0)
+      for (int i = threadIdx.x; i < R * 32; i += UT)
+        if (active) {
+          const double2 v = out_value(part[0][i >> 5][lane]);
+          double2* yp = y + (i >> 5) * ldy + grow + lane;
+          *yp = accumulate ? cadd(*yp, v) : v;
+        }
+    __syncthreads();
   }
+}
+
+// FP32 and two-float copies of the vectors, the R values of an index together
+__global__ void to_float_kernel(const double2* __restrict__ x, int64_t ldx, int R,
+                                float2* __restrict__ xf, HmvGate gate) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= ldx || gate_closed(gate)) return;
+  for (int r = 0; r < R; r++) {
+    const double2 v = x[r * ldx + i];
+    xf[i * R + r] = make_float2((float)v.x, (float)v.y);
+  }
+}
+
+__global__ void to_df_kernel(const double2* __restrict__ x, int64_t ldx, int R,
+                             float4* __restrict__ xd) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= ldx) return;
+  for (int r = 0; r < R; r++) {
+    const double2 v = x[r * ldx + i];
+    const float rh = (float)v.x, ih = (float)v.y;
+    xd[i * R + r] =
+        make_float4(rh, (float)(v.x - (double)rh), ih, (float)(v.y - (double)ih));
+  }
+}
+
+// streaming multiprocessors of the current device (cached per device)
+int sm_count() {
+  static int cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
+  if (!cached[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 152;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
+
+template <class A, int R>
+void launch_passes(const HmvArgs& a, const typename A::X* x, typename A::X* t, cudaStream_t s) {
+  using S = typename A::S;
+  // rows per lane group: as many as about 64 accumulator registers hold
+  constexpr int G = A::kWords * R * 4 <= 64 ? 4 : (A::kWords * R * 2 <= 64 ? 2 : 1);
+  if (a.nvwork > 0) {
+    const int64_t rest = (a.nvwork - a.nlong + VT / 32 - 1) / (VT / 32);
+    const int64_t grid = a.nlong + std::min<int64_t>(rest, (int64_t)VCTAS_PER_SM * sm_count());
+    hmv_vpass<A, R, G><<<(unsigned)grid, VT, 0, s>>>(a.vrec, (int)a.nlong, a.nvwork, (const S*)a.V,
+                                                     (const S*)a.S, x, a.ldx, t, a.gate);
+  }
+  if (a.nleaves <= 0) return;
+  // CTAs per leaf: with fewer than 16 warps per SM a leaf's columns go to a
+  // cluster of two, below 5 to one of four (64 leaves at 1,280 elements)
+  const int64_t per_sm = a.nleaves * (UT / 32) / sm_count();
+  const int ncta = per_sm >= 16 ? 1 : (per_sm >= 5 ? 2 : 4);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(a.nleaves * ncta));
+  cfg.blockDim = dim3(UT);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)ncta;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = ncta > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, hmv_upass<A, R, uctas(R), ucolumns<A>(R)>, a.leaves, a.list_off, a.list,
+                     a.far, a.rank, a.nearb, (const S*)a.U, (const S*)a.F, (const S*)a.Flo, x,
+                     a.ldx, (const typename A::X*)t, a.y, a.ldy, a.accumulate, ncta, a.gate);
+}
+
+template <int R>
+void launch32_r(const HmvArgs& a, cudaStream_t s) {
+  to_float_kernel<<<(unsigned)((a.ldx + 255) / 256), 256, 0, s>>>(a.x, a.ldx, R, a.xf, a.gate);
+  launch_passes<ArF32, R>(a, a.xf, a.tf, s);
 }
 
 template <int R>
 void launchdf_r(const HmvArgs& a, cudaStream_t s) {
   float4* xd = (float4*)a.xf;
-  float4* td = (float4*)a.tf;
-  to_df_kernel<<<(unsigned)((a.ldx * R + 255) / 256), 256, 0, s>>>(a.x, xd, a.ldx * R);
-  const int64_t nv = a.vwork ? a.nvwork : a.nfar;
-  if (nv > 0)
-    hmvdf_vpass<R><<<(unsigned)nv, VT, 0, s>>>(a.far, a.rank, (const float2*)a.V,
-                                               (const float2*)a.S, xd, a.ldx, td, a.ldt,
-                                               a.vwork);
-  if (a.nleaves > 0)
-    hmvdf_upass<R><<<(unsigned)a.nleaves, UT, 0, s>>>(
-        a.leaves, a.list_off, a.list, a.far, a.rank, a.nearb, (const float2*)a.U,
-        (const float2*)a.F, (const float2*)a.Flo, xd, a.ldx, td, a.ldt, a.y, a.ldy, a.accumulate);
+  to_df_kernel<<<(unsigned)((a.ldx + 255) / 256), 256, 0, s>>>(a.x, a.ldx, R, xd);
+  launch_passes<ArDF, R>(a, xd, (float4*)a.tf, s);
+}
+
+void launch32(const HmvArgs& a, cudaStream_t s) {
+  switch (a.nrhs) {
+    case 1: launch32_r<1>(a, s); break;
+    case 2: launch32_r<2>(a, s); break;
+    case 3: launch32_r<3>(a, s); break;
+    case 4: launch32_r<4>(a, s); break;
+    case 5: launch32_r<5>(a, s); break;
+    case 6: launch32_r<6>(a, s); break;
+    case 7: launch32_r<7>(a, s); break;
+    default: launch32_r<8>(a, s); break;
+  }
 }
 
 void launchdf(const HmvArgs& a, cudaStream_t s) {
@@ -670,10 +807,24 @@ void launchdf(const HmvArgs& a, cudaStream_t s) {
     case 1: launchdf_r<1>(a, s); break;
     case 2: launchdf_r<2>(a, s); break;
     case 3: launchdf_r<3>(a, s); break;
-    case 4: launchdf_r<4>(a, s); break;
     default: launchdf_r<4>(a, s); break;  // the runtime passes at most 4 per pass
   }
 }
+
+template <typename T>
+void launch64(const HmvArgs& a, cudaStream_t s) {
+  switch (a.nrhs) {
+    case 1: launch_passes<ArF64<T>, 1>(a, a.x, a.t, s); break;
+    case 2: launch_passes<ArF64<T>, 2>(a, a.x, a.t, s); break;
+    case 3: launch_passes<ArF64<T>, 3>(a, a.x, a.t, s); break;
+    case 4: launch_passes<ArF64<T>, 4>(a, a.x, a.t, s); break;
+    case 5: launch_passes<ArF64<T>, 5>(a, a.x, a.t, s); break;
+    case 6: launch_passes<ArF64<T>, 6>(a, a.x, a.t, s); break;
+    case 7: launch_passes<ArF64<T>, 7>(a, a.x, a.t, s); break;
+    default: launch_passes<ArF64<T>, 8>(a, a.x, a.t, s); break;  // the runtime splits R > 8
+  }
+}
+}  // namespace
 
 // ---------------------------------------------------------------------------
 // Fixed scratch for bem_hmatvec_noalloc: the per-block projections t = s o (V x)
@@ -711,15 +862,21 @@ cudaError_t hmatvec_noalloc_scratch(double2** out) {
   return cudaSuccess;
 }
 
+void launch_vrec(const HmvArgs& a, HmvVRec* rec, cudaStream_t s) {
+  if (a.nvwork > 0)
+    vrec_kernel<<<(unsigned)((a.nvwork + 255) / 256), 256, 0, s>>>(a.vwork, (int)a.nlong, a.nvwork,
+                                                                   a.far, a.rank, rec);
+}
+
 int launch_hmatvec(const HmvArgs& a, cudaStream_t s) {
-  if (a.precision == 0) launch_t<double2, false>(a, s);
+  if (a.precision == 0) launch64<double2>(a, s);
   else if (a.fp32_math == 1) {
     launch32(a, s);
     return 1 + (a.nfar > 0) + (a.nleaves > 0);
   } else if (a.fp32_math == 2) {
     launchdf(a, s);
     return 1 + (a.nfar > 0) + (a.nleaves > 0);
-  } else launch_t<float2, false>(a, s);
+  } else launch64<float2>(a, s);
   return (a.nfar > 0) + (a.nleaves > 0);
 }
 

@@ -62,6 +62,7 @@ struct Layout {
   std::vector<NearBlock> near;
   std::vector<FarBlock> far;
   std::vector<int32_t> far_order;   // launch order (largest first)
+  std::vector<int32_t> v_order;     // far blocks by columns, most first (H-matvec pass V)
   int64_t nbig = 0;                 // leading far_order entries on the 512-thread ACA kernel
   std::vector<NearTile> tiles;
   std::vector<uint32_t> special_bits;
