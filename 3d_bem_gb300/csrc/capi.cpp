@@ -202,16 +202,23 @@ struct bem_handle {
   DBuf<double2> dP1, dP2;
   // dataflow form of the sweeps (one plan per factor) and its workspace
   struct DfDev {
-    DBuf<unsigned char> chunks, rows, erows, cols, diag;
-    DBuf<int64_t> slot;
+    DBuf<HluDfItem> items;
+    DBuf<HluDfColumn> columns;
+    DBuf<HluDfDot> dots;
+    DBuf<HluDfInner> inner;
+    DBuf<HluDfChunk> chunks;
+    DBuf<HluDfSuper> supers;
+    DBuf<HluDfPanel> panels;
+    DBuf<int32_t> need;
+    DBuf<unsigned char> diag, minv;
     HluDfDev view;
   } dfL, dfU;
+  DBuf<unsigned char> dfDense;  // dense diagonal blocks while they are inverted
   bool df_ok = false;
   int df_helpers = 32;  // helper CTAs per dataflow sweep (12 while concurrent sweep workers run)
   int hlu_ctas_per_sm = 0;  // > 0: the executor's grid, per SM, below hp_grid (sweep workers)
   std::string df_why;
-  DBuf<unsigned char> dfXi, dfAcc, dfEacc;  // factor-type vectors
-  DBuf<unsigned char> dfPre, dfFin;
+  DBuf<unsigned char> dfXi, dfS, dfT;  // factor-type vectors
   DBuf<int> dfCtrl, dfErr;
   DBuf<int> dBad;
   DBuf<double2> dNear64[2];  // near_fp64: FP64 near field before the split
@@ -238,7 +245,6 @@ struct bem_handle {
   DBuf<HluQrOut> dHQr;
   DBuf<int> dHCtrl;
   DBuf<unsigned char> dArena, dHScr, dHBig;
-  HluDfPlan hpl, hpu;       // sweep plans of the program's factors (structure)
   // impedance plane (bem_set_impedance_plane): point, unit normal and the
   // elements reflected in it (cluster order)
   // point sources of the right-hand side (bem_set_point_sources)
@@ -876,28 +882,75 @@ void upload_bytes(DBuf<unsigned char>& d, const std::vector<T>& v, cudaStream_t 
     CK(cudaMemcpyAsync(d.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
 }
 
-// Plans of the dataflow sweeps for both factors; when either factor lacks
+// Device copy of a sweep plan (all but the apply matrices and inverses).
+void upload_df_plan(bem_handle* h, const HluDfPlan& p, int prec, bem_handle::DfDev& d) {
+  cudaStream_t s = h->stream;
+  d.items.upload(p.items, s);
+  d.columns.upload(p.columns, s);
+  d.dots.upload(p.dots, s);
+  d.inner.upload(p.inner, s);
+  d.chunks.upload(p.chunks, s);
+  d.supers.upload(p.supers, s);
+  const std::vector<HluDfPanel> panels = p.panels(prec);
+  d.panels.upload(panels, s);
+  d.need.upload(p.need, s);
+  HluDfDev v;
+  v.items = d.items.p;
+  v.columns = d.columns.p;
+  v.dots = d.dots.p;
+  v.inner = d.inner.p;
+  v.chunks = d.chunks.p;
+  v.supers = d.supers.p;
+  v.panels = d.panels.p;
+  v.need = d.need.p;
+  v.nt = p.nt;
+  v.msize = p.msize;
+  v.nitems = (int)p.items.size();
+  v.ninner = (int)p.inner.size();
+  v.npanels = (int)panels.size();
+  v.D = p.D();
+  v.lower = p.lower ? 1 : 0;
+  for (const HluDfSuper& u : p.supers) v.maxm = std::max(v.maxm, u.m);
+  d.view = v;
+}
+
+// The sweeps' vectors and flags, and the inverses of the supers' diagonal blocks
+// (views of both plans set; leaf data of both factors on the device).
+const void* hlu_data(const bem_handle* h, int which);
+void finish_df(bem_handle* h) {
+  cudaStream_t s = h->stream;
+  const size_t cs = h->hlu_prec == 0 ? sizeof(double2) : sizeof(float2);
+  bem_handle::DfDev* d[2] = {&h->dfL, &h->dfU};
+  h->dfXi.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
+  h->dfS.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
+  h->dfT.ensure((size_t)HLU_DF_MAX_R * std::max<int64_t>({d[0]->view.nt, d[1]->view.nt, 1}) * cs);
+  h->dfCtrl.ensure((size_t)(1 + 3 * std::max(d[0]->view.D, d[1]->view.D)));
+  h->dfErr.ensure(1);
+  CK(cudaMemsetAsync(h->dfErr.p, 0, sizeof(int), s));
+  h->dfDense.ensure((size_t)std::max(d[0]->view.msize, d[1]->view.msize) * cs);
+  for (int q = 0; q < 2; q++) {
+    d[q]->minv.ensure((size_t)d[q]->view.msize * cs);
+    d[q]->view.minv = d[q]->minv.p;
+    h->launches += launch_hlu_df_invert(d[q]->view, hlu_data(h, q), h->hlu_prec, h->dfDense.p, s);
+  }
+  CK(cudaGetLastError());
+}
+
+// Plans of the dataflow sweeps for both host factors; when either factor lacks
 // their structure both sweeps stay on the sequential kernel (df_why says why).
 void upload_df_plans(bem_handle* h) {
   h->df_ok = false;
   h->df_why.clear();
   HluDfPlan pl, pu;
-  const int eb = h->hlu_prec == 0 ? (int)sizeof(double2) : (int)sizeof(float2);
-  if (!hlu_df_plan(h->hL, h->N, eb, pl, &h->df_why) ||
-      !hlu_df_plan(h->hU, h->N, eb, pu, &h->df_why))
+  const std::vector<int64_t> cuts = hlu_df_cuts(h->rows, h->hlu_prec);
+  if (!hlu_df_plan(h->hL, h->N, cuts, pl, &h->df_why) ||
+      !hlu_df_plan(h->hU, h->N, cuts, pu, &h->df_why))
     return;
   cudaStream_t s = h->stream;
-  const size_t cs = h->hlu_prec == 0 ? sizeof(double2) : sizeof(float2);
-  int64_t nslot = 0;
-  int D = 0;
   for (int q = 0; q < 2; q++) {
     const HluDfPlan& p = q ? pu : pl;
     bem_handle::DfDev& d = q ? h->dfU : h->dfL;
-    upload_bytes(d.chunks, p.chunks, s);
-    upload_bytes(d.rows, p.rows, s);
-    upload_bytes(d.erows, p.erows, s);
-    upload_bytes(d.cols, p.cols, s);
-    d.slot.upload(p.slot, s);
+    upload_df_plan(h, p, h->hlu_prec, d);
     if (h->hlu_prec == 0) {
       upload_bytes(d.diag, p.diag, s);
     } else {
@@ -908,25 +961,9 @@ void upload_df_plans(bem_handle* h) {
       upload_bytes(d.diag, fd, s);
       CK(cudaStreamSynchronize(s));  // fd goes out of scope
     }
-    d.view.chunks = (const HluDfChunk*)d.chunks.p;
-    d.view.rows = (const HluDfRow*)d.rows.p;
-    d.view.erows = (const HluDfRow*)d.erows.p;
-    d.view.cols = (const HluDfCol*)d.cols.p;
-    d.view.slot = d.slot.p;
-    d.view.nslot = p.nslot;
     d.view.diag = d.diag.p;
-    d.view.D = p.D();
-    nslot = std::max(nslot, p.nslot);
-    D = std::max(D, p.D());
   }
-  h->dfXi.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
-  h->dfAcc.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
-  h->dfEacc.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
-  h->dfPre.ensure((size_t)std::max<int64_t>(2 * nslot, 1) * cs);  // pre and pre2
-  h->dfFin.ensure((size_t)std::max<int64_t>(nslot, 1) * cs);
-  h->dfCtrl.ensure((size_t)(4 + 4 * D));
-  h->dfErr.ensure(1);
-  CK(cudaMemsetAsync(h->dfErr.p, 0, sizeof(int), s));
+  finish_df(h);
   h->df_ok = true;
 }
 
@@ -1024,58 +1061,22 @@ void prepare_hlu_arena(bem_handle* h, int prec) {
   CK(cudaMemsetAsync(h->dArena.p, 0, (size_t)P.arena * es, h->stream));
   h->dHScr.ensure((size_t)h->hp_grid * P.scratch * es);
   h->dHBig.ensure((size_t)std::max<int64_t>(P.big_scratch, 1) * es);
-  // sweep plans: the staging offsets of their late leaves depend on the
-  // element size of the factors
-  h->hpl = HluDfPlan();
-  h->hpu = HluDfPlan();
+  // sweep plans of the program's factors (the inversion's panels depend on the
+  // element type)
   if (P.df_ok) {
     std::string w;
-    const bool ok = hlu_df_plan_structure(P.L, h->N, (int)es, h->hpl, &w) &&
-                    hlu_df_plan_structure(P.U, h->N, (int)es, h->hpu, &w);
+    HluDfPlan pl, pu;
+    const std::vector<int64_t> cuts = hlu_df_cuts(h->rows, prec);
+    const bool ok = hlu_df_plan_structure(P.L, h->N, cuts, pl, &w) &&
+                    hlu_df_plan_structure(P.U, h->N, cuts, pu, &w);
     require(ok, BEM_EINVAL, "H-LU program: sweep plan");
+    upload_df_plan(h, pl, prec, h->dfL);
+    upload_df_plan(h, pu, prec, h->dfU);
+    h->dfL.view.diag = h->dArena.p + (size_t)P.qh_base * es;
+    h->dfU.view.diag = h->dArena.p + (size_t)P.rinv_base * es;
+    CK(cudaStreamSynchronize(h->stream));  // the plans go out of scope
   }
   h->hp_prec = prec;
-}
-
-// The dataflow sweeps of the program's factors: plans uploaded without their
-// apply matrices, which the QR tasks write into the arena at the plans'
-// offsets.
-void upload_df_plans_device(bem_handle* h) {
-  h->df_ok = false;
-  h->df_why = h->hp.df_why;
-  if (!h->hp.df_ok) return;
-  cudaStream_t s = h->stream;
-  const size_t cs = h->hlu_prec == 0 ? sizeof(double2) : sizeof(float2);
-  int64_t nslot = 0;
-  int D = 0;
-  for (int q = 0; q < 2; q++) {
-    const HluDfPlan& p = q ? h->hpu : h->hpl;
-    bem_handle::DfDev& d = q ? h->dfU : h->dfL;
-    upload_bytes(d.chunks, p.chunks, s);
-    upload_bytes(d.rows, p.rows, s);
-    upload_bytes(d.erows, p.erows, s);
-    upload_bytes(d.cols, p.cols, s);
-    d.slot.upload(p.slot, s);
-    d.view.chunks = (const HluDfChunk*)d.chunks.p;
-    d.view.rows = (const HluDfRow*)d.rows.p;
-    d.view.erows = (const HluDfRow*)d.erows.p;
-    d.view.cols = (const HluDfCol*)d.cols.p;
-    d.view.slot = d.slot.p;
-    d.view.nslot = p.nslot;
-    d.view.diag = h->dArena.p + (size_t)(q ? h->hp.rinv_base : h->hp.qh_base) * cs;
-    d.view.D = p.D();
-    nslot = std::max(nslot, p.nslot);
-    D = std::max(D, p.D());
-  }
-  h->dfXi.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
-  h->dfAcc.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
-  h->dfEacc.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
-  h->dfPre.ensure((size_t)std::max<int64_t>(2 * nslot, 1) * cs);  // pre and pre2
-  h->dfFin.ensure((size_t)std::max<int64_t>(nslot, 1) * cs);
-  h->dfCtrl.ensure((size_t)(4 + 4 * D));
-  h->dfErr.ensure(1);
-  CK(cudaMemsetAsync(h->dfErr.p, 0, sizeof(int), s));
-  h->df_ok = true;
 }
 
 // H-LU of the truncated copy of the assembled dPhi matrix, on the GPU: one
@@ -1269,6 +1270,15 @@ bool build_hlu_device(bem_handle* h) {
   CK(cudaGetLastError());
   launch_hlu_finite_check(h->dArena.p, P.arena, m.prec, h->dHCtrl.p + 3, h->nsm, s);
   h->launches++;
+  if (P.df_ok) {  // the sweeps' inverses, and their own check
+    h->hlu_prec = m.prec;
+    h->hlu_dev = true;
+    finish_df(h);
+    h->hlu_dev = false;
+    for (bem_handle::DfDev* d : {&h->dfL, &h->dfU})
+      launch_hlu_finite_check(d->minv.p, d->view.msize, m.prec, h->dHCtrl.p + 3, h->nsm, s);
+    h->launches += 2;
+  }
   int ctrl[4] = {0, 0, 0, 0};
   CK(cudaMemcpyAsync(ctrl, h->dHCtrl.p, sizeof(ctrl), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
@@ -1283,7 +1293,8 @@ bool build_hlu_device(bem_handle* h) {
   h->dLl.upload(P.L.leaves, s);
   h->dUs.upload(P.U.schedule, s);
   h->dUl.upload(P.U.leaves, s);
-  upload_df_plans_device(h);
+  h->df_ok = P.df_ok;
+  h->df_why = P.df_why;
   CK(cudaStreamSynchronize(s));
   h->hlu_dev = true;
   h->have_hlu = true;
@@ -1401,47 +1412,6 @@ const void* hlu_data(const bem_handle* h, int which) {
   return which ? h->dUd.p : h->dLd.p;
 }
 
-// mean driver phase times of a traced lower sweep: wait for R(i), corner,
-// solve, hand-over to the next chunk (appended to path)
-void df_trace_summary(bem_handle* h, const DBuf<unsigned long long>& tr, int R, const char* path) {
-  const int D = h->dfL.view.D;
-  std::vector<unsigned long long> t(4 * (size_t)D);
-  CK(cudaStreamSynchronize(h->stream));
-  CK(cudaMemcpy(t.data(), tr.p, t.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
-  double ph[4] = {};
-  for (int i = 0; i + 1 < D; i++) {
-    ph[0] += 1e-3 * (double)(t[4 * i + 1] - t[4 * i]);
-    ph[1] += 1e-3 * (double)(t[4 * i + 2] - t[4 * i + 1]);
-    ph[2] += 1e-3 * (double)(t[4 * i + 3] - t[4 * i + 2]);
-    ph[3] += 1e-3 * (double)(t[4 * (i + 1)] - t[4 * i + 3]);
-  }
-  FILE* f = std::fopen(path, "a");
-  if (!f) return;
-  const double n = D > 1 ? (double)(D - 1) : 1.0;
-  std::fprintf(f, "df L sweep: chunks %d R %d total_us %.1f per chunk us: wait %.3f corner %.3f "
-               "solve %.3f handover %.3f\n", D, R, 1e-3 * (double)(t[4 * (D - 1) + 3] - t[0]),
-               ph[0] / n, ph[1] / n, ph[2] / n, ph[3] / n);
-  // the wait by corner kind (device factors: the program's plan): none,
-  // full, low rank, low rank with a prefix (R(i) then waits for C(i - 2))
-  if (h->hlu_dev && (int)h->hpl.chunks.size() == D + 1) {
-    double wsum[4] = {}, late[4] = {};
-    int64_t cnt[4] = {};
-    for (int i = 1; i + 1 < D; i++) {
-      const HluDfChunk& c = h->hpl.chunks[i];
-      const int kind = c.corner < 0 ? 0 : (!(c.cflags & 1) ? 1 : ((c.cflags & 2) ? 3 : 2));
-      wsum[kind] += 1e-3 * (double)(t[4 * i + 1] - t[4 * i]);
-      late[kind] += (double)(h->hpl.chunks[i + 1].rbeg - c.rbeg);
-      cnt[kind]++;
-    }
-    const char* nm[4] = {"none", "full", "lowrank", "lowrank+pre"};
-    for (int k = 0; k < 4; k++)
-      if (cnt[k])
-        std::fprintf(f, "  corner %-11s chunks %6lld wait_us %.3f late_entries %.2f\n", nm[k],
-                     (long long)cnt[k], wsum[k] / cnt[k], late[k] / cnt[k]);
-  }
-  std::fclose(f);
-}
-
 // w := U^{-1} L^{-1} w for R device vectors (LUPrecondidionedHMatrixWrapper's
 // two substitutions, gmres.h:134-147)
 void apply_precond(bem_handle* h, double2* w, int R, const int* gate_flags = nullptr) {
@@ -1449,31 +1419,20 @@ void apply_precond(bem_handle* h, double2* w, int R, const int* gate_flags = nul
   cudaStream_t s = h->stream;
   if (h->df_ok) {  // dataflow sweeps: w -> dP2 -> w, up to 8 vectors per launch
     h->dP2.ensure((size_t)std::min(R, HLU_DF_MAX_R) * N);
-    HluDfWork ws{h->dfXi.p, h->dfAcc.p, h->dfEacc.p, h->dfPre.p, h->dfFin.p, h->dfCtrl.p, h->dfErr.p};
+    HluDfWork ws{h->dfXi.p, h->dfS.p, h->dfT.p, h->dfCtrl.p, h->dfErr.p};
     if (const char* e = std::getenv("BEM_DF_WAIT_US"))  // tests of the timeout path
       if (std::atof(e) > 0) ws.wait_ns = (unsigned long long)(std::atof(e) * 1000.0);
     const int hp = df_helpers(h);
-    // BEM_DF_TRACE=<file>: the lower sweep's driver phases of this
-    // application, summarised into the file (profiling)
-    const char* trace_path = std::getenv("BEM_DF_TRACE");
-    DBuf<unsigned long long> trace;
-    if (trace_path && *trace_path) {
-      trace.ensure(4 * (size_t)h->dfL.view.D);
-      ws.trace = trace.p;
-    }
     for (int r0 = 0; r0 < R; r0 += HLU_DF_MAX_R) {
       const int rc = std::min(HLU_DF_MAX_R, R - r0);
       double2* wr = w + (size_t)r0 * N;
       const HmvGate gate = gate_flags ? HmvGate{gate_flags + r0 * GATE_STRIDE, GATE_STRIDE, rc}
                                       : HmvGate{nullptr, 0, 0};
-      h->launches += launch_hlu_df(h->dfL.view, h->dLl.p, hlu_data(h, 0), h->hlu_prec, wr, h->dP2.p,
-                                   N, rc, ws, hp, s, gate);
-      HluDfWork wu = ws;
-      wu.trace = nullptr;
-      h->launches += launch_hlu_df(h->dfU.view, h->dUl.p, hlu_data(h, 1), h->hlu_prec, h->dP2.p, wr,
-                                   N, rc, wu, hp, s, gate);
+      h->launches += launch_hlu_df(h->dfL.view, hlu_data(h, 0), h->hlu_prec, wr, h->dP2.p, N, rc, ws,
+                                   hp, s, gate);
+      h->launches += launch_hlu_df(h->dfU.view, hlu_data(h, 1), h->hlu_prec, h->dP2.p, wr, N, rc, ws,
+                                   hp, s, gate);
     }
-    if (ws.trace) df_trace_summary(h, trace, R, trace_path);
     return;
   }
   h->dP1.ensure((size_t)R * N);

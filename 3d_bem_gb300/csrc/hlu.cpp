@@ -806,8 +806,35 @@ void hlu_factor(const HTree& tree, const std::vector<HBlockDesc>& blocks, std::v
   flatten_upper(Un, U);
 }
 
+std::vector<int64_t> hlu_df_cuts(const HTree& tree, int precision) {
+  std::vector<int64_t> cuts;
+  std::vector<int64_t> todo{0};
+  while (!todo.empty()) {
+    const HCluster& c = tree.c[todo.back()];
+    todo.pop_back();
+    if (c.size <= hlu_df_super(precision) || c.leaf || c.son1 < 0) {
+      cuts.push_back(c.start);
+      continue;
+    }
+    todo.push_back(c.son1);
+    todo.push_back(c.son2);
+  }
+  cuts.push_back(tree.c[0].start + tree.c[0].size);
+  std::sort(cuts.begin(), cuts.end());
+  cuts.erase(std::unique(cuts.begin(), cuts.end()), cuts.end());
+  return cuts;
+}
+
+std::vector<HluDfPanel> HluDfPlan::panels(int precision) const {
+  std::vector<HluDfPanel> v;
+  const int w = hlu_df_panel_cols(precision);
+  for (int i = 0; i < D(); i++)
+    for (int p0 = 0; p0 < supers[i].m; p0 += w) v.push_back(HluDfPanel{i, p0});
+  return v;
+}
+
 namespace {
-bool df_plan_impl(const FlatFactor& f, int64_t N, int elem_bytes, HluDfPlan& p,
+bool df_plan_impl(const FlatFactor& f, int64_t N, const std::vector<int64_t>& cuts, HluDfPlan& p,
                   std::string* why, bool with_diag) {
   p = HluDfPlan();
   auto fail = [&](const char* s) {
@@ -820,11 +847,13 @@ bool df_plan_impl(const FlatFactor& f, int64_t N, int elem_bytes, HluDfPlan& p,
   std::vector<int32_t> diag;
   for (int32_t op : f.schedule)
     if (op >= 0) diag.push_back(op);
-  const int D = (int)diag.size();
-  if (D == 0 || N <= 0) return fail("no diagonal leaves");
+  const int C = (int)diag.size();  // chunks
+  if (C == 0 || N <= 0) return fail("no diagonal leaves");
+  if (cuts.size() < 2 || cuts.front() != 0 || cuts.back() != N) return fail("cuts");
+  p.lower = lv[7 * (int64_t)diag[0] + 4] == 2;  // Q leaves: L, R leaves: U
   std::vector<int32_t> chunk_of(N, -1);
-  std::vector<int64_t> cr0(D), cm(D);
-  for (int i = 0; i < D; i++) {
+  std::vector<int64_t> cr0(C), cm(C);
+  for (int i = 0; i < C; i++) {
     const int64_t* L = lv + 7 * (int64_t)diag[i];
     if (L[0] != L[2] || L[1] != L[3] || L[1] < 1 || L[1] > HLU_DF_MAX_M || L[0] < 0 ||
         L[0] + L[1] > N)
@@ -838,127 +867,156 @@ bool df_plan_impl(const FlatFactor& f, int64_t N, int elem_bytes, HluDfPlan& p,
   }
   for (int64_t r = 0; r < N; r++)
     if (chunk_of[r] < 0) return fail("diagonal leaves do not cover the rows");
-  // chunks [lo, hi] (solve order) that tile [a, a + len) exactly
-  auto span = [&](int64_t a, int64_t len, int& lo, int& hi) {
-    if (len < 1 || a < 0 || a + len > N) return false;
-    const int c1 = chunk_of[a], c2 = chunk_of[a + len - 1];
-    lo = std::min(c1, c2);
-    hi = std::max(c1, c2);
-    int64_t tot = 0;
-    for (int c = lo; c <= hi; c++) {
-      if (cr0[c] < a || cr0[c] + cm[c] > a + len) return false;
-      tot += cm[c];
-    }
-    return tot == len;
-  };
-  std::vector<std::vector<HluDfRow>> rl(D), el(D);  // late, early
-  std::vector<std::vector<HluDfCol>> cl(D);
-  std::vector<HluDfChunk> ch(D + 1);
-  for (int i = 0; i <= D; i++) {
-    ch[i] = HluDfChunk{};
-    ch[i].corner = -1;
+  for (int i = 1; i < C; i++)  // the sweeps go through the rows in one direction
+    if (p.lower ? cr0[i] != cr0[i - 1] + cm[i - 1] : cr0[i] + cm[i] != cr0[i - 1])
+      return fail("diagonal leaves out of order");
+  // supers in solve order
+  const int D = (int)cuts.size() - 1;
+  std::vector<int32_t> super_of(N);
+  p.supers.resize(D);
+  for (int q = 0; q < D; q++) {
+    const int i = p.lower ? q : D - 1 - q;
+    HluDfSuper& s = p.supers[i];
+    s.r0 = (int32_t)cuts[q];
+    s.m = (int32_t)(cuts[q + 1] - cuts[q]);
+    if (s.m < 1 || s.m > HLU_DF_SUPER) return fail("super too large");
+    for (int64_t r = cuts[q]; r < cuts[q + 1]; r++) super_of[r] = i;
   }
-  p.slot.assign(nl, -1);
+  for (HluDfSuper& s : p.supers) {
+    s.moff = p.msize;
+    p.msize += (int64_t)s.m * s.m;
+    s.chunk_beg = s.chunk_end = -1;
+  }
+  p.chunks.resize(C);
+  int64_t aoff = 0;
+  for (int i = 0; i < C; i++) {
+    HluDfSuper& s = p.supers[super_of[cr0[i]]];
+    if (super_of[cr0[i] + cm[i] - 1] != super_of[cr0[i]]) return fail("a cut inside a diagonal leaf");
+    if (s.chunk_beg < 0) s.chunk_beg = i;
+    s.chunk_end = i + 1;
+    p.chunks[i].r0 = (int32_t)(cr0[i] - s.r0);
+    p.chunks[i].m = (int32_t)cm[i];
+    p.chunks[i].aoff = aoff;
+    aoff += cm[i] * cm[i];
+  }
+  std::vector<std::vector<HluDfColumn>> rowc(C);
+  std::vector<std::vector<HluDfDot>> dots(D);
   for (int32_t op : f.schedule) {
     if (op >= 0) continue;
-    const int32_t o = -op - 1;
-    const int64_t* L = lv + 7 * (int64_t)o;
-    const int64_t kind = L[4], k = L[5];
+    const int64_t* L = lv + 7 * (int64_t)(-op - 1);
+    const int64_t r0 = L[0], m = L[1], c0 = L[2], n = L[3], kind = L[4], k = L[5], off = L[6];
     if (kind != 0 && kind != 1) return fail("off-diagonal leaf kind");
     const bool lr = kind == 1;
     if (lr && (k < 1 || k > HLU_DF_MAX_RANK)) return fail("low-rank leaf rank");
-    int ra, rb, ca, cb;
-    if (!span(L[0], L[1], ra, rb) || !span(L[2], L[3], ca, cb))
-      return fail("leaf not aligned with the diagonal leaves");
-    if (cb >= ra) return fail("leaf not below the diagonal in solve order");
-    bool uses_fin = false;
-    for (int i = ra; i <= rb; i++) {
-      const int32_t ro = (int32_t)(cr0[i] - L[0]);
-      if (cb == i - 1) {
-        if (ch[i].corner >= 0) return fail("two corner leaves");
-        ch[i].corner = o;
-        ch[i].cro = ro;
-        ch[i].cco = (int32_t)(cr0[i - 1] - L[2]);
-        ch[i].cflags = (lr ? 1 : 0) | (lr && ca < cb ? 2 : 0) | (!lr && ca == cb ? 4 : 0) |
-                       (lr && ca + 1 < cb ? 8 : 0);
-        ch[i].cco2 = lr && ca < cb ? (int32_t)(cr0[i - 2] - L[2]) : 0;
-        ch[i].cw2 = lr && ca < cb ? (int32_t)cm[i - 2] : 0;
-        ch[i].cm = (int32_t)L[1];
-        ch[i].cn = (int32_t)L[3];
-        ch[i].ck = (int32_t)k;
-        ch[i].cc0 = (int32_t)L[2];
-        ch[i].cdata = L[6];
-      } else {
-        auto& list = cb <= i - HLU_DF_LAG ? el[i] : rl[i];
-        if (!lr) {
-          list.push_back(HluDfRow{o, ro, 0, 0, -1});
-        } else if (cb == i - 2) {
-          list.push_back(HluDfRow{o, ro, ca < cb ? 2 : 3, (int32_t)(cr0[i - 2] - L[2]), -1});
-        } else {
-          list.push_back(HluDfRow{o, ro, 1, 0, -1});
-          uses_fin = true;
-        }
-      }
-    }
-    if (!lr) continue;
-    // prefixes of t = V x: pre over cols ca..cb-2, read by the corner (rows
-    // cb + 1, which adds chunks cb - 1 and cb itself, so it waits on nothing
-    // solved after chunk cb - 2); pre2 over ca..cb-1, read by mode 2 (rows
-    // cb + 2) and by the last step into fin (mode 1)
-    const bool uses_pre = ca < cb && ra <= cb + 2;
-    if (!uses_pre && !uses_fin) continue;
-    p.slot[o] = p.nslot;
-    p.nslot += k * HLU_DF_MAX_R;
-    for (int j = ca; j <= cb; j++) {
-      const bool last = j == cb;
-      if (last && !uses_fin) continue;
-      const int32_t fl = (j == ca ? 1 : 0) | (last ? 2 : 0) | (j == cb - 1 ? 4 : 0) |
-                         (last && ca < cb ? 8 : 0);
-      for (int32_t l = 0; l < (int32_t)k; l++)
-        cl[j].push_back(HluDfCol{o, (int32_t)(cr0[j] - L[2]), fl, l});
-    }
-  }
-  // CSR lists, apply matrices
-  int64_t moff = 0;
-  for (int i = 0; i < D; i++) {
-    ch[i].r0 = (int32_t)cr0[i];
-    ch[i].m = (int32_t)cm[i];
-    ch[i].moff = moff;
-    // late entries: at most one per column chunk i - LAG + 1 .. i - 2; their
-    // constants (full: F rows, low rank: U rows and V over cols(i - 2)) get
-    // staging offsets, 32 rows per column / rank, within the staging budget
-    if ((int)rl[i].size() > HLU_DF_NLATE) return fail("too many late leaves");
-    int64_t so = 0;
-    const int64_t budget = HLU_DF_STAGE_BYTES / elem_bytes;
-    for (HluDfRow& r : rl[i]) {
-      const int64_t* L = lv + 7 * (int64_t)r.leaf;
-      const int64_t need = L[4] == 0 ? (L[3] <= 2 * HLU_DF_MAX_M ? 32 * L[3] : budget + 1)
-                                     : 32 * L[5] * (r.mode >= 2 ? 2 : 1);
-      if (so + need <= budget) {
-        r.soff = (int32_t)so;
-        so += need;
-      }
-    }
-    ch[i].rbeg = (int32_t)p.rows.size();
-    p.rows.insert(p.rows.end(), rl[i].begin(), rl[i].end());
-    ch[i].ebeg = (int32_t)p.erows.size();
-    p.erows.insert(p.erows.end(), el[i].begin(), el[i].end());
-    ch[i].cbeg = (int32_t)p.cols.size();
-    p.cols.insert(p.cols.end(), cl[i].begin(), cl[i].end());
-    const int64_t* L = lv + 7 * (int64_t)diag[i];
-    const int64_t m = L[1];
-    if (!with_diag) {
-      if (L[4] != 2 && L[4] != 3) return fail("diagonal leaf kind");
-      moff += m * m;
+    if (m < 1 || n < 1 || r0 < 0 || c0 < 0 || r0 + m > N || c0 + n > N || off < 0)
+      return fail("leaf out of range");
+    if (p.lower ? c0 + n > r0 : r0 + m > c0) return fail("leaf not below the diagonal in solve order");
+    const int ra = super_of[r0], rb = super_of[r0 + m - 1];
+    const int ca = super_of[c0], cb = super_of[c0 + n - 1];
+    const int rlo = std::min(ra, rb), chi = std::max(ca, cb);
+    if (chi == rlo) {  // inside one diagonal block
+      if (ra != rb || ca != cb) return fail("leaf not aligned with the cuts");
+      const HluDfSuper& s = p.supers[ra];
+      HluDfInner in{};
+      in.off = off;
+      in.dst = s.moff + (r0 - s.r0) * s.m + (c0 - s.r0);
+      in.lowrank = lr ? 1 : 0;
+      in.m = (int32_t)m;
+      in.n = (int32_t)n;
+      in.k = (int32_t)k;
+      in.ld = s.m;
+      p.inner.push_back(in);
       continue;
     }
+    if (chi > rlo) return fail("leaf not aligned with the cuts");
+    // chunks of its rows
+    const int qa = chunk_of[r0], qb = chunk_of[r0 + m - 1];
+    const int64_t slot = p.nt;
+    for (int q = std::min(qa, qb); q <= std::max(qa, qb); q++) {
+      if (cr0[q] < r0 || cr0[q] + cm[q] > r0 + m) return fail("leaf not aligned with the diagonal leaves");
+      for (int64_t l = 0; l < (lr ? k : n); l++)
+        rowc[q].push_back(HluDfColumn{off + (cr0[q] - r0) + l * m,
+                                      (int32_t)(lr ? slot + l : -1 - (c0 + l)), 0});
+    }
+    if (!lr) continue;
+    p.nt += k;
+    for (int j = std::min(ca, cb); j <= chi; j++) {
+      const HluDfSuper& s = p.supers[j];
+      const int64_t a = std::max<int64_t>(c0, s.r0), b = std::min<int64_t>(c0 + n, s.r0 + s.m);
+      for (int64_t l = 0; l < k; l += 2)
+        dots[j].push_back(HluDfDot{off + m * k + l * n + (a - c0), (int32_t)n,
+                                   (int32_t)std::min<int64_t>(2, k - l), (int32_t)(b - a),
+                                   (int32_t)(a - s.r0), (int32_t)(slot + l),
+                                   j == std::min(ca, cb) ? 1 : 0});
+    }
+  }
+  if (p.nt > INT32_MAX / 2) return fail("too many low-rank leaves");
+  // items in claim order: ROW(I), DIAG(I), DOT(I) (an empty DOT item keeps the
+  // chain DOT(I) after DOT(I - 1))
+  p.need.assign(3 * (size_t)D, 0);
+  for (int i = 0; i < D; i++) {
+    const HluDfSuper& s = p.supers[i];
+    for (int q = s.chunk_beg; q < s.chunk_end; q++) {
+      HluDfItem it{};
+      it.type = HLU_DF_ROW;
+      it.level = i;
+      it.beg = (int32_t)p.columns.size();
+      p.columns.insert(p.columns.end(), rowc[q].begin(), rowc[q].end());
+      it.end = (int32_t)p.columns.size();
+      it.r0 = (int32_t)cr0[q];
+      it.m = (int32_t)cm[q];
+      p.items.push_back(it);
+      p.need[3 * i]++;
+    }
+    for (int t0 = 0; t0 < s.m; t0 += HLU_DF_TILE) {
+      HluDfItem it{};
+      it.type = HLU_DF_DIAG;
+      it.level = i;
+      it.r0 = s.r0;
+      it.m = s.m;
+      it.t0 = t0;
+      it.moff = s.moff;
+      // block lower triangular in solve order: the columns up to the end (lower)
+      // or from the start (upper) of the chunks of its rows
+      const int64_t last = std::min<int64_t>(t0 + HLU_DF_TILE, s.m) - 1;
+      const int qe = chunk_of[s.r0 + (p.lower ? last : t0)];
+      it.c0 = p.lower ? 0 : (int32_t)(cr0[qe] - s.r0);
+      it.c1 = p.lower ? (int32_t)(cr0[qe] + cm[qe] - s.r0) : s.m;
+      p.items.push_back(it);
+      p.need[3 * i + 1]++;
+    }
+    // long dots first, so that one does not end an item alone
+    std::stable_sort(dots[i].begin(), dots[i].end(),
+                     [](const HluDfDot& x, const HluDfDot& y) { return x.w > y.w; });
+    for (size_t b = 0; b == 0 || b < dots[i].size(); b += HLU_DF_WARPS) {
+      HluDfItem it{};
+      it.type = HLU_DF_DOT;
+      it.level = i;
+      it.beg = (int32_t)p.dots.size();
+      p.dots.insert(p.dots.end(), dots[i].begin() + b,
+                    dots[i].begin() + std::min(dots[i].size(), b + HLU_DF_WARPS));
+      it.end = (int32_t)p.dots.size();
+      it.r0 = s.r0;
+      it.m = s.m;
+      p.items.push_back(it);
+      p.need[3 * i + 2]++;
+    }
+  }
+  if (p.columns.size() > (size_t)INT32_MAX || p.dots.size() > (size_t)INT32_MAX)
+    return fail("too many leaves");
+  // apply matrices
+  for (int i = 0; i < C; i++) {
+    const int64_t* L = lv + 7 * (int64_t)diag[i];
+    const int64_t m = L[1], moff = p.chunks[i].aoff;
+    if (L[4] != (p.lower ? 2 : 3)) return fail("diagonal leaf kind");
+    if (!with_diag) continue;
     const cd* Dd = f.data.data() + L[6];
     if (L[6] < 0 || L[6] + m * m > (int64_t)f.data.size()) return fail("diagonal leaf data");
     p.diag.resize(moff + m * m);
     cd* M = p.diag.data() + moff;
-    if (L[4] == 2) {  // Q (column-major): M[row][t] = conj(Q[t, row]) = conj(Q[row * m + t])
+    if (p.lower) {  // Q (column-major): M[row][t] = conj(Q[t, row]) = conj(Q[row * m + t])
       for (int64_t e = 0; e < m * m; e++) M[e] = std::conj(Dd[e]);
-    } else if (L[4] == 3) {  // R upper (column-major): M = R^{-1} row-major
+    } else {  // R upper (column-major): M = R^{-1} row-major
       for (int64_t t = 0; t < m; t++) {
         if (Dd[t + t * m] == cd(0.0)) return fail("zero pivot");
         for (int64_t row = 0; row < m; row++) M[row * m + t] = 0.0;
@@ -970,30 +1028,20 @@ bool df_plan_impl(const FlatFactor& f, int64_t N, int elem_bytes, HluDfPlan& p,
           M[row * m + t] = -acc / Dd[row + row * m];
         }
       }
-    } else {
-      return fail("diagonal leaf kind");
     }
-    moff += m * m;
   }
-  ch[D].r0 = (int32_t)N;
-  ch[D].rbeg = (int32_t)p.rows.size();
-  ch[D].ebeg = (int32_t)p.erows.size();
-  ch[D].cbeg = (int32_t)p.cols.size();
-  ch[D].moff = moff;
-  p.chunks = std::move(ch);
   return true;
 }
 }  // namespace
 
-bool hlu_df_plan(const FlatFactor& f, int64_t N, int elem_bytes, HluDfPlan& p,
+bool hlu_df_plan(const FlatFactor& f, int64_t N, const std::vector<int64_t>& cuts, HluDfPlan& p,
                  std::string* why) {
-  return df_plan_impl(f, N, elem_bytes, p, why, true);
+  return df_plan_impl(f, N, cuts, p, why, true);
 }
 
-bool hlu_df_plan_structure(const FlatFactor& f, int64_t N, int elem_bytes, HluDfPlan& p,
-                           std::string* why) {
-  return df_plan_impl(f, N, elem_bytes, p, why, false);
+bool hlu_df_plan_structure(const FlatFactor& f, int64_t N, const std::vector<int64_t>& cuts,
+                           HluDfPlan& p, std::string* why) {
+  return df_plan_impl(f, N, cuts, p, why, false);
 }
 
 }  // namespace bemgpu
-

@@ -52,27 +52,35 @@ void hlu_factor(const HTree& tree, const std::vector<HBlockDesc>& blocks,
                 std::vector<InBlock>& in, int64_t max_rank, double tol, FlatFactor& L,
                 FlatFactor& U);
 
-// Plan of the dataflow sweep (hlu_solve.h) for one flattened factor: chunks
-// in solve order with their corner leaves, row and column lists, pre/fin slot
-// offsets, and the m x m apply matrix of every diagonal leaf, row-major:
-// conj(Q) stored like Q (y = Q^H s) for L, R^{-1} for U (back substitution
-// done once here, per column of the identity, instead of once per sweep).
+// Plan of the dataflow sweep (hlu_solve.h) for one flattened factor: items in
+// claim order with their columns and dots, what the inversion of the supers'
+// diagonal blocks needs, and (host factors) the m x m apply matrix of every
+// diagonal leaf in solve order, row-major: conj(Q) stored like Q (y = Q^H s) for
+// L, R^{-1} for U.
 struct HluDfPlan {
-  std::vector<HluDfChunk> chunks;  // D + 1, the last one a sentinel
-  std::vector<HluDfRow> rows, erows;  // late and early row lists
-  std::vector<HluDfCol> cols;
-  std::vector<int64_t> slot;       // per leaf, -1 for none
-  int64_t nslot = 0;               // complex values in each of pre and fin
+  std::vector<HluDfItem> items;
+  std::vector<HluDfColumn> columns;
+  std::vector<HluDfDot> dots;
+  std::vector<HluDfInner> inner;
+  std::vector<HluDfChunk> chunks;
+  std::vector<HluDfSuper> supers;
+  std::vector<int32_t> need;  // 3 per super
   std::vector<cd> diag;
-  int D() const { return (int)chunks.size() - 1; }
+  int64_t nt = 0, msize = 0;
+  bool lower = false;
+  int D() const { return (int)supers.size(); }
+  std::vector<HluDfPanel> panels(int precision) const;
 };
+
+// Row boundaries of the supers: the cluster-tree nodes of at most
+// hlu_df_super(precision) rows whose parents are larger; ascending, 0 to N.
+std::vector<int64_t> hlu_df_cuts(const HTree& tree, int precision);
 
 // False (with the reason) when the factor does not have the dataflow form's
 // structure: diagonal leaves that do not tile [0, N) or exceed 32 rows, a leaf
-// that is not aligned with them or not below the diagonal in solve order, a
-// rank above 32, a zero pivot. The sweep then runs on launch_hlu_sweep.
-// elem_bytes: size of one factor element (16 complex FP64, 8 complex FP32),
-// for the staging offsets of the late entries.
-bool hlu_df_plan(const FlatFactor& f, int64_t N, int elem_bytes, HluDfPlan& p, std::string* why);
+// that is not aligned with them and the cuts or not below the diagonal in solve
+// order, a rank above 32, a zero pivot. The sweep then runs on launch_hlu_sweep.
+bool hlu_df_plan(const FlatFactor& f, int64_t N, const std::vector<int64_t>& cuts, HluDfPlan& p,
+                 std::string* why);
 
 }  // namespace bemgpu

@@ -150,9 +150,9 @@ bool hlu_gpu_plan(const HTree& tree, const Layout& L, int64_t kc, HluProgram& P,
                   std::string* why);
 
 // The dataflow sweeps' plan without the apply matrices (those are written by
-// the QR tasks at the offsets `moff` of the plan); false as hlu_df_plan.
-bool hlu_df_plan_structure(const FlatFactor& f, int64_t N, int elem_bytes, HluDfPlan& p,
-                           std::string* why);
+// the QR tasks at the offsets `aoff` of the plan's chunks); false as hlu_df_plan.
+bool hlu_df_plan_structure(const FlatFactor& f, int64_t N, const std::vector<int64_t>& cuts,
+                           HluDfPlan& p, std::string* why);
 
 struct HluExecArgs {
   int precision;                 // 0 complex FP64, 1 complex FP32 (FP32 arithmetic)

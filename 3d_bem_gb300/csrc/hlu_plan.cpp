@@ -900,21 +900,20 @@ class Planner {
     // the sweep plans' chunk offsets must equal this layout
     HluDfPlan pl, pu;
     std::string w;
-    const bool okl = hlu_df_plan_structure(P_.L, L_.N, 8, pl, &w);
-    const bool oku = okl && hlu_df_plan_structure(P_.U, L_.N, 8, pu, &w);
+    const std::vector<int64_t> cuts = hlu_df_cuts(t_, 1);
+    const bool okl = hlu_df_plan_structure(P_.L, L_.N, cuts, pl, &w);
+    const bool oku = okl && hlu_df_plan_structure(P_.U, L_.N, cuts, pu, &w);
     P_.df_ok = okl && oku;
     P_.df_why = w;
     if (!P_.df_ok) return;
-    for (int i = 0; i < pl.D(); i++) {
-      const int64_t o = leaf_of_[pl.chunks[i].r0];
-      if (qh_base_ + pl.chunks[i].moff != qh_off_[o])
-        throw std::runtime_error("lower sweep apply matrices out of place");
-    }
-    for (int i = 0; i < pu.D(); i++) {
-      const int64_t o = leaf_of_[pu.chunks[i].r0];
-      if (rinv_base_ + pu.chunks[i].moff != rinv_off_[o])
-        throw std::runtime_error("upper sweep apply matrices out of place");
-    }
+    for (const HluDfSuper& u : pl.supers)
+      for (int i = u.chunk_beg; i < u.chunk_end; i++)
+        if (qh_base_ + pl.chunks[i].aoff != qh_off_[leaf_of_[u.r0 + pl.chunks[i].r0]])
+          throw std::runtime_error("lower sweep apply matrices out of place");
+    for (const HluDfSuper& u : pu.supers)
+      for (int i = u.chunk_beg; i < u.chunk_end; i++)
+        if (rinv_base_ + pu.chunks[i].aoff != rinv_off_[leaf_of_[u.r0 + pu.chunks[i].r0]])
+          throw std::runtime_error("upper sweep apply matrices out of place");
   }
 
   // ---- order, dependencies, statistics, bounds ----

@@ -103,3 +103,33 @@ def test_products_at_tile_edges(bem, meshes, body, n, leaf):
                     err = torch.linalg.vector_norm(y - want, dim=1)
                     assert (err < tol * torch.linalg.vector_norm(want, dim=1)).all(), (R, arith, acc)
         s.close()
+
+
+@pytest.mark.parametrize("n,leaf,rank", [(12, 32, 2), (36, 32, 2), (300, 32, 2), (701, 20, 3),
+                                         (1283, 32, 2), (2600, 28, 5)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_substitution_at_super_edges(bem, meshes, orc, n, leaf, rank, precision):
+    """The dataflow sweeps against the oracle's leaf-by-leaf solves with one
+    diagonal block, several, ragged ones, and 1 to 11 right-hand sides (1, 2, 4
+    and 8 per pass, remainders). FP64 factors: rounding times the conditioning of
+    the diagonal blocks, 1e-11; FP32 factors: 1e-4, as for the other FP32 sweep
+    test. One right-hand side does not depend on the others beside it."""
+    tri = meshes.box(n_target=max(n, 12), seed=3)[:n]
+    n = tri.shape[0]
+    s = bem.Solver(aca_tol=1e-6, precision=precision, precond_rank=rank, leaf_size=leaf)
+    s.set_mesh(tri)
+    s.set_bc(np.zeros(n), np.ones(n))
+    s.assemble(300.0)
+    s.hlu_build()
+    assert s.hlu_sweep_kind() == 1
+    Ll, Ld, _ = s.hlu_export(0)
+    Ul, Ud, _ = s.hlu_export(1)
+    rng = np.random.default_rng(n)
+    B = rng.standard_normal((n, 11)) + 1j * rng.standard_normal((n, 11))
+    ref = np.stack([orc.upper_solve(n, Ul, Ud, orc.lower_solve(n, Ll, Ld, B[:, q]))
+                    for q in range(11)], axis=1)
+    for R in (1, 2, 3, 5, 8, 11):
+        X = s.hlu_solve(B[:, :R])
+        for q in range(R):
+            assert rel(X[:, q], ref[:, q]) < (1e-11, 1e-4)[precision], (R, q)
+    s.close()
