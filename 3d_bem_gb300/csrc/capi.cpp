@@ -2808,9 +2808,10 @@ void field_dev(bem_handle* h, double freq, const double* pts, int64_t M, const d
     h->field_src.assign(src, src + 5 * nsrc);
     h->dFsrc.upload(h->field_src, s);
   }
-  const size_t fes = prec == 1 ? sizeof(FieldElemF) : sizeof(FieldElem);
-  h->dFe.ensure((size_t)N * fes);
-  h->dFcoef.ensure((size_t)N * R * (prec == 1 ? sizeof(FieldCoefF) : sizeof(FieldCoef)));
+  const size_t fes = prec == 1 ? field_pairs(N) * sizeof(FieldPairF) : N * sizeof(FieldElem);
+  h->dFe.ensure(fes);
+  h->dFcoef.ensure((size_t)R * (prec == 1 ? field_pairs(N) * sizeof(FieldCoefPairF)
+                                          : N * sizeof(FieldCoef)));
   const int S = field_split(h, M, R);
   // with an impedance plane the reflected elements add a second set of S
   // partial sums with the same coefficients (:2305-2311)
@@ -2821,7 +2822,7 @@ void field_dev(bem_handle* h, double freq, const double* pts, int64_t M, const d
   h->launches += launch_field_sum(h->dFe.p, h->dFcoef.p, N, (int)R, pts, M, k, prec, S,
                                   h->dFpart.p, s);
   if (h->have_plane) {
-    h->dFeR.ensure((size_t)N * fes);
+    h->dFeR.ensure(fes);
     h->launches += launch_field_prep(h->dEr.p, nullptr, N, nullptr, nullptr, 0, prec, h->dFeR.p,
                                      nullptr, s);
     h->launches += launch_field_sum(h->dFeR.p, h->dFcoef.p, N, (int)R, pts, M, k, prec,

@@ -13,8 +13,7 @@
 // centroids (p - c_j keeps ~7 digits, the rule points are offsets from c_j),
 // exp(ikr) from the hardware sin / cos after an exact reduction of
 // k r / (2 pi) to [-1/2, 1/2] (absolute error ~4e-7 on [-pi, pi]), per-tile
-// sums in FP32
-// folded into FP64 accumulators every FIELD_TILE elements. Precision 0: the
+// sums in FP32 folded into FP64 accumulators every 128 (32) elements. Precision 0: the
 // same sum in FP64.
 #include "field.h"
 
@@ -57,28 +56,29 @@ __global__ void field_prep_kernel(const Elem* __restrict__ E, const int64_t* __r
   if (j >= N) return;
   const Elem& e = E[j];
   if (precision == 1) {
-    FieldElemF f;
+    // the element's half of its pair; the last one of an odd count writes both
+    float* f = reinterpret_cast<float*>(static_cast<FieldPairF*>(fe) + (j >> 1));
+    float v[30];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       const float hi = (float)e.c[d];
-      f.c_hi[d] = hi;
-      f.c_lo[d] = (float)(e.c[d] - (double)hi);
-      f.nrm[d] = (float)e.nrm[d];
+      v[d] = -hi;
+      v[3 + d] = -(float)(e.c[d] - (double)hi);
+      v[27 + d] = (float)e.nrm[d];
     }
 #pragma unroll
     for (int i = 0; i < 7; i++) {
       const double a1 = cR7x1[i], a2 = cR7x2[i], a3 = 1.0 - a2 - a1;
-      double on = 0.0;
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const double o = (a1 * e.n1[d] + a2 * e.n2[d] + a3 * e.n3[d]) - e.c[d];
-        f.q[3 * i + d] = (float)o;
-        on += o * e.nrm[d];
-      }
-      f.qn[i] = (float)on;
+      for (int d = 0; d < 3; d++)
+        v[6 + 3 * i + d] = -(float)((a1 * e.n1[d] + a2 * e.n2[d] + a3 * e.n3[d]) - e.c[d]);
     }
-    f.pad[0] = f.pad[1] = f.pad[2] = 0.0f;
-    static_cast<FieldElemF*>(fe)[j] = f;
+    const bool alone = j == N - 1 && !(j & 1);
+#pragma unroll
+    for (int i = 0; i < 30; i++) {
+      f[2 * i + (j & 1)] = v[i];
+      if (alone) f[2 * i + 1] = v[i];
+    }
   } else {
     FieldElem f;
     double rho = 0.0;
@@ -108,10 +108,14 @@ __global__ void field_prep_kernel(const Elem* __restrict__ E, const int64_t* __r
   for (int r = 0; r < R; r++) {
     const double2 p = phi[(int64_t)r * N + cj], dp = dphi[(int64_t)r * N + cj];
     if (precision == 1) {
-      FieldCoefF c;
-      c.a = make_float2((float)(A * p.x), (float)(A * p.y));
-      c.b = make_float2((float)(A * dp.x), (float)(A * dp.y));
-      static_cast<FieldCoefF*>(coef)[(int64_t)r * N + j] = c;
+      float* c = reinterpret_cast<float*>(static_cast<FieldCoefPairF*>(coef) +
+                                          (int64_t)r * ((N + 1) / 2) + (j >> 1));
+      const float v[4] = {(float)(A * p.x), (float)(A * p.y), (float)(A * dp.x), (float)(A * dp.y)};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        c[2 * i + (j & 1)] = v[i];
+        if (j == N - 1 && !(j & 1)) c[2 * i + 1] = 0.0f;
+      }
     } else {
       FieldCoef c;
       c.a = make_double2(A * p.x, A * p.y);
@@ -121,84 +125,144 @@ __global__ void field_prep_kernel(const Elem* __restrict__ E, const int64_t* __r
   }
 }
 
-// Columns r0 .. r0 + RB - 1, element chunk blockIdx.y.
+// Two FP32 values as one operand: an add, multiply or FMA of both takes one
+// issue slot (and twice the pipe cycles of a scalar one).
+struct P2 {
+  uint64_t v;
+};
+__device__ __forceinline__ P2 p2(float a, float b) {
+  P2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2(P2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ P2 add2(P2 a, P2 b) {
+  P2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ P2 mul2(P2 a, P2 b) {
+  P2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c) {
+  P2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Columns r0 .. r0 + RB - 1, element chunk blockIdx.y. Bound by the special
+// functions (rsqrt, sin and cos of every rule point, 8 cycles a warp each: 168 of
+// them per element) beside the FMA pipe (about as much); issue slots were the
+// limit with scalar arithmetic (258 per element, 86 % of the cycles), so two
+// elements go through every operation together. (p - q) . n is the same for all
+// points of an element's plane, and the radial part is summed as
+// sum w (cos, sin) / r^3 and k sum w (cos, sin) / r^2. 20,480 elements x 20,480
+// points, one column: 2.31 ms (3.07 ms with scalar arithmetic).
 template <int RB, int FIELD_PTS>
 __global__ void __launch_bounds__(FIELD_PTS)
-    field_sum32_kernel(const FieldElemF* __restrict__ fe, const FieldCoefF* __restrict__ coef,
-                       int64_t N, int64_t chunk, const double* __restrict__ pts, int64_t M,
+    field_sum32_kernel(const FieldPairF* __restrict__ fe, const FieldCoefPairF* __restrict__ coef,
+                       int64_t NP, int64_t chunk, const double* __restrict__ pts, int64_t M,
                        float k, float kc, int r0, int R, double2* __restrict__ partial) {
-  constexpr int FIELD_TILE = FIELD_PTS / 2;
-  __shared__ FieldElemF se[FIELD_TILE];
-  __shared__ FieldCoefF sc[RB][FIELD_TILE];
+  constexpr int TILE = FIELD_PTS / 4;  // pairs
+  __shared__ FieldPairF se[TILE];
+  __shared__ FieldCoefPairF sc[RB][TILE];
   const int64_t ip = (int64_t)blockIdx.x * FIELD_PTS + threadIdx.x;
   const int64_t e0 = (int64_t)blockIdx.y * chunk;
-  const int64_t e1 = min(N, e0 + chunk);
-  float ph[3] = {0.0f, 0.0f, 0.0f}, pl[3] = {0.0f, 0.0f, 0.0f};
-  if (ip < M) {
+  const int64_t e1 = min(NP, e0 + chunk);
+  P2 ph[3], pl[3];
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const double v = pts[3 * ip + d];
-      ph[d] = (float)v;
-      pl[d] = (float)(v - (double)ph[d]);
-    }
+  for (int d = 0; d < 3; d++) {
+    const double v = ip < M ? pts[3 * ip + d] : 0.0;
+    const float hi = (float)v, lo = (float)(v - (double)hi);
+    ph[d] = p2(hi, hi);
+    pl[d] = p2(lo, lo);
   }
+  const P2 kc2 = p2(kc, kc), k2 = p2(k, k), nk2 = p2(-k, -k), minus = p2(-1.0f, -1.0f);
+  const float magic = 12582912.0f;  // 1.5 2^23: adding it rounds to an integer
+  const P2 mg = p2(magic, magic), nmg = p2(-magic, -magic);
+  const P2 twopi = p2(6.28318530717959f, 6.28318530717959f);
   double ax[RB], ay[RB];
 #pragma unroll
   for (int r = 0; r < RB; r++) ax[r] = ay[r] = 0.0;
-  for (int64_t t0 = e0; t0 < e1; t0 += FIELD_TILE) {
-    const int nt = (int)min((int64_t)FIELD_TILE, e1 - t0);
+  for (int64_t t0 = e0; t0 < e1; t0 += TILE) {
+    const int nt = (int)min((int64_t)TILE, e1 - t0);
     __syncthreads();
     const float4* src = reinterpret_cast<const float4*>(fe + t0);
     float4* dst = reinterpret_cast<float4*>(se);
-    constexpr int PIECES = (int)(sizeof(FieldElemF) / sizeof(float4));
+    constexpr int PIECES = (int)(sizeof(FieldPairF) / sizeof(float4));
     for (int i = threadIdx.x; i < nt * PIECES; i += FIELD_PTS) dst[i] = src[i];
     for (int i = threadIdx.x; i < RB * nt; i += FIELD_PTS) {
       const int r = i / nt, j = i - r * nt;
-      sc[r][j] = coef[(int64_t)(r0 + r) * N + t0 + j];
+      sc[r][j] = coef[(int64_t)(r0 + r) * NP + t0 + j];
     }
     __syncthreads();
-    float tx[RB], ty[RB];
+    P2 tx[RB], ty[RB];
 #pragma unroll
-    for (int r = 0; r < RB; r++) tx[r] = ty[r] = 0.0f;
+    for (int r = 0; r < RB; r++) tx[r] = ty[r] = p2(0.0f, 0.0f);
     for (int j = 0; j < nt; j++) {
-      const FieldElemF& E = se[j];
-      const float dx = (ph[0] - E.c_hi[0]) + (pl[0] - E.c_lo[0]);
-      const float dy = (ph[1] - E.c_hi[1]) + (pl[1] - E.c_lo[1]);
-      const float dz = (ph[2] - E.c_hi[2]) + (pl[2] - E.c_lo[2]);
-      const float dn = dx * E.nrm[0] + dy * E.nrm[1] + dz * E.nrm[2];
-      float Lx = 0.0f, Ly = 0.0f, Mx = 0.0f, My = 0.0f;
+      const ulonglong2* E = reinterpret_cast<const ulonglong2*>(&se[j]);
+      P2 f[30];
+#pragma unroll
+      for (int i = 0; i < 15; i++) {
+        const ulonglong2 v = E[i];
+        f[2 * i].v = v.x;
+        f[2 * i + 1].v = v.y;
+      }
+      const P2 dx = add2(add2(ph[0], f[0]), add2(pl[0], f[3]));
+      const P2 dy = add2(add2(ph[1], f[1]), add2(pl[1], f[4]));
+      const P2 dz = add2(add2(ph[2], f[2]), add2(pl[2], f[5]));
+      const P2 dn = fma2(dx, f[27], fma2(dy, f[28], mul2(dz, f[29])));
+      const P2 zero = p2(0.0f, 0.0f);
+      P2 Lx = zero, Ly = zero, Ax = zero, Ay = zero, Bx = zero, By = zero;
 #pragma unroll
       for (int i = 0; i < 7; i++) {
-        const float rx = dx - E.q[3 * i], ry = dy - E.q[3 * i + 1], rz = dz - E.q[3 * i + 2];
-        const float rr = rx * rx + ry * ry + rz * rz;
-        const float ir = rsqrtf(rr);
-        const float r = rr * ir;
+        const P2 rx = add2(dx, f[6 + 3 * i]), ry = add2(dy, f[7 + 3 * i]), rz = add2(dz, f[8 + 3 * i]);
+        const P2 rr = fma2(rx, rx, fma2(ry, ry, mul2(rz, rz)));
+        const float2 q = f2(rr);
+        const P2 ir = p2(rsqrt_approx(q.x), rsqrt_approx(q.y));
         // exp(ikr): x = k r / (2 pi) reduced exactly to [-1/2, 1/2] (x - rint(x)
         // has no rounding), then the hardware sin / cos on 2 pi (x - rint(x))
-        const float x = kc * r;
-        const float xr = x - rintf(x);
-        float sn, cs;
-        __sincosf(6.28318530717959f * xr, &sn, &cs);
-        const float kr = k * r;
-        const float g0 = ir * cR7gf[i];  // w / (4 pi r)
-        Lx = fmaf(g0, cs, Lx);
-        Ly = fmaf(g0, sn, Ly);
-        // w dG/dr rnq = g0 (p - q_i) . n / r^2 (cos + kr sin, sin - kr cos)
-        const float tg = (dn - E.qn[i]) * (ir * ir * g0);
-        Mx = fmaf(tg, fmaf(kr, sn, cs), Mx);
-        My = fmaf(tg, fmaf(-kr, cs, sn), My);
+        const P2 x = mul2(kc2, mul2(rr, ir));
+        const P2 xr = mul2(fma2(add2(add2(x, mg), nmg), minus, x), twopi);
+        const float2 t = f2(xr);
+        const P2 cs = p2(__cosf(t.x), __cosf(t.y)), sn = p2(__sinf(t.x), __sinf(t.y));
+        const P2 g0 = mul2(ir, p2(cR7gf[i], cR7gf[i]));  // w / (4 pi r)
+        const P2 g1 = mul2(g0, ir), g2 = mul2(g1, ir);
+        Lx = fma2(g0, cs, Lx);
+        Ly = fma2(g0, sn, Ly);
+        Ax = fma2(g2, cs, Ax);
+        Ay = fma2(g2, sn, Ay);
+        Bx = fma2(g1, cs, Bx);
+        By = fma2(g1, sn, By);
       }
+      // w dG/dr rnq = (p - q) . n w / r^3 (cos + kr sin, sin - kr cos)
+      const P2 Mx = mul2(dn, fma2(k2, By, Ax)), My = mul2(dn, fma2(nk2, Bx, Ay));
+      const P2 nMy = mul2(My, minus), nLx = mul2(Lx, minus), nLy = mul2(Ly, minus);
 #pragma unroll
       for (int r = 0; r < RB; r++) {
-        const FieldCoefF c = sc[r][j];
-        tx[r] += (Mx * c.a.x - My * c.a.y) - (Lx * c.b.x - Ly * c.b.y);
-        ty[r] += (Mx * c.a.y + My * c.a.x) - (Lx * c.b.y + Ly * c.b.x);
+        const ulonglong2* C = reinterpret_cast<const ulonglong2*>(&sc[r][j]);
+        const ulonglong2 c0 = C[0], c1 = C[1];
+        const P2 cax{c0.x}, cay{c0.y}, cbx{c1.x}, cby{c1.y};
+        tx[r] = fma2(Mx, cax, fma2(nMy, cay, fma2(nLx, cbx, fma2(Ly, cby, tx[r]))));
+        ty[r] = fma2(Mx, cay, fma2(My, cax, fma2(nLx, cby, fma2(nLy, cbx, ty[r]))));
       }
     }
 #pragma unroll
     for (int r = 0; r < RB; r++) {
-      ax[r] += (double)tx[r];
-      ay[r] += (double)ty[r];
+      const float2 sx = f2(tx[r]), sy = f2(ty[r]);
+      ax[r] += (double)(sx.x + sx.y);
+      ay[r] += (double)(sy.x + sy.y);
     }
   }
   if (ip < M) {
@@ -401,8 +465,8 @@ void sum_pass(const void* fe, const void* coef, int64_t N, int R, const double* 
   if (precision == 1) {
     const double kc = k / (2.0 * 3.14159265358979323846);
     field_sum32_kernel<RB, PTS><<<grid, PTS, 0, s>>>(
-        static_cast<const FieldElemF*>(fe), static_cast<const FieldCoefF*>(coef), N, chunk, pts, M,
-        (float)k, (float)kc, r0, R, partial);
+        static_cast<const FieldPairF*>(fe), static_cast<const FieldCoefPairF*>(coef),
+        field_pairs(N), (chunk + 1) / 2, pts, M, (float)k, (float)kc, r0, R, partial);
   } else {
     field_sum64_kernel<RB, PTS><<<grid, PTS, 0, s>>>(static_cast<const FieldElem*>(fe),
                                                      static_cast<const FieldCoef*>(coef), N, chunk,

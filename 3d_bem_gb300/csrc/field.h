@@ -11,23 +11,23 @@
 
 namespace bemgpu {
 
-// FP32 element record of the mixed-precision field kernel (160 bytes):
-// centroid as two floats (c_hi + c_lo), the 7 rule points as offsets o_i from
-// the centroid, unit normal n, and n . o_i (so (p - q_i) . n costs one
-// subtraction per rule point).
-struct __align__(16) FieldElemF {
-  float c_hi[3], c_lo[3];
-  float q[21];
-  float nrm[3];
-  float qn[7];
-  float pad[3];
+// FP32 record of two consecutive elements for the mixed-precision field kernel
+// (240 bytes), every value as the pair (even element, odd element): the centroid
+// as two floats c_hi + c_lo and the 7 rule points as offsets from it, all
+// negated (p - q is an addition), and the unit normal. An odd last element is
+// paired with a copy of itself that has zero coefficients.
+struct __align__(16) FieldPairF {
+  float2 nc_hi[3], nc_lo[3];
+  float2 nq[21];
+  float2 nrm[3];
 };
-static_assert(sizeof(FieldElemF) == 160, "FieldElemF is ten 16-byte pieces");
+static_assert(sizeof(FieldPairF) == 240, "FieldPairF is fifteen 16-byte pieces");
+inline int64_t field_pairs(int64_t N) { return (N + 1) / 2; }
 
-// Coefficients of one element and right-hand side: a = A phi, b = A dphi
-// (A the element area), complex.
-struct FieldCoefF {
-  float2 a, b;
+// Coefficients of the elements and right-hand sides: a = A phi, b = A dphi (A
+// the element area), complex; two elements at a time in FP32.
+struct __align__(16) FieldCoefPairF {
+  float2 ax, ay, bx, by;
 };
 struct FieldCoef {
   double2 a, b;
@@ -53,8 +53,8 @@ constexpr int FIELD_RB = 4;     // right-hand sides per pass
 
 // Element records and the coefficients of R columns: phi, dphi are N x R
 // complex FP64 in the caller's order, perm[j] the caller index of cluster-order
-// element j. fe: N FieldElemF (precision 1) or FieldElem (precision 0); coef:
-// R x N FieldCoefF or FieldCoef. R = 0: the records only (perm, phi, dphi,
+// element j. Precision 1: fe field_pairs(N) FieldPairF, coef R x field_pairs(N)
+// FieldCoefPairF; precision 0: fe N FieldElem, coef R x N FieldCoef. R = 0: the records only (perm, phi, dphi,
 // coef unused).
 int launch_field_prep(const Elem* E, const int64_t* perm, int64_t N, const double2* phi,
                       const double2* dphi, int R, int precision, void* fe, void* coef,
