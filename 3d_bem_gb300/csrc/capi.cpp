@@ -804,10 +804,10 @@ void ensure_gmres(bem_handle* h, int R) {
   g.sn.ensure((size_t)R * m);
   g.h.ensure((size_t)R * (m + 1));
   g.y.ensure((size_t)R * m);
-  g.cpart.ensure((size_t)nct * R * (m + 1));
-  // norm partials: one per partial-sum CTA, or one per 256 elements (the
+  g.cpart.ensure((size_t)krylov_partials(N, R, m));
+  // norm partials: one per partial-sum CTA, or one per 128 elements (the
   // fused Arnoldi update writes those)
-  g.npart.ensure((size_t)std::max<int64_t>(nct, (h->N + 255) / 256) * R);
+  g.npart.ensure((size_t)std::max<int64_t>(nct, (h->N + 127) / 128) * R);
   g.hnorm.ensure(R);
   g.st.ensure(R);
   g.hst.resize(R);

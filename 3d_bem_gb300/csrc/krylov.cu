@@ -21,6 +21,8 @@ namespace bemgpu {
 namespace {
 
 constexpr int DT = 256;
+constexpr int AT = 128;  // threads of the update kernel: N R / 256 CTAs left half the SMs idle
+                         // at N = 5,123, R = 4, and its FP64 work is what bounds it
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -80,7 +82,7 @@ __global__ void __launch_bounds__(DT) nrm_partial_kernel(const double2* __restri
   }
 }
 
-// Fused Arnoldi kernels: grid (ceil(N / DT), R), one right-hand side r per
+// Fused Arnoldi kernels: grid (ceil(N / AT), R), one right-hand side r per
 // blockIdx.y. Every CTA reduces the dot partials itself (one warp per q, lane
 // l sums partials l, l + 32, ... in order, fixed shuffle tree: the same sums
 // in every CTA), so no separate reduction launch sits between the passes.
@@ -88,12 +90,12 @@ __global__ void __launch_bounds__(DT) nrm_partial_kernel(const double2* __restri
 // w[r] -= sum_q h[r][q] V[q][r] with h reduced from the partials; CTA x = 0
 // writes h into the Hessenberg column. With norm_out, the CTA also writes the
 // squared norm of its updated slice of w to norm_out[blockIdx.x * R + r].
-__global__ void __launch_bounds__(DT) reduce_axpy_kernel(
+__global__ void __launch_bounds__(AT) reduce_axpy_kernel(
     const double2* __restrict__ partial, int nct, const double2* __restrict__ Vb,
     double2* __restrict__ w, int64_t N, int R, int nq, int m, int j, int first,
     const GmresState* __restrict__ st, double2* __restrict__ H, double* __restrict__ norm_out) {
   extern __shared__ double2 hs[];  // nq
-  __shared__ double red[DT / 32];
+  __shared__ double red[AT / 32];
   const int r = blockIdx.y;
   if (st[r].done) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -103,7 +105,7 @@ __global__ void __launch_bounds__(DT) reduce_axpy_kernel(
   // queue q by q on the warps
   const int64_t cstride = (int64_t)R * nq;
   if (nct >= 64) {
-    for (int q = warp; q < nq; q += DT / 32) {
+    for (int q = warp; q < nq; q += AT / 32) {
       double sx = 0, sy = 0;
       for (int c = lane; c < nct; c += 32) {
         const double2 v = partial[c * cstride + (int64_t)r * nq + q];
@@ -122,7 +124,7 @@ __global__ void __launch_bounds__(DT) reduce_axpy_kernel(
       }
     }
   } else {
-  for (int q = threadIdx.x; q < nq; q += DT) {
+  for (int q = threadIdx.x; q < nq; q += AT) {
     const double2* pq = partial + (int64_t)r * nq + q;
     double a0 = 0, a1 = 0, a2 = 0, a3 = 0, b0 = 0, b1 = 0, b2 = 0, b3 = 0;
     int c = 0;
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(DT) reduce_axpy_kernel(
   }
   }
   __syncthreads();
-  const int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x;
+  const int64_t i = (int64_t)blockIdx.x * AT + threadIdx.x;
   double n2 = 0;
   if (i < N) {
     double2 acc = w[(int64_t)r * N + i];
@@ -166,66 +168,75 @@ __global__ void __launch_bounds__(DT) reduce_axpy_kernel(
     __syncthreads();
     if (threadIdx.x == 0) {
       double t = 0;
-      for (int q = 0; q < DT / 32; q++) t += red[q];
+      for (int q = 0; q < AT / 32; q++) t += red[q];
       norm_out[(int64_t)blockIdx.x * R + r] = t;
     }
   }
 }
 
 // Finish Arnoldi step j and write V[j + 1] = w / ||w||: every CTA sums the
-// nct norm partials (warp 0, fixed order) for its scaling; CTA x = 0 also
-// applies the Givens rotations and updates the state (as finish_step_kernel).
+// nct norm partials (warp 0, fixed order) for its scaling; CTA x = 0 also forms
+// the new Givens rotation and updates the state. The column of H stays
+// unrotated: the rotations' product turns its entries 0 .. j into one number,
+// sum_i p_i H_i, p the last row of the product so far (p <- (-conj(s) p, c) per
+// step). That is a dot product of one warp, where applying j rotations one
+// after the other was a chain of 2 j dependent loads and complex products
+// (18 us at j = 16, 40 us at j = 70). krylov_update rotates the columns, all at
+// once, when the cycle ends.
 // A right-hand side that converges at this step may or may not get its next
 // vector written; it is not used afterwards.
 __global__ void __launch_bounds__(DT) finish_scale_kernel(
     const double* __restrict__ partial, int nct, int R, int m, int j, double tol,
     GmresState* __restrict__ st, double2* __restrict__ H, double2* __restrict__ g,
-    double2* __restrict__ cs, double2* __restrict__ sn, double* __restrict__ hnorm,
-    const double2* __restrict__ w, double2* __restrict__ vnext, int64_t N) {
+    double2* __restrict__ cs, double2* __restrict__ sn, double2* __restrict__ prow,
+    double* __restrict__ hnorm, const double2* __restrict__ w, double2* __restrict__ vnext,
+    int64_t N) {
   __shared__ double hn_s;
   const int r = blockIdx.y, lane = threadIdx.x & 31;
   GmresState s = st[r];
   if (s.done) return;
   if (threadIdx.x < 32) {
+    double2* Hc = H + ((int64_t)r * m + j) * (m + 1);
+    double2* pr = prow + (int64_t)r * (m + 1);
+    double2 a = make_double2(0.0, 0.0);
+    if (blockIdx.x == 0) {
+      for (int q = lane; q <= j; q += 32)
+        a = cadd(a, cmul(j == 0 ? make_double2(1.0, 0.0) : pr[q], Hc[q]));
+    }
     double n2 = 0;
     for (int c = lane; c < nct; c += 32) n2 += partial[(int64_t)c * R + r];
     n2 = warp_sum(n2);
-    if (lane == 0) {
-      const double hn = sqrt(n2);
-      hn_s = hn;
-      if (blockIdx.x == 0) {
+    const double hn = sqrt(n2);
+    if (lane == 0) hn_s = hn;
+    if (blockIdx.x == 0) {
+      a.x = warp_sum(a.x);
+      a.y = warp_sum(a.y);
+      const double2 b = make_double2(hn, 0.0);
+      const double aa = sqrt(cabs2(a)), rho = sqrt(cabs2(a) + n2);
+      double2 c, sv;
+      if (aa == 0.0) {
+        c = make_double2(0, 0);
+        sv = make_double2(1, 0);
+      } else {
+        c = make_double2(aa / rho, 0.0);
+        sv = cscale(1.0 / (aa * rho), cmul(a, cconj(b)));
+      }
+      const double2 ns = cscale(-1.0, cconj(sv));
+      for (int q = lane; q <= j; q += 32)
+        pr[q] = cmul(ns, j == 0 ? make_double2(1.0, 0.0) : pr[q]);
+      if (lane == 0) {
+        pr[j + 1] = c;
         hnorm[r] = hn;
-        double2* Hc = H + ((int64_t)r * m + j) * (m + 1);
-        double2* cr = cs + (int64_t)r * m;
-        double2* sr = sn + (int64_t)r * m;
+        Hc[j + 1] = b;
+        cs[(int64_t)r * m + j] = c;
+        sn[(int64_t)r * m + j] = sv;
         double2* gr = g + (int64_t)r * (m + 1);
-        Hc[j + 1] = make_double2(hn, 0.0);
-        for (int q = 0; q < j; q++) {
-          double2 a = Hc[q], b = Hc[q + 1];
-          Hc[q] = cadd(cmul(cr[q], a), cmul(sr[q], b));
-          Hc[q + 1] = cadd(cscale(-1.0, cmul(cconj(sr[q]), a)), cmul(cr[q], b));
-        }
-        double2 a = Hc[j], b = Hc[j + 1];
-        double aa = sqrt(cabs2(a));
-        double rho = sqrt(cabs2(a) + cabs2(b));
-        double2 c, sv;
-        if (aa == 0.0) {
-          c = make_double2(0, 0);
-          sv = make_double2(1, 0);
-        } else {
-          c = make_double2(aa / rho, 0.0);
-          sv = cscale(1.0 / (aa * rho), cmul(a, cconj(b)));
-        }
-        cr[j] = c;
-        sr[j] = sv;
-        Hc[j] = cadd(cmul(c, a), cmul(sv, b));
-        Hc[j + 1] = make_double2(0, 0);
-        double2 gj = gr[j];
-        gr[j + 1] = cscale(-1.0, cmul(cconj(sv), gj));
+        const double2 gj = gr[j], gn = cmul(ns, gj);
+        gr[j + 1] = gn;
         gr[j] = cmul(c, gj);
         s.jcount = j + 1;
         s.iters += 1;
-        s.resid = sqrt(cabs2(gr[j + 1])) / s.bnorm;
+        s.resid = sqrt(cabs2(gn)) / s.bnorm;
         if (s.resid < tol || hn == 0.0) s.done = 1;
         st[r] = s;
       }
@@ -239,20 +250,68 @@ __global__ void __launch_bounds__(DT) finish_scale_kernel(
   vnext[(int64_t)r * N + i] = hn > 0 ? cscale(1.0 / hn, v) : make_double2(0, 0);
 }
 
-// One thread per RHS: solve the jcount x jcount triangular system H y = g.
-__global__ void trisolve_kernel(int R, int m, const GmresState* __restrict__ st,
-                                const double2* __restrict__ H, const double2* __restrict__ g,
-                                double2* __restrict__ y) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
+// One CTA per RHS: the Givens rotations on the columns of H (a thread per
+// column; columns are independent), then the jcount x jcount triangular system
+// H y = g by columns: y_q from the reciprocal of the diagonal, g -= y_q H_q with
+// the next column already loaded. One thread per RHS took 890 us at 130 steps.
+__global__ void __launch_bounds__(DT) trisolve_kernel(int R, int m,
+                                                      const GmresState* __restrict__ st,
+                                                      double2* __restrict__ H,
+                                                      double2* g, const double2* __restrict__ cs,
+                                                      const double2* __restrict__ sn, double2* y,
+                                                      int shared) {
+  extern __shared__ double2 sh[];
+  const int r = blockIdx.x;
+  // right-hand side and reciprocals of the diagonal: in shared memory, or for
+  // very long cycles in place of g and y
+  double2* gs = shared ? sh : g + (int64_t)r * (m + 1);
+  double2* inv = shared ? sh + m : y + (int64_t)r * m;
   const int kk = st[r].jcount;
-  double2* yr = y + (int64_t)r * m;
-  for (int q = kk - 1; q >= 0; q--) {
-    double2 s = g[(int64_t)r * (m + 1) + q];
-    for (int t = q + 1; t < kk; t++) s = csub(s, cmul(H[((int64_t)r * m + t) * (m + 1) + q], yr[t]));
-    yr[q] = cdiv(s, H[((int64_t)r * m + q) * (m + 1) + q]);
+  double2* Hr = H + (int64_t)r * m * (m + 1);
+  const double2* cr = cs + (int64_t)r * m;
+  const double2* sr = sn + (int64_t)r * m;
+  for (int t = threadIdx.x; t < kk; t += DT) {
+    double2* Hc = Hr + (int64_t)t * (m + 1);
+    double2 a = Hc[0];
+#pragma unroll 4
+    for (int q = 0; q <= t; q++) {
+      const double2 b = Hc[q + 1], c = cr[q], s = sr[q];
+      const double2 top = cadd(cmul(c, a), cmul(s, b));
+      a = cadd(cscale(-1.0, cmul(cconj(s), a)), cmul(c, b));
+      Hc[q] = top;
+      if (q == t) inv[t] = cdiv(make_double2(1.0, 0.0), top);
+    }
+    gs[t] = g[(int64_t)r * (m + 1) + t];
   }
-  for (int q = kk; q < m; q++) yr[q] = make_double2(0, 0);
+  __syncthreads();  // the CTA's own writes of H are read below
+  double2* yr = y + (int64_t)r * m;
+  for (int q = kk + threadIdx.x; q < m; q += DT) yr[q] = make_double2(0, 0);
+  constexpr int PF = 2;  // rows a thread covers: up to 512 columns without a loop
+  double2 h[PF];
+  const auto load = [&](int q) {
+#pragma unroll
+    for (int p = 0; p < PF; p++) {
+      const int i = threadIdx.x + p * DT;
+      h[p] = q > 0 && i < q ? Hr[(int64_t)q * (m + 1) + i] : make_double2(0, 0);
+    }
+  };
+  load(kk - 1);
+  for (int q = kk - 1; q >= 0; q--) {
+    const double2 yq = cmul(gs[q], inv[q]);
+    double2 cur[PF];
+#pragma unroll
+    for (int p = 0; p < PF; p++) cur[p] = h[p];
+    load(q - 1);
+#pragma unroll
+    for (int p = 0; p < PF; p++) {
+      const int i = threadIdx.x + p * DT;
+      if (i < q) gs[i] = csub(gs[i], cmul(cur[p], yq));
+    }
+    for (int i = threadIdx.x + PF * DT; i < q; i += DT)
+      gs[i] = csub(gs[i], cmul(Hr[(int64_t)q * (m + 1) + i], yq));
+    __syncthreads();
+    if (threadIdx.x == 0) yr[q] = yq;
+  }
 }
 
 // x[r] += sum_q y[r][q] V[q][r]
@@ -325,31 +384,46 @@ __global__ void __launch_bounds__(DT) copy_scale_kernel(const double2* __restric
 
 }  // namespace
 
-// CTAs of the partial-sum kernels: one per 128 elements, at most 4 per SM
-// (with 5 CTAs at N = 20,480 the Arnoldi dots ran at ~160 GB/s)
+// CTAs of the norm partials: one per 128 elements, at most 4 per SM
 int krylov_num_ctas(int64_t N) {
   int64_t c = (N + 127) / 128;
   return (int)std::max<int64_t>(1, std::min<int64_t>(c, 608));
+}
+
+// Chunks of `tasks` dot products over N elements: warps for every SM while the
+// basis is short (up to one chunk per 128 elements), one per 1,024 elements when
+// it is long -- every CTA of the update kernel adds up the partials of all
+// chunks, which took a third of it at 41 chunks and 70 vectors (N = 5,123).
+int krylov_dot_chunks(int64_t N, int64_t tasks) {
+  const int64_t want = (2432 + tasks - 1) / tasks;
+  return (int)std::max<int64_t>(
+      1, std::min<int64_t>(std::max<int64_t>(want, (N + 1023) / 1024), (N + 127) / 128));
+}
+// complex values the partial dot products of any step take
+int64_t krylov_partials(int64_t N, int R, int m) {
+  const int64_t t = (int64_t)R * (m + 1);
+  return (N + 1023) / 1024 * t + 2432 + t;
 }
 
 // CGS2 step j in five launches: dot partials, reduction + update (twice; the
 // second also takes the norm partials of w), then the Givens step + scaling
 int krylov_orthogonalize(const KrylovArgs& a, int j, cudaStream_t s) {
   const int nq = j + 1;
-  const int nct = krylov_num_ctas(a.N);
+  const int nct = krylov_dot_chunks(a.N, (int64_t)nq * a.R);
   const int64_t chunk = (a.N + nct - 1) / nct;
   const dim3 g((unsigned)((a.N + DT - 1) / DT), (unsigned)a.R);
+  const dim3 ga((unsigned)((a.N + AT - 1) / AT), (unsigned)a.R);
   const size_t hsm = (size_t)nq * sizeof(double2);
   // task groups: about two (q, r) dot products per warp
   const int tg = std::max(1, std::min(128, (nq * a.R + 2 * (DT / 32) - 1) / (2 * (DT / 32))));
   for (int pass = 0; pass < 2; pass++) {
     dot_partial_kernel<<<dim3((unsigned)nct, (unsigned)tg), DT, 0, s>>>(a.Vb, a.w, a.N, a.R, nq,
                                                                         chunk, a.st, a.cpart);
-    reduce_axpy_kernel<<<g, DT, hsm, s>>>(a.cpart, nct, a.Vb, a.w, a.N, a.R, nq, a.m, j,
+    reduce_axpy_kernel<<<ga, AT, hsm, s>>>(a.cpart, nct, a.Vb, a.w, a.N, a.R, nq, a.m, j,
                                           pass == 0, a.st, a.H, pass == 1 ? a.npart : nullptr);
   }
-  finish_scale_kernel<<<g, DT, 0, s>>>(a.npart, (int)g.x, a.R, a.m, j, a.tol, a.st, a.H, a.g,
-                                       a.cs, a.sn, a.hnorm, a.w,
+  finish_scale_kernel<<<g, DT, 0, s>>>(a.npart, (int)ga.x, a.R, a.m, j, a.tol, a.st, a.H, a.g,
+                                       a.cs, a.sn, a.h, a.hnorm, a.w,
                                        a.Vb + (int64_t)(j + 1) * a.R * a.N, a.N);
   return 5;
 }
@@ -381,7 +455,9 @@ void krylov_residual(const double2* b, double2* w, int64_t n, cudaStream_t s) {
 }
 
 void krylov_update(const KrylovArgs& a, cudaStream_t s) {
-  trisolve_kernel<<<(a.R + 31) / 32, 32, 0, s>>>(a.R, a.m, a.st, a.H, a.g, a.y);
+  const int sh = a.m <= 1536;  // 48 KiB
+  trisolve_kernel<<<a.R, DT, sh ? 2 * (size_t)a.m * sizeof(double2) : 0, s>>>(
+      a.R, a.m, a.st, a.H, a.g, a.cs, a.sn, a.y, sh);
   dim3 g((unsigned)((a.N + DT - 1) / DT), (unsigned)a.R);
   update_x_kernel<<<g, DT, 0, s>>>(a.Vb, a.x, a.N, a.R, a.m, a.y, a.st);
 }

@@ -23,19 +23,20 @@ struct KrylovArgs {
   double2* Vb;     // (m+1) x R x N basis
   double2* w;      // R x N work vector (operator output)
   double2* x;      // R x N solution
-  double2* H;      // R x m x (m+1) Hessenberg columns
+  double2* H;      // R x m x (m+1) Hessenberg columns (rotated by krylov_update)
   double2* g;      // R x (m+1)
   double2* cs;     // R x m
   double2* sn;     // R x m
-  double2* h;      // R x (m+1) projection coefficients
+  double2* h;      // R x (m+1) last row of the rotations' product
   double2* y;      // R x m
-  double2* cpart;  // nct x R x (m+1) partial dots
+  double2* cpart;  // partial dots (krylov_partials)
   double* npart;   // nct x R partial norms
   double* hnorm;   // R
   GmresState* st;  // R
 };
 
 int krylov_num_ctas(int64_t N);
+int64_t krylov_partials(int64_t N, int R, int m);  // size of cpart
 // one CGS2 Arnoldi step j on a.w; returns the kernels launched
 int krylov_orthogonalize(const KrylovArgs& a, int j, cudaStream_t s);
 void krylov_restart(const KrylovArgs& a, int init, cudaStream_t s);

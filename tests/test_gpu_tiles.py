@@ -133,3 +133,30 @@ def test_substitution_at_super_edges(bem, meshes, orc, n, leaf, rank, precision)
         for q in range(R):
             assert rel(X[:, q], ref[:, q]) < (1e-11, 1e-4)[precision], (R, q)
     s.close()
+
+
+@pytest.mark.parametrize("n", [12, 130, 1300])
+@pytest.mark.parametrize("restart", [4, 300, 1600])
+def test_gmres_cycles_against_dense(bem, meshes, n, restart):
+    """GMRES against the dense solve of the assembled matrix: short cycles, one
+    cycle, cycles too long for the triangular solve's shared memory; one and
+    three right-hand sides, one of them zero. The relative residual is below
+    1e-10, so the error is below that times the conditioning (~1e2): 1e-7."""
+    tri = meshes.box(n_target=max(n, 12), seed=9)[:n]
+    n = tri.shape[0]
+    s = bem.Solver(aca_tol=1e-7, gmres_tol=1e-10, gmres_restart=restart, gmres_maxit=1600)
+    s.set_mesh(tri)
+    s.set_bc(np.zeros(n), np.ones(n))
+    s.assemble(400.0)
+    A = s.dense(1)
+    rng = np.random.default_rng(n)
+    B = rng.standard_normal((n, 3)) + 1j * rng.standard_normal((n, 3))
+    B[:, 1] = 0.0
+    x1, i1 = s.gmres(B[:, 0])
+    x3, i3 = s.gmres(B)
+    ref = np.linalg.solve(A, B)
+    assert i1["status"] == 0 and i3["status"] == 0
+    assert rel(x1, ref[:, 0]) < 1e-7
+    assert rel(x3, ref) < 1e-7 and np.abs(x3[:, 1]).max() == 0.0
+    assert rel(A @ x1, B[:, 0]) < 1.1e-10
+    s.close()
