@@ -152,6 +152,12 @@ __device__ __forceinline__ void block_argmax(R v, int idx, Red<R>& red, R& best,
     }
 }
 
+// FP32 rule tables in shared memory
+struct AcaTables {
+  float x1[16], x2[16], w[16];
+  float cx1[SEL_CLASS_POINTS], cx2[SEL_CLASS_POINTS], cw[SEL_CLASS_POINTS];
+};
+
 // FP32 near-singular test on the two-float centroid difference; used only to
 // pick the rule inside ACA rows/columns (the near-field blocks use the host's
 // exact classification).
@@ -166,12 +172,22 @@ __device__ __forceinline__ bool near_pair32(const ElemF* __restrict__ EF, int64_
 // every pair of the plain path); kept out of line so the FP32 fast path does
 // not carry its registers
 __device__ __noinline__ double2 entry64(const AcaArgs& a, int64_t row, int64_t col) {
-  Ops o = ops_eval(a.E, row, col, a.k, a.near_r, c_rules);
+  Ops o;
+  const BcCoef& bc = a.bc[col];
+  if (a.EQ && row != col && !near_pair(a.E[row], a.E[col], a.near_r)) {
+    bool x, y;
+    needs(bc, a.which, x, y);
+    if (x && y) o = ops_regular_part<true, true>(a.E[row], a.E[col], a.EQ[col], a.k, c_rules);
+    else if (x) o = ops_regular_part<true, false>(a.E[row], a.E[col], a.EQ[col], a.k, c_rules);
+    else o = ops_regular_part<false, true>(a.E[row], a.E[col], a.EQ[col], a.k, c_rules);
+  } else {
+    o = ops_eval(a.E, row, col, a.k, a.near_r, c_rules);
+  }
   // impedance plane: the reflected element with the regular rule
   // (implicitPhiMatrixPlusReflected, boundaryelementsolver.cpp:2042-2050)
   if (a.Er) ops_add(o, ops_regular(a.E[row], a.Er[col], a.k, c_rules));
   double2 p, d;
-  substitute(o, row == col, a.bc[col], a.alpha, p, d);
+  substitute(o, row == col, bc, a.alpha, p, d);
   return a.which ? d : p;
 }
 
@@ -180,38 +196,12 @@ __device__ __noinline__ float2 entry64f(const AcaArgs& a, int64_t row, int64_t c
   return make_float2((float)v.x, (float)v.y);
 }
 
-// MODE 0: BEM entries; 2: BEM entries with an impedance plane (the
-// reflected element's operators added); 1: point-cloud test kernel.
+// Whole entries in FP64. MODE 0: BEM entries; 2: BEM entries with an impedance
+// plane (the reflected element's operators added); 1: point-cloud test kernel.
 template <int MODE, typename T>
 __device__ __forceinline__ T aca_entry(const AcaArgs& a, int64_t row, int64_t col) {
   if constexpr (MODE == 0 || MODE == 2) {
-    if constexpr (sizeof(T) == sizeof(float2)) {
-      // mixed precision: FP32 regular rule, FP64 singular / near-singular
-      if (row != col && !near_pair32(a.EF, row, col, a.near_r2f)) {
-        OpsF o;
-        if (a.rule_tab) {  // learned order: table bin of (d / e_max, k e_max)
-          float dx, dy, dz;
-          centroid_diff(a.EF[row], a.EF[col], dx, dy, dz);
-          const float em = a.EF[col].emax;
-          const float x = __logf(sqrtf(dx * dx + dy * dy + dz * dz) / em);
-          const float y = __logf(a.kf * em);
-          const int ix = min(max((int)floorf((x - a.tab_x0) / a.tab_dx), 0), ACA_TAB_N - 1);
-          const int iy = min(max((int)floorf((y - a.tab_y0) / a.tab_dy), 0), ACA_TAB_N - 1);
-          const int c = min((int)a.rule_tab[ix * ACA_TAB_N + iy], SEL_C - 1);
-          o = ops_rule32_pts(a.EF, row, col, a.kf, c_cls.off[c], c_cls.off[c + 1], c_cls.x1,
-                             c_cls.x2, c_cls.w);
-        } else {
-          o = ops_regular32(a.EF, row, col, a.kf, c_rules);
-        }
-        if constexpr (MODE == 2) ops_add(o, ops_regular32_pq(a.EF[row], a.EFr[col], a.kf, c_rules));
-        float2 p, d;
-        substitute32(o, a.bc[col], a.alphaf, p, d);
-        return a.which ? d : p;
-      }
-      return entry64f(a, row, col);
-    } else {
-      return entry64(a, row, col);
-    }
+    return entry64(a, row, col);
   } else {
     // point-cloud Helmholtz kernel of the reference's tests
     // (Tests/tests.h:30-42): exp(ikr)/(4 pi r), 1 at r = 0
@@ -231,11 +221,16 @@ __device__ __forceinline__ T aca_entry(const AcaArgs& a, int64_t row, int64_t co
 // FP32 regular rule over the points q, q + Q, ..; entries on the FP64 path
 // (singular / near-singular pairs, the complex-FP64 method, the point-cloud
 // kernel) come whole from lane 0. The Q shares sum to the entry (the BC
-// substitution of regular entries is linear in the operators).
-template <int MODE, typename T>
-__device__ __forceinline__ T aca_entry_part(const AcaArgs& a, int64_t row, int64_t col, int q,
-                                            int Q) {
+// substitution of regular entries is linear in the operators). NEED: 1 entries
+// of X = L + alpha Mt only, 2 of Y = M + alpha N only (rigid walls), 3 any.
+// Lanes that split an entry, or take different class rules, read different
+// points, which a constant-memory table serves one by one: they read the copy
+// in shared memory.
+template <int MODE, typename T, int NEED>
+__device__ __forceinline__ T aca_entry_part(const AcaArgs& a, const AcaTables& tab, int64_t row,
+                                            int64_t col, int q, int Q) {
   if constexpr ((MODE == 0 || MODE == 2) && sizeof(T) == sizeof(float2)) {
+    constexpr bool X = NEED & 1, Y = NEED & 2;
     if (row != col && !near_pair32(a.EF, row, col, a.near_r2f)) {
       const ElemF& P = a.EF[row];
       const ElemF& Qe = a.EF[col];
@@ -249,13 +244,15 @@ __device__ __forceinline__ T aca_entry_part(const AcaArgs& a, int64_t row, int64
         const int ix = min(max((int)floorf((x - a.tab_x0) / a.tab_dx), 0), ACA_TAB_N - 1);
         const int iy = min(max((int)floorf((y - a.tab_y0) / a.tab_dy), 0), ACA_TAB_N - 1);
         const int c = min((int)a.rule_tab[ix * ACA_TAB_N + iy], SEL_C - 1);
-        o = ops_pts32(P, Qe, a.kf, c_cls.x1, c_cls.x2, c_cls.w, c_cls.off[c] + q, c_cls.off[c + 1], Q);
+        o = ops_pts32<X, Y>(P, Qe, a.kf, tab.cx1, tab.cx2, tab.cw, c_cls.off[c] + q,
+                            c_cls.off[c + 1], Q);
+      } else if (Q == 1) {
+        o = ops_pts32<X, Y>(P, Qe, a.kf, c_rules.freg_x1, c_rules.freg_x2, c_rules.freg_w, 0, 16, 1);
       } else {
-        o = ops_pts32(P, Qe, a.kf, c_rules.freg_x1, c_rules.freg_x2, c_rules.freg_w, q, 16, Q);
+        o = ops_pts32<X, Y>(P, Qe, a.kf, tab.x1, tab.x2, tab.w, q, 16, Q);
       }
       if constexpr (MODE == 2)
-        ops_add(o, ops_pts32(P, a.EFr[col], a.kf, c_rules.freg_x1, c_rules.freg_x2,
-                             c_rules.freg_w, q, 16, Q));
+        ops_add(o, ops_pts32<X, Y>(P, a.EFr[col], a.kf, tab.x1, tab.x2, tab.w, q, 16, Q));
       float2 p, d;
       substitute32(o, a.bc[col], a.alphaf, p, d);
       return a.which ? d : p;
@@ -325,8 +322,8 @@ __device__ __forceinline__ T dot_strided(const T* p, int64_t stride, const T* c,
 }
 
 // dst[i] = A(r0+i, c0+ci) - sum_l U[:,l] (s_l V[l,ci])
-template <int MODE, typename T, int NT>
-__device__ void residual_col(const AcaArgs& a, const FarBlock& fb, const T* U, const T* V,
+template <int MODE, typename T, int NT, int NEED>
+__device__ void residual_col(const AcaArgs& a, const AcaTables& tab, const FarBlock& fb, const T* U, const T* V,
                              const T* S, int k, int ci, T* dst, T* coef) {
   for (int l = threadIdx.x; l < k; l += NT) coef[l] = cx_mul(S[l], V[(int64_t)l * fb.n + ci]);
   __syncthreads();
@@ -337,7 +334,7 @@ __device__ void residual_col(const AcaArgs& a, const FarBlock& fb, const T* U, c
     const int i = base + threadIdx.x / Q;
     T v{0, 0};
     if (i < fb.m)
-      v = cx_sub(aca_entry_part<MODE, T>(a, fb.r0 + i, fb.c0 + ci, q, Q),
+      v = cx_sub(aca_entry_part<MODE, T, NEED>(a, tab, fb.r0 + i, fb.c0 + ci, q, Q),
                  Q == 1 ? dot_strided(U + i, (int64_t)fb.m, coef, k)
                         : dot_strided_part(U + i, (int64_t)fb.m, coef, k, q, Q));
     for (int o = Q / 2; o > 0; o >>= 1) {
@@ -350,8 +347,8 @@ __device__ void residual_col(const AcaArgs& a, const FarBlock& fb, const T* U, c
 }
 
 // dst[j] = A(r0+ri, c0+j) - sum_l (U[ri,l] s_l) V[l,:]
-template <int MODE, typename T, int NT>
-__device__ void residual_row(const AcaArgs& a, const FarBlock& fb, const T* U, const T* V,
+template <int MODE, typename T, int NT, int NEED>
+__device__ void residual_row(const AcaArgs& a, const AcaTables& tab, const FarBlock& fb, const T* U, const T* V,
                              const T* S, int k, int ri, T* dst, T* coef) {
   for (int l = threadIdx.x; l < k; l += NT) coef[l] = cx_mul(U[(int64_t)l * fb.m + ri], S[l]);
   __syncthreads();
@@ -361,7 +358,7 @@ __device__ void residual_row(const AcaArgs& a, const FarBlock& fb, const T* U, c
     const int j = base + threadIdx.x / Q;
     T v{0, 0};
     if (j < fb.n)
-      v = cx_sub(aca_entry_part<MODE, T>(a, fb.r0 + ri, fb.c0 + j, q, Q),
+      v = cx_sub(aca_entry_part<MODE, T, NEED>(a, tab, fb.r0 + ri, fb.c0 + j, q, Q),
                  Q == 1 ? dot_strided(V + j, (int64_t)fb.n, coef, k)
                         : dot_strided_part(V + j, (int64_t)fb.n, coef, k, q, Q));
     for (int o = Q / 2; o > 0; o >>= 1) {
@@ -460,8 +457,22 @@ __device__ void norm_increment(const FarBlock& fb, const T* U, const T* V, const
 // (8 CTAs per SM), the 512-thread one at 64 (2 CTAs per SM). Despite the
 // spills this causes, the ACA phase at 20,480 elements drops from 24.4 ms
 // (uncapped, 168 registers, 3 CTAs per SM) to 19.7 ms.
-template <int MODE, typename T, int NT>
+template <int MODE, typename T, int NT, int NEED>
 __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) aca_kernel(AcaArgs a) {
+  __shared__ AcaTables tab;
+  if constexpr (MODE != 1 && sizeof(T) == sizeof(float2)) {
+    for (int i = threadIdx.x; i < 16; i += NT) {
+      tab.x1[i] = c_rules.freg_x1[i];
+      tab.x2[i] = c_rules.freg_x2[i];
+      tab.w[i] = c_rules.freg_w[i];
+    }
+    for (int i = threadIdx.x; i < SEL_CLASS_POINTS; i += NT) {
+      tab.cx1[i] = c_cls.x1[i];
+      tab.cx2[i] = c_cls.x2[i];
+      tab.cw[i] = c_cls.w[i];
+    }
+    __syncthreads();
+  }
   __shared__ T coef[ACA_MAX_KCAP];
   using R = typename Cx<T>::R;
   __shared__ Red<R> red;
@@ -483,7 +494,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) aca_kernel(AcaArgs a) {
   if (!a.extra) {
     // --- partialPivotACA ---
     int ci = (int)(pivot_hash(a.seed, (uint64_t)fb.id, 0) % (uint64_t)n);
-    residual_col<MODE, T, NT>(a, fb, U, V, S, 0, ci, U, coef);  // start column into slot 0
+    residual_col<MODE, T, NT, NEED>(a, tab, fb, U, V, S, 0, ci, U, coef);  // start column into slot 0
     int ri = -1;
     while (k < kmax) {
       const T* colv = U + (int64_t)(k > 0 ? k - 1 : 0) * m;
@@ -491,12 +502,12 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) aca_kernel(AcaArgs a) {
       argmax_abs<T, NT>(colv, m, k >= 1 ? ri : -1, red, cmax, ri);
       if (cmax <= tiny && k >= 1) break;
       T* rowv = V + (int64_t)k * n;
-      residual_row<MODE, T, NT>(a, fb, U, V, S, k, ri, rowv, coef);
+      residual_row<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ri, rowv, coef);
       R rmax;
       argmax_abs<T, NT>(rowv, n, -1, red, rmax, ci);
       if (rmax <= tiny && k >= 1) break;
       T* newcol = U + (int64_t)k * m;
-      residual_col<MODE, T, NT>(a, fb, U, V, S, k, ci, newcol, coef);
+      residual_col<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ci, newcol, coef);
       const T alpha = cx_recip(rowv[ci]);
       if (threadIdx.x == 0) S[k] = alpha;
       __syncthreads();
@@ -518,7 +529,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) aca_kernel(AcaArgs a) {
     const int npiv = a.piv_cnt[bi];
     for (int p = 0; p < npiv && k < kmax; p++) {
       int ri = piv[2 * p], ci = piv[2 * p + 1];
-      const T pivv = aca_entry_part<MODE, T>(a, fb.r0 + ri, fb.c0 + ci, 0, 1);
+      const T pivv = aca_entry_part<MODE, T, NEED>(a, tab, fb.r0 + ri, fb.c0 + ci, 0, 1);
       const R pabs2 = mag2(pivv);
       if (sqrt(pabs2) < tiny) continue;
       // approximation already good at the seed?
@@ -529,7 +540,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) aca_kernel(AcaArgs a) {
         approx.y += t.y;
       }
       if (sqrt(mag2(cx_sub(pivv, approx)) / pabs2) < tol) continue;
-      residual_col<MODE, T, NT>(a, fb, U, V, S, k, ci, U + (int64_t)k * m, coef);
+      residual_col<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ci, U + (int64_t)k * m, coef);
       bool first = true;
       while (k < kmax) {
         const T* colv = first ? U + (int64_t)k * m : U + (int64_t)(k - 1) * m;
@@ -538,12 +549,12 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) aca_kernel(AcaArgs a) {
         first = false;
         if (cmax <= tiny && k >= 1) break;
         T* rowv = V + (int64_t)k * n;
-        residual_row<MODE, T, NT>(a, fb, U, V, S, k, ri, rowv, coef);
+        residual_row<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ri, rowv, coef);
         R rmax;
         argmax_abs<T, NT>(rowv, n, -1, red, rmax, ci);
         if (rmax <= tiny && k >= 1) break;
         T* newcol = U + (int64_t)k * m;
-        residual_col<MODE, T, NT>(a, fb, U, V, S, k, ci, newcol, coef);
+        residual_col<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ci, newcol, coef);
         const T alpha = cx_recip(rowv[ci]);
         if (threadIdx.x == 0) S[k] = alpha;
         __syncthreads();
@@ -579,13 +590,15 @@ void launch_nt(const AcaArgs& a, cudaStream_t s) {
   const unsigned g = (unsigned)a.nfar;
   const bool plane = a.mode == 0 && a.Er != nullptr;
   if (a.precision == 0) {
-    if (plane) aca_kernel<2, double2, NT><<<g, NT, 0, s>>>(a);
-    else if (a.mode == 0) aca_kernel<0, double2, NT><<<g, NT, 0, s>>>(a);
-    else aca_kernel<1, double2, NT><<<g, NT, 0, s>>>(a);
+    if (plane) aca_kernel<2, double2, NT, 3><<<g, NT, 0, s>>>(a);
+    else if (a.mode == 0) aca_kernel<0, double2, NT, 3><<<g, NT, 0, s>>>(a);
+    else aca_kernel<1, double2, NT, 3><<<g, NT, 0, s>>>(a);
   } else {
-    if (plane) aca_kernel<2, float2, NT><<<g, NT, 0, s>>>(a);
-    else if (a.mode == 0) aca_kernel<0, float2, NT><<<g, NT, 0, s>>>(a);
-    else aca_kernel<1, float2, NT><<<g, NT, 0, s>>>(a);
+    if (plane) aca_kernel<2, float2, NT, 3><<<g, NT, 0, s>>>(a);
+    else if (a.mode != 0) aca_kernel<1, float2, NT, 3><<<g, NT, 0, s>>>(a);
+    else if (a.need == 1) aca_kernel<0, float2, NT, 1><<<g, NT, 0, s>>>(a);
+    else if (a.need == 2) aca_kernel<0, float2, NT, 2><<<g, NT, 0, s>>>(a);
+    else aca_kernel<0, float2, NT, 3><<<g, NT, 0, s>>>(a);
   }
 }
 

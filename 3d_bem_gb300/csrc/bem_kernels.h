@@ -54,6 +54,7 @@ struct NearfieldArgs {
   // without a plane; every entry adds the reflected element's operators
   const Elem* Er = nullptr;
   const ElemF* EFr = nullptr;
+  const ElemQ* EQ = nullptr;  // rule points of the elements (complex FP64 regular entries)
 };
 
 struct AcaArgs {
@@ -69,6 +70,7 @@ struct AcaArgs {
   float near_r2f;
   float2 alphaf;
   int which;  // 0 phi, 1 dphi
+  int need;   // operators the entries of any column need: bit 0 X, bit 1 Y (substitute)
   const double* rowpts;
   const double* colpts;
   const FarBlock* far;
@@ -93,6 +95,7 @@ struct AcaArgs {
   // impedance plane (mode 0 only): reflected elements, null without a plane
   const Elem* Er;
   const ElemF* EFr;
+  const ElemQ* EQ;  // rule points of the elements (complex FP64 regular entries)
 };
 
 constexpr int ACA_TAB_N = 12;  // rule-table bins per axis
@@ -161,6 +164,8 @@ struct HmvArgs {
   const void* Flo = nullptr;
 };
 
+// rule points of n elements
+void launch_rule_points(const Elem* E, int64_t n, ElemQ* o, cudaStream_t s);
 void nearfield_upload_rules(const QuadRules& r, cudaStream_t s);
 // hi = (float) v, lo = (float) (v - hi) for n complex values
 void launch_split_twofloat(const double2* v, float2* hi, float2* lo, int64_t n, cudaStream_t s);

@@ -18,6 +18,13 @@ struct __align__(16) Elem {
   double area;
 };
 
+// The 16 rule points of an element and the largest distance of one from the
+// centroid, for the FP64 regular rule (400 bytes).
+struct __align__(16) ElemQ {
+  double q[48];
+  double rho, pad;
+};
+
 // FP32 companion of Elem for the mixed-precision rules: vertices relative to
 // the element's own centroid (small numbers, so FP32 keeps ~7 digits of the
 // local geometry), unit normal, area, and the centroid as an unevaluated sum

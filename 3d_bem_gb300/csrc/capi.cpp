@@ -156,6 +156,8 @@ struct bem_handle {
   Layout L;
   DBuf<Elem> dE;
   DBuf<ElemF> dEF;
+  DBuf<ElemQ> dEQ;  // rule points, built with the first complex-FP64 assembly of a mesh
+  bool have_eq = false;
   DBuf<NearBlock> dNear;
   DBuf<FarBlock> dFar;
   DBuf<int32_t> dOrder, dSpRow, dSpCol, dListOff, dList, dPivCnt, dPivRc;
@@ -173,6 +175,7 @@ struct bem_handle {
   DBuf<BcCoef> dBc;
   DBuf<double2> dA, dB;
   double k = 0;
+  int need[2] = {3, 3};  // operators the entries of each matrix need (AcaArgs::need)
   DevHM hm[2];
   DBuf<double2> dT;
   DBuf<float2> dTf, dXf;
@@ -425,6 +428,7 @@ void set_frequency(bem_handle* h, double k) {
   const int64_t N = h->N;
   std::vector<BcCoef> bc(N);
   std::vector<double2> av(N), bv(N);
+  int need[2] = {0, 0};
   for (int64_t i = 0; i < N; i++) {
     // impedance walls: a = i k beta (beta = rho c / Z), rescaled per frequency
     const cplx a = h->impedance ? cplx(0.0, k) * h->beta[i] : h->a[i], b = h->b[i];
@@ -436,6 +440,12 @@ void set_frequency(bem_handle* h, double k) {
     c.ratio = make_double2(ratio.real(), ratio.imag());
     c.finv_main = make_float2((float)inv.real(), (float)inv.imag());
     c.fratio = make_float2((float)ratio.real(), (float)ratio.imag());
+    for (int q = 0; q < 2; q++) {
+      // rigid columns (ratio 0) take one of X and Y, the others both in dPhi
+      const bool main_x = (q == 0) == (c.subst != 0);
+      const bool both = q == 1 && ratio != 0.0;
+      need[q] |= (main_x || both ? 1 : 0) | (!main_x || both ? 2 : 0);
+    }
     bc[i] = c;
     av[i] = make_double2(a.real(), a.imag());
     bv[i] = make_double2(b.real(), b.imag());
@@ -443,6 +453,8 @@ void set_frequency(bem_handle* h, double k) {
   h->dBc.upload(bc, h->stream);
   h->dA.upload(av, h->stream);
   h->dB.upload(bv, h->stream);
+  h->need[0] = need[0];
+  h->need[1] = need[1];
   h->k = k;
 }
 
@@ -503,6 +515,7 @@ AcaArgs aca_args(bem_handle* h, DevHM& m, int which, int extra) {
   a.EF = h->dEF.p;
   a.Er = h->have_plane && !h->points_mode ? h->dEr.p : nullptr;
   a.EFr = h->have_plane && !h->points_mode ? h->dEFr.p : nullptr;
+  a.EQ = h->have_eq && !h->points_mode && m.prec == 0 ? h->dEQ.p : nullptr;
   a.bc = h->dBc.p;
   a.k = h->k;
   a.near_r = h->near_r;
@@ -512,6 +525,7 @@ AcaArgs aca_args(bem_handle* h, DevHM& m, int which, int extra) {
   a.near_r2f = (float)(h->near_r * h->near_r);
   a.alphaf = make_float2((float)al.real(), (float)al.imag());
   a.which = which;
+  a.need = h->need[which];
   a.rowpts = h->dRowPts.p;
   a.colpts = h->dColPts.p;
   a.far = h->dFar.p;
@@ -630,6 +644,14 @@ void assemble(bem_handle* h, double freq, double* t_near, double* t_aca) {
   na.alpha = make_double2(al.real(), al.imag());
   na.phi = h->hm[0].F.p;
   na.dphi = h->hm[1].F.p;
+  const bool fp64_near = na.precision == 1 && h->cfg.near_fp64;
+  if ((na.precision == 0 || fp64_near) && !h->have_eq) {
+    h->dEQ.ensure((size_t)h->N);
+    launch_rule_points(h->dE.p, h->N, h->dEQ.p, s);
+    h->launches++;
+    h->have_eq = true;
+  }
+  na.EQ = h->have_eq ? h->dEQ.p : nullptr;
   CK(cudaEventRecord(h->ev[0], s));
   // the near field (FP64-pipe-bound singular rules, FP32 regular rules) runs
   // on its own stream beside the barrier-bound ACA kernels; both write
@@ -638,7 +660,6 @@ void assemble(bem_handle* h, double freq, double* t_near, double* t_aca) {
   CK(cudaStreamWaitEvent(ns, h->ev[0], 0));
   // the learned near-field orders were trained on free-space pairs: with an
   // impedance plane the near field keeps the 16-point rule
-  const bool fp64_near = na.precision == 1 && h->cfg.near_fp64;
   const bool learned = (h->cfg.selector & 1) && na.precision == 1 && !h->have_plane && !fp64_near;
   for (auto& m : h->hm) m.has_lo = false;
   if (fp64_near) {  // FP64 quadrature into temporaries, split into hi + lo below
@@ -1730,6 +1751,7 @@ void clone_state(bem_handle* c, bem_handle* p) {
   c->L = p->L;
   c->points_mode = false;
   c->dE.upload(c->E, c->stream);
+  c->have_eq = false;
   c->dEF.upload(make_elemf(c->E), c->stream);
   c->dPerm.upload(c->rows.perm, c->stream);
   upload_layout(c);
@@ -2094,6 +2116,7 @@ bem_status bem_set_mesh(bem_handle* h, const double* tri, int64_t n) {
     h->N = n;
     prepare_elements(tri, h->rows.perm, h->E, h->avgdim);
     h->have_plane = false;  // a plane belongs to the mesh it was set for
+    h->have_eq = false;
     h->src.clear();
     for (const Elem& e : h->E)
       require(e.area > 0 && std::isfinite(e.nrm[0]), BEM_EINVAL, "degenerate (zero-area) triangle");

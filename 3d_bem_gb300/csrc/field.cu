@@ -16,6 +16,7 @@
 // sums in FP32 folded into FP64 accumulators every 128 (32) elements. Precision 0: the
 // same sum in FP64.
 #include "field.h"
+#include "phase.cuh"
 
 namespace bemgpu {
 namespace {
@@ -270,40 +271,6 @@ __global__ void __launch_bounds__(FIELD_PTS)
     for (int r = 0; r < RB; r++)
       partial[((int64_t)blockIdx.y * R + r0 + r) * M + ip] = make_double2(ax[r], ay[r]);
   }
-}
-
-// sin and cos of x, |x| <= X, by their Taylor series to x^(2 NS + 1) and
-// x^(2 NC): for X = 0.35 (6, 6) the first terms left out are below 3e-19 and
-// 5e-18 of the functions, for X = 1 (8, 9) below 9e-18 and 5e-19.
-template <int NS, int NC>
-__device__ __forceinline__ void sincos_taylor(double x, double& sn, double& cs) {
-  constexpr double is[9] = {1.0,
-                            -1.0 / 6,
-                            1.0 / 120,
-                            -1.0 / 5040,
-                            1.0 / 362880,
-                            -1.0 / 39916800,
-                            1.0 / 6227020800.0,
-                            -1.0 / 1307674368000.0,
-                            1.0 / 355687428096000.0};
-  constexpr double ic[10] = {1.0,
-                             -1.0 / 2,
-                             1.0 / 24,
-                             -1.0 / 720,
-                             1.0 / 40320,
-                             -1.0 / 3628800,
-                             1.0 / 479001600.0,
-                             -1.0 / 87178291200.0,
-                             1.0 / 20922789888000.0,
-                             -1.0 / 6402373705728000.0};
-  const double t = x * x;
-  double ps = is[NS], pc = ic[NC];
-#pragma unroll
-  for (int q = NS - 1; q >= 1; q--) ps = fma(ps, t, is[q]);
-#pragma unroll
-  for (int q = NC - 1; q >= 0; q--) pc = fma(pc, t, ic[q]);
-  sn = fma(x * t, ps, x);
-  cs = pc;
 }
 
 // Sums over the 7 rule points of w G / (4 pi r) and of its radial part

@@ -44,7 +44,8 @@ __global__ void __launch_bounds__(256) nearfield_regular_kernel(
     const Elem* __restrict__ E, const BcCoef* __restrict__ bc,
     const NearBlock* __restrict__ blocks, const NearTile* __restrict__ tiles,
     const uint32_t* __restrict__ special_bits, double k, double2 alpha,
-    double2* __restrict__ phi, double2* __restrict__ dphi, const Elem* __restrict__ Er) {
+    double2* __restrict__ phi, double2* __restrict__ dphi, const Elem* __restrict__ Er,
+    const ElemQ* __restrict__ EQ) {
   const NearTile t = tiles[blockIdx.x];
   if ((int)threadIdx.x >= t.count) return;
   const NearBlock b = blocks[t.block];
@@ -53,7 +54,8 @@ __global__ void __launch_bounds__(256) nearfield_regular_kernel(
   if (special_bits[g >> 5] & (1u << (g & 31))) return;
   const int r = e % b.m, c = e / b.m;
   const int64_t row = b.r0 + r, col = b.c0 + c;
-  Ops o = ops_regular(E[row], E[col], k, c_rules);
+  Ops o = EQ ? ops_regular_fast(E[row], E[col], EQ[col], k, c_rules)
+             : ops_regular(E[row], E[col], k, c_rules);
   if (Er) ops_add(o, ops_regular(E[row], Er[col], k, c_rules));
   double2 p, d;
   substitute(o, false, bc[col], alpha, p, d);
@@ -85,7 +87,9 @@ __global__ void __launch_bounds__(256) nearfield_regular32_kernel(
 }
 
 // Special entries: (global entry index, row, col) triples sorted so that the
-// singular (row == col) ones come first. Always FP64 arithmetic.
+// singular (row == col) ones come first. Always FP64 arithmetic, which bounds
+// it (one warp instruction per 64 cycles and SM quarter): accumulate_fast takes
+// about a third of the FP64 instructions of accumulate.
 template <typename T>
 __global__ void __launch_bounds__(128) nearfield_special_kernel(
     const Elem* __restrict__ E, const BcCoef* __restrict__ bc,
@@ -96,7 +100,7 @@ __global__ void __launch_bounds__(128) nearfield_special_kernel(
   if (i >= count) return;
   const int64_t row = sp_row[i], col = sp_col[i];
   Ops o = (row == col) ? ops_singular(E[row], k, c_rules)
-                       : ops_nearsing(E[row], E[col], k, c_rules);
+                       : nearsing_rule<true>(E[row], E[col], k, c_rules);
   // the reflected element always takes the regular rule (BemOperatorsReflected,
   // boundaryelementsolver.cpp:1516-1554)
   if (Er) ops_add(o, ops_regular(E[row], Er[col], k, c_rules));
@@ -169,6 +173,17 @@ __global__ void split_twofloat_kernel(const double2* __restrict__ v, float2* __r
 }
 }  // namespace
 
+namespace {
+__global__ void rule_points_kernel(const Elem* __restrict__ E, int64_t n, ElemQ* __restrict__ o) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) rule_points(E[i], c_rules, o[i]);
+}
+}  // namespace
+
+void launch_rule_points(const Elem* E, int64_t n, ElemQ* o, cudaStream_t s) {
+  if (n > 0) rule_points_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(E, n, o);
+}
+
 void launch_split_twofloat(const double2* v, float2* hi, float2* lo, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
   split_twofloat_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(v, hi, lo, n);
@@ -180,7 +195,7 @@ void launch_nearfield(const NearfieldArgs& a, cudaStream_t s) {
     if (a.ntiles > 0)
       nearfield_regular_kernel<<<(unsigned)a.ntiles, 256, 0, s>>>(
           a.E, a.bc, a.blocks, a.tiles, a.special_bits, a.k, a.alpha, (double2*)a.phi,
-          (double2*)a.dphi, a.Er);
+          (double2*)a.dphi, a.Er, a.EQ);
     if (a.nspecial > 0)
       nearfield_special_kernel<double2><<<g, 128, 0, s>>>(a.E, a.bc, a.sp_entry, a.sp_row,
                                                           a.sp_col, a.nspecial, a.k, a.alpha,

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "bem_types.h"
+#include "phase.cuh"
 
 namespace bemgpu {
 
@@ -41,7 +42,10 @@ struct Ops {
 
 // ----- the element integrand, shared by the regular and near-singular rules -----
 // G = exp(ikr) / (4 pi r); dG/dr = G/r (ikr - 1); d2G/dr2 = G/r^2 (2 - 2ikr - k^2 r^2)
-// (boundaryelementsolver.cpp:872-887, :1486-1500)
+// (boundaryelementsolver.cpp:872-887, :1486-1500). X: L and Mt, Y: M and N. What
+// is left out changes no bit of the others; the order of the statements decides
+// which products the compiler fuses, so it is the same for all.
+template <bool X = true, bool Y = true>
 __device__ __forceinline__ void accumulate(Ops& o, double w, double px, double py, double pz,
                                            double qx, double qy, double qz, const double* np,
                                            const double* nq, double upNq, double k) {
@@ -49,8 +53,8 @@ __device__ __forceinline__ void accumulate(Ops& o, double w, double px, double p
   double rr = rx * rx + ry * ry + rz * rz;
   double r = sqrt(rr);
   double ir = 1.0 / r;
-  double rnq = -(rx * nq[0] + ry * nq[1] + rz * nq[2]) * ir;
   double rnp = (rx * np[0] + ry * np[1] + rz * np[2]) * ir;
+  double rnq = -(rx * nq[0] + ry * nq[1] + rz * nq[2]) * ir;
   double s, c;
   sincos(k * r, &s, &c);
   double g0 = ir * (1.0 / (4.0 * 3.14159265358979323846));
@@ -63,16 +67,24 @@ __device__ __forceinline__ void accumulate(Ops& o, double w, double px, double p
   double2 Grr = cscale(ir * ir, G);
   double a2 = 2.0 - kr * kr, b2 = -2.0 * kr;
   double2 d2G = cmk(Grr.x * a2 - Grr.y * b2, Grr.x * b2 + Grr.y * a2);
-  o.L.x += w * G.x;
-  o.L.y += w * G.y;
   double wm = w * rnq, wt = w * rnp;
-  o.M.x += wm * dG.x;
-  o.M.y += wm * dG.y;
-  o.Mt.x += wt * dG.x;
-  o.Mt.y += wt * dG.y;
   double f1 = -(upNq + rnp * rnq) * ir, f2 = rnp * rnq;
-  o.N.x += w * (f1 * dG.x + f2 * d2G.x);
-  o.N.y += w * (f1 * dG.y + f2 * d2G.y);
+  if constexpr (X) {
+    o.L.x += w * G.x;
+    o.L.y += w * G.y;
+  }
+  if constexpr (Y) {
+    o.M.x += wm * dG.x;
+    o.M.y += wm * dG.y;
+  }
+  if constexpr (X) {
+    o.Mt.x += wt * dG.x;
+    o.Mt.y += wt * dG.y;
+  }
+  if constexpr (Y) {
+    o.N.x += w * (f1 * dG.x + f2 * d2G.x);
+    o.N.y += w * (f1 * dG.y + f2 * d2G.y);
+  }
 }
 
 // Regular rule: 16-point triangle rule scaled by the area (:857-893).
@@ -94,6 +106,135 @@ __device__ __forceinline__ Ops ops_regular(const Elem& P, const Elem& Q, double 
   o.Mt = cscale(A, o.Mt);
   o.N = cscale(A, o.N);
   return o;
+}
+
+// ops_regular with the rule points ready and only the operators asked for (the
+// others zero), the same to the bit: the pivots of the cross approximation are
+// chosen by these values, and a symmetric mesh has exact ties that a change of
+// rounding would decide otherwise.
+template <bool X, bool Y>
+__device__ __forceinline__ Ops ops_regular_part(const Elem& P, const Elem& Q, const ElemQ& qq,
+                                                double k, const QuadRules& R) {
+  Ops o{};
+  const double upNq = P.nrm[0] * Q.nrm[0] + P.nrm[1] * Q.nrm[1] + P.nrm[2] * Q.nrm[2];
+#pragma unroll 4
+  for (int i = 0; i < 16; i++)
+    accumulate<X, Y>(o, R.reg_w[i], P.c[0], P.c[1], P.c[2], qq.q[3 * i], qq.q[3 * i + 1],
+                     qq.q[3 * i + 2], P.nrm, Q.nrm, upNq, k);
+  if constexpr (X) {
+    o.L = cscale(Q.area, o.L);
+    o.Mt = cscale(Q.area, o.Mt);
+  }
+  if constexpr (Y) {
+    o.M = cscale(Q.area, o.M);
+    o.N = cscale(Q.area, o.N);
+  }
+  return o;
+}
+
+// Rule points of an element as ops_regular places them.
+__device__ __forceinline__ void rule_points(const Elem& e, const QuadRules& R, ElemQ& o) {
+  double rho = 0.0;
+  for (int i = 0; i < 16; i++) {
+    const double a1 = R.reg_x1[i], a2 = R.reg_x2[i], a3 = 1.0 - a2 - a1;
+    double d2 = 0.0;
+    for (int d = 0; d < 3; d++) {
+      const double q = a1 * e.n1[d] + a2 * e.n2[d] + a3 * e.n3[d];
+      o.q[3 * i + d] = q;
+      d2 += (q - e.c[d]) * (q - e.c[d]);
+    }
+    rho = fmax(rho, d2);
+  }
+  o.rho = sqrt(rho);
+  o.pad = 0.0;
+}
+
+// The four integrands at a point in fewer FP64 instructions, whose rate bounds
+// the near field of either precision (the pipe 88 % busy; at 5,120 elements 2.9
+// ms for the regular entries, 0.8 ms for the near-singular ones): 1 / r from one
+// rsqrt, exp(ikr) relative to exp(ik r_c), krc = k r_c, by a short series (FULL:
+// krc = 0, full sincos), and the radial parts collected by powers of 1 / r:
+//   dG = -G/r (1 - ikr);  with A = rnp rnq,  -(up + A) dG/r + A d2G =
+//   G/r^2 ((up + 3 A) (1 - ikr) - A (kr)^2).
+// (p - q) . n_q = dnq is the same for every point of the plane: o.M lacks that
+// factor, and all sums lack exp(ik r_c) / (4 pi).
+template <bool FULL, int NS, int NC>
+__device__ __forceinline__ void accumulate_fast(Ops& o, double w, const Elem& P, double qx,
+                                                double qy, double qz, double dnq, double up,
+                                                double k, double krc) {
+  const double rx = P.c[0] - qx, ry = P.c[1] - qy, rz = P.c[2] - qz;
+  const double rr = fma(rx, rx, fma(ry, ry, rz * rz));
+  const double ir = rsqrt(rr);
+  double r = rr * ir;
+  r = fma(0.5 * ir, fma(-r, r, rr), r);  // one correction: r to half an ulp
+  const double kr = k * r;
+  double sn, cs;
+  if constexpr (FULL) sincos(kr, &sn, &cs);
+  else sincos_taylor<NS, NC>(fma(k, r, -krc), sn, cs);
+  const double u = fma(kr, sn, cs), v = fma(-kr, cs, sn);  // (1 - ikr) exp
+  const double g0 = w * ir, g1 = g0 * ir, g2 = g1 * ir;
+  const double dnp = fma(rx, P.nrm[0], fma(ry, P.nrm[1], rz * P.nrm[2]));
+  o.L.x = fma(g0, cs, o.L.x);
+  o.L.y = fma(g0, sn, o.L.y);
+  const double t = -dnp * g2;
+  o.Mt.x = fma(t, u, o.Mt.x);
+  o.Mt.y = fma(t, v, o.Mt.y);
+  const double A = -dnp * dnq * (ir * ir), gB = g2 * fma(3.0, A, up), gA = g2 * A * (kr * kr);
+  o.M.x = fma(g2, u, o.M.x);
+  o.M.y = fma(g2, v, o.M.y);
+  o.N.x = fma(gB, u, fma(-gA, cs, o.N.x));
+  o.N.y = fma(gB, v, fma(-gA, sn, o.N.y));
+}
+
+// The common factors of the sums of accumulate_fast.
+__device__ __forceinline__ Ops finish_fast(const Ops& s, double scale, double dnq, double krc) {
+  double sn, cs;
+  sincos(krc, &sn, &cs);
+  scale *= 1.0 / (4.0 * 3.14159265358979323846);
+  const double2 ph = cmk(scale * cs, scale * sn);
+  Ops o;
+  o.L = cmul(ph, s.L);
+  o.M = cscale(dnq, cmul(ph, s.M));
+  o.Mt = cmul(ph, s.Mt);
+  o.N = cmul(ph, s.N);
+  return o;
+}
+
+// ops_regular by accumulate_fast (near-field blocks: no pivot hangs on them).
+__device__ __forceinline__ Ops ops_regular_fast(const Elem& P, const Elem& Q, const ElemQ& qq,
+                                                double k, const QuadRules& R) {
+  Ops o{};
+  const double up = P.nrm[0] * Q.nrm[0] + P.nrm[1] * Q.nrm[1] + P.nrm[2] * Q.nrm[2];
+  const double dx = P.c[0] - Q.c[0], dy = P.c[1] - Q.c[1], dz = P.c[2] - Q.c[2];
+  const double dnq = fma(dx, Q.nrm[0], fma(dy, Q.nrm[1], dz * Q.nrm[2]));
+  const double krho = k * qq.rho;
+  double krc = 0.0;
+  if (krho <= 1.0) {
+    krc = k * sqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+#pragma unroll 2
+    for (int i = 0; i < 16; i++)
+      if (krho <= 0.35)
+        accumulate_fast<false, 6, 6>(o, R.reg_w[i], P, qq.q[3 * i], qq.q[3 * i + 1],
+                                     qq.q[3 * i + 2], dnq, up, k, krc);
+      else
+        accumulate_fast<false, 8, 9>(o, R.reg_w[i], P, qq.q[3 * i], qq.q[3 * i + 1],
+                                     qq.q[3 * i + 2], dnq, up, k, krc);
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < 16; i++)
+      accumulate_fast<true, 1, 1>(o, R.reg_w[i], P, qq.q[3 * i], qq.q[3 * i + 1], qq.q[3 * i + 2],
+                                  dnq, up, k, 0.0);
+  }
+  return finish_fast(o, Q.area, dnq, krc);
+}
+
+// Whether an entry of matrix `which` (0 phi, 1 dPhi) needs X = L + alpha Mt and
+// Y = M + alpha N (substitute): rigid walls (ratio 0) need one of them.
+__host__ __device__ __forceinline__ void needs(const BcCoef& bc, int which, bool& x, bool& y) {
+  const bool mixed = bc.ratio.x != 0.0 || bc.ratio.y != 0.0;
+  const bool main_x = (which == 0) == (bc.subst != 0);
+  x = main_x || (which == 1 && mixed);
+  y = !main_x || (which == 1 && mixed);
 }
 
 // Singular rule for the panel's own collocation point (:896-1029): three
@@ -253,9 +394,23 @@ __device__ __forceinline__ int project_point(const Elem& Q, const double* p, dou
 
 // Near-singular split-polar rule (:1387-1514): project p onto the source
 // triangle, split there into 1-3 sub-triangles, 5 x 5 polar Gauss-Legendre.
-static __device__ __noinline__ Ops ops_nearsing(const Elem& P, const Elem& Q, double k,
-                                         const QuadRules& R) {
+// FAST: by accumulate_fast (near-field blocks).
+template <bool FAST>
+static __device__ __forceinline__ Ops nearsing_rule(const Elem& P, const Elem& Q, double k,
+                                                    const QuadRules& R) {
   Ops o{};
+  double dnq = 0.0, krho = 2.0, krc = 0.0;
+  if constexpr (FAST) {
+    const double dx = P.c[0] - Q.c[0], dy = P.c[1] - Q.c[1], dz = P.c[2] - Q.c[2];
+    dnq = fma(dx, Q.nrm[0], fma(dy, Q.nrm[1], dz * Q.nrm[2]));
+    double far = 0.0;  // of the corners from the centroid
+    for (const double* v : {Q.n1, Q.n2, Q.n3}) {
+      const double a = v[0] - Q.c[0], b = v[1] - Q.c[1], c = v[2] - Q.c[2];
+      far = fmax(far, a * a + b * b + c * c);
+    }
+    krho = k * sqrt(far);
+    if (krho <= 1.0) krc = k * sqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+  }
   double upNq = P.nrm[0] * Q.nrm[0] + P.nrm[1] * Q.nrm[1] + P.nrm[2] * Q.nrm[2];
   double Pp[3];
   int reg = project_point(Q, P.c, Pp);
@@ -322,7 +477,14 @@ static __device__ __noinline__ Ops ops_nearsing(const Elem& P, const Elem& Q, do
         double qy = A1[1] + x * e0[1] + y * e1[1];
         double qz = A1[2] + x * e0[2] + y * e1[2];
         double w = rmax / 2.0 * rs * R.line_w[i] * R.line_w[j];
-        accumulate(acc, w, P.c[0], P.c[1], P.c[2], qx, qy, qz, P.nrm, Q.nrm, upNq, k);
+        if constexpr (FAST) {
+          if (krho <= 0.35) accumulate_fast<false, 6, 6>(acc, w, P, qx, qy, qz, dnq, upNq, k, krc);
+          else if (krho <= 1.0)
+            accumulate_fast<false, 8, 9>(acc, w, P, qx, qy, qz, dnq, upNq, k, krc);
+          else accumulate_fast<true, 1, 1>(acc, w, P, qx, qy, qz, dnq, upNq, k, 0.0);
+        } else {
+          accumulate(acc, w, P.c[0], P.c[1], P.c[2], qx, qy, qz, P.nrm, Q.nrm, upNq, k);
+        }
       }
     }
     double f = angP / 2.0;
@@ -331,7 +493,12 @@ static __device__ __noinline__ Ops ops_nearsing(const Elem& P, const Elem& Q, do
     o.Mt = cadd(o.Mt, cscale(f, acc.Mt));
     o.N = cadd(o.N, cscale(f, acc.N));
   }
+  if constexpr (FAST) return finish_fast(o, 1.0, dnq, krc);
   return o;
+}
+static __device__ __noinline__ Ops ops_nearsing(const Elem& P, const Elem& Q, double k,
+                                                const QuadRules& R) {
+  return nearsing_rule<false>(P, Q, k, R);
 }
 
 // Near-singular test |p_i - p_j| < 4 * averageTriangleDim (:851), evaluated
@@ -530,6 +697,8 @@ __device__ __forceinline__ void sincos_turns(float x, float& sn, float& cs) {
 // The same FP32 integrand over the points b, b + s, b + 2 s, .. < e of the
 // tables x1, x2, wt: one lane's share when s lanes split an entry's rule (the
 // operators are sums over the points, so the shares add up to the entry).
+// X: L and Mt, Y: M and N, as in accumulate.
+template <bool X = true, bool Y = true>
 __device__ __forceinline__ OpsF ops_pts32(const ElemF& P, const ElemF& Q, float k,
                                           const float* x1, const float* x2, const float* wt,
                                           int b, int e, int s) {
@@ -561,16 +730,24 @@ __device__ __forceinline__ OpsF ops_pts32(const ElemF& P, const ElemF& Q, float 
     const float Grrx = Grx * ir, Grry = Gry * ir;
     const float a2c = 2.0f - kr * kr, b2c = -2.0f * kr;
     const float d2Gx = Grrx * a2c - Grry * b2c, d2Gy = Grrx * b2c + Grry * a2c;
-    Lx += w * Gx;
-    Ly += w * Gy;
     const float wm = w * rnq, wtt = w * rnp;
-    Mx += wm * dGx;
-    My += wm * dGy;
-    Tx += wtt * dGx;
-    Ty += wtt * dGy;
     const float f1 = -(upNq + rnp * rnq) * ir, f2 = rnp * rnq;
-    Nx += w * (f1 * dGx + f2 * d2Gx);
-    Ny += w * (f1 * dGy + f2 * d2Gy);
+    if constexpr (X) {
+      Lx += w * Gx;
+      Ly += w * Gy;
+    }
+    if constexpr (Y) {
+      Mx += wm * dGx;
+      My += wm * dGy;
+    }
+    if constexpr (X) {
+      Tx += wtt * dGx;
+      Ty += wtt * dGy;
+    }
+    if constexpr (Y) {
+      Nx += w * (f1 * dGx + f2 * d2Gx);
+      Ny += w * (f1 * dGy + f2 * d2Gy);
+    }
   }
   const float A = Q.area;
   OpsF o;

@@ -160,3 +160,39 @@ def test_gmres_cycles_against_dense(bem, meshes, n, restart):
     assert rel(x3, ref) < 1e-7 and np.abs(x3[:, 1]).max() == 0.0
     assert rel(A @ x1, B[:, 0]) < 1.1e-10
     s.close()
+
+
+@pytest.mark.parametrize("freq", [200.0, 440.0, 1400.0])
+@pytest.mark.parametrize("wall", ["rigid", "soft", "mixed"])
+def test_fp64_entries_in_each_phase_range(bem, meshes, orc, freq, wall):
+    """Near-field blocks (regular, near-singular and singular rules) with the
+    three forms of the phase (k rho below 0.35, below 1 and above; rho ~ 0.08 m)
+    and columns that need one or both pairs of operators. Differences from the
+    oracle are the rounding of k r (60 at most) and of the terms of N, which
+    cancel by less than 1e3: 1e-12 of a block's largest entry. The far blocks
+    together hold theirs to a hundred times the ACA tolerance."""
+    tri = meshes.icosphere(3, 1.0)[:-1]
+    n = tri.shape[0]
+    i = np.arange(n)
+    a = {"rigid": 0 * i, "soft": 1 + 0 * i, "mixed": (i % 3 == 1) * 0.7j + (i % 3 == 2) * 2.0}[wall] + 0j
+    b = {"rigid": 1 + 0 * i, "soft": 0 * i, "mixed": 1 + 0 * i}[wall] + 0j
+    s = bem.Solver(leaf_size=32, aca_tol=1e-6, wave_speed=343.0)
+    s.set_mesh(tri)
+    s.set_bc(a, b)
+    s.assemble(freq)
+    P = orc.Problem(tri, 32, s.config.eta)
+    perm = P.perm
+    exact = P.dense(2 * np.pi * freq / 343.0, s.config.coupling, a[perm], b[perm])
+    info = s.partition()
+    for which in (0, 1):
+        D = s.dense(which)
+        far = np.zeros(2)
+        for r0, m, c0, nn, adm in info:
+            ref = exact[which][r0:r0 + m, c0:c0 + nn]
+            got = D[r0:r0 + m, c0:c0 + nn]
+            if adm:
+                far += [np.linalg.norm(got - ref) ** 2, np.linalg.norm(ref) ** 2]
+            else:
+                assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
+        assert far[0] < 1e-8 * far[1]
+    s.close()
