@@ -152,6 +152,18 @@ __device__ __forceinline__ void block_argmax(R v, int idx, Red<R>& red, R& best,
     }
 }
 
+template <int NT, typename R>
+__device__ __forceinline__ int block_min(int v, Red<R>& red) {
+  v = __reduce_min_sync(0xffffffffu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red.i[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = red.i[0];
+#pragma unroll
+  for (int q = 1; q < NT / 32; q++) v = min(v, red.i[q]);
+  return v;
+}
+
 // FP32 rule tables in shared memory
 struct AcaTables {
   float x1[16], x2[16], w[16];
@@ -525,53 +537,68 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) aca_kernel(AcaArgs a) {
     }
   } else {
     // --- partialPivotACAextra with host-computed normal-filtered seeds ---
+    // Every thread holds one seed: its entry, and the crosses' value there, taken
+    // on from where it stopped whenever the rank has grown. The seeds run in
+    // their order, the next one is the first that the crosses do not hold.
+    // (One seed after the other, its entry evaluated by all threads: 93.7 instead
+    // of 89.0 ms for the FP64 solve at 5,120 elements.)
     const int32_t* piv = a.piv_rc + 2 * a.piv_off[bi];
     const int npiv = a.piv_cnt[bi];
-    for (int p = 0; p < npiv && k < kmax; p++) {
-      int ri = piv[2 * p], ci = piv[2 * p + 1];
-      const T pivv = aca_entry_part<MODE, T, NEED>(a, tab, fb.r0 + ri, fb.c0 + ci, 0, 1);
+    for (int base = 0; base < npiv && k < kmax; base += NT) {
+      const int mine = base + threadIdx.x;
+      const int sr = mine < npiv ? piv[2 * mine] : 0, sc = mine < npiv ? piv[2 * mine + 1] : 0;
+      T pivv{0, 0}, approx{0, 0};
+      if (mine < npiv)
+        pivv = aca_entry_part<MODE, T, NEED>(a, tab, fb.r0 + sr, fb.c0 + sc, 0, 1);
       const R pabs2 = mag2(pivv);
-      if (sqrt(pabs2) < tiny) continue;
-      // approximation already good at the seed?
-      T approx = Cx<T>::make(0, 0);
-      for (int l = 0; l < k; l++) {
-        const T t = cx_mul(cx_mul(U[(int64_t)l * m + ri], S[l]), V[(int64_t)l * n + ci]);
-        approx.x += t.x;
-        approx.y += t.y;
-      }
-      if (sqrt(mag2(cx_sub(pivv, approx)) / pabs2) < tol) continue;
-      residual_col<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ci, U + (int64_t)k * m, coef);
-      bool first = true;
+      const bool live = mine < npiv && !(sqrt(pabs2) < tiny);
+      int held = 0, p = base - 1;
       while (k < kmax) {
-        const T* colv = first ? U + (int64_t)k * m : U + (int64_t)(k - 1) * m;
-        R cmax;
-        argmax_abs<T, NT>(colv, m, first ? -1 : ri, red, cmax, ri);
-        first = false;
-        if (cmax <= tiny && k >= 1) break;
-        T* rowv = V + (int64_t)k * n;
-        residual_row<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ri, rowv, coef);
-        R rmax;
-        argmax_abs<T, NT>(rowv, n, -1, red, rmax, ci);
-        if (rmax <= tiny && k >= 1) break;
-        T* newcol = U + (int64_t)k * m;
-        residual_col<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ci, newcol, coef);
-        const T alpha = cx_recip(rowv[ci]);
-        if (threadIdx.x == 0) S[k] = alpha;
-        __syncthreads();
-        R gain;
-        T incr;
-        norm_increment<T, NT>(fb, U, V, S, k, newcol, rowv, alpha, red, gain, incr);
-        const T old = est;
-        k++;
-        est.x += incr.x;
-        est.y += incr.y;
-        const R target = tol * tol * est.x;
-        if (tol > 0 && gain < target) {
-          if (gain < 0.1 * target) {  // roll back the last rank (hmatrix.cpp:724-728)
-            k--;
-            est = old;
+        if (live)
+          for (; held < k; held++) {
+            const T t = cx_mul(cx_mul(U[(int64_t)held * m + sr], S[held]),
+                               V[(int64_t)held * n + sc]);
+            approx.x += t.x;
+            approx.y += t.y;
           }
-          break;
+        const bool open =
+            live && mine > p && !(sqrt(mag2(cx_sub(pivv, approx)) / pabs2) < tol);
+        p = block_min<NT, R>(open ? mine : 0x7fffffff, red);
+        if (p == 0x7fffffff) break;
+        int ri = 0, ci = piv[2 * p + 1];
+        residual_col<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ci, U + (int64_t)k * m, coef);
+        bool first = true;
+        while (k < kmax) {
+          const T* colv = first ? U + (int64_t)k * m : U + (int64_t)(k - 1) * m;
+          R cmax;
+          argmax_abs<T, NT>(colv, m, first ? -1 : ri, red, cmax, ri);
+          first = false;
+          if (cmax <= tiny && k >= 1) break;
+          T* rowv = V + (int64_t)k * n;
+          residual_row<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ri, rowv, coef);
+          R rmax;
+          argmax_abs<T, NT>(rowv, n, -1, red, rmax, ci);
+          if (rmax <= tiny && k >= 1) break;
+          T* newcol = U + (int64_t)k * m;
+          residual_col<MODE, T, NT, NEED>(a, tab, fb, U, V, S, k, ci, newcol, coef);
+          const T alpha = cx_recip(rowv[ci]);
+          if (threadIdx.x == 0) S[k] = alpha;
+          __syncthreads();
+          R gain;
+          T incr;
+          norm_increment<T, NT>(fb, U, V, S, k, newcol, rowv, alpha, red, gain, incr);
+          const T old = est;
+          k++;
+          est.x += incr.x;
+          est.y += incr.y;
+          const R target = tol * tol * est.x;
+          if (tol > 0 && gain < target) {
+            if (gain < 0.1 * target) {  // roll back the last rank (hmatrix.cpp:724-728)
+              k--;
+              est = old;
+            }
+            break;
+          }
         }
       }
     }
