@@ -1048,12 +1048,14 @@ bool prepare_hlu_program(bem_handle* h) {
     h->dHPendInit.upload(pend, s);
   }
   h->dHQueueInit.upload(P.queue_init, s);
-  h->dHCtrlInit.upload(std::vector<int32_t>{0, 0, 0, 0, P.nready0, 0, 0, 0}, s);
+  std::vector<int32_t> ctrl0(HLU_CTRL, 0);
+  ctrl0[4] = P.nready0;
+  h->dHCtrlInit.upload(ctrl0, s);
   h->dHPend.ensure(P.tasks.size());
   h->dHQueue.ensure(P.tasks.size());
   h->dHPairs.upload(P.pairs, s);
   h->dHQr.upload(P.qr, s);
-  h->dHCtrl.ensure(8);
+  h->dHCtrl.ensure(HLU_CTRL);
   sync(h);
   h->hp_gen = h->layout_gen;
   h->hp_kc = h->cfg.precond_rank;
@@ -1246,7 +1248,7 @@ bool build_hlu_device(bem_handle* h) {
   const size_t nt = P.tasks.size();
   CK(cudaMemcpyAsync(h->dHPend.p, h->dHPendInit.p, nt * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
   CK(cudaMemcpyAsync(h->dHQueue.p, h->dHQueueInit.p, nt * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-  CK(cudaMemcpyAsync(h->dHCtrl.p, h->dHCtrlInit.p, 8 * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+  CK(cudaMemcpyAsync(h->dHCtrl.p, h->dHCtrlInit.p, HLU_CTRL * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
   HluExecArgs a{};
   a.precision = m.prec;
   a.arena = h->dArena.p;

@@ -1,11 +1,11 @@
 // hlu_exec.cu -- executor of the H-LU task program (hlu_gpu.h): one persistent
 // kernel over a ready queue. A CTA takes the next queue slot, waits (bounded)
 // until a task is pushed into it, runs the task with all its threads, then
-// releases the task's successors; the release that completes a successor's
-// dependencies pushes it. Only CTAs that are running hold slots and tasks, so
-// the queue advances with any number of resident CTAs: the launch needs no
-// co-residency and starts on the SMs that are free (beside other streams'
-// kernels) instead of waiting for a whole idle GPU.
+// releases the task's successors; of those whose last dependency this was, it
+// goes on with one and pushes the others. Only CTAs that are running hold slots
+// and tasks, so the queue advances with any number of resident CTAs: the launch
+// needs no co-residency and starts on the SMs that are free (beside other
+// streams' kernels) instead of waiting for a whole idle GPU.
 //
 // Data that other CTAs wrote during the launch is read through L2
 // (ld.global.cg) and written with st.global.cg, so no SM reads a stale L1
@@ -22,6 +22,7 @@ namespace {
 constexpr int HX_THREADS = 256;
 constexpr int HX_WARPS = HX_THREADS / 32;
 constexpr int HX_MAX_PAIRS = 64;  // truncation inputs per task (checked on the host)
+constexpr int HX_PAIRS_SMEM = 8;  // so many are read from shared memory
 
 template <typename T2>
 struct Cx;
@@ -74,6 +75,21 @@ __device__ __forceinline__ T2 cmul(T2 a, T2 b) {
 template <typename T2>
 __device__ __forceinline__ T2 cmulc(T2 a, T2 b) {
   return Cx<T2>::mk(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
+}
+// acc += a b and acc += conj(a) b, four fused operations (cadd of cmul takes six)
+template <typename T2>
+__device__ __forceinline__ void cfma(T2& acc, T2 a, T2 b) {
+  acc.x = fma(a.x, b.x, acc.x);
+  acc.y = fma(a.x, b.y, acc.y);
+  acc.x = fma(-a.y, b.y, acc.x);
+  acc.y = fma(a.y, b.x, acc.y);
+}
+template <typename T2>
+__device__ __forceinline__ void cfmac(T2& acc, T2 a, T2 b) {
+  acc.x = fma(a.x, b.x, acc.x);
+  acc.y = fma(a.x, b.y, acc.y);
+  acc.x = fma(a.y, b.y, acc.x);
+  acc.y = fma(-a.y, b.x, acc.y);
 }
 template <typename T2>
 __device__ __forceinline__ T2 cconj(T2 a) {
@@ -150,14 +166,10 @@ __device__ void task_gemm(const HluTask& t, T2* arena, T2* sm) {
     const int w = tid >> 5, ln = tid & 31;
     for (int o = w; o < m * n; o += HX_WARPS) {
       const int i = o % m, j = o / m;
-      R sr = 0, si = 0;
-      for (int l = ln; l < q; l += 32) {
-        const T2 p = cmul(opget(A, opa, i, l, t.lda), opget(B, opb, l, j, t.ldb));
-        sr += p.x;
-        si += p.y;
-      }
-      sr = warp_sum(sr);
-      si = warp_sum(si);
+      T2 d = cz<T2>();
+      for (int l = ln; l < q; l += 32)
+        cfma(d, opget(A, opa, i, l, t.lda), opget(B, opb, l, j, t.ldb));
+      const R sr = warp_sum(d.x), si = warp_sum(d.y);
       if (ln == 0) {
         T2 v = Cx<T2>::mk(neg ? -sr : sr, neg ? -si : si);
         T2* c = C + i + (int64_t)j * t.ldc;
@@ -190,13 +202,10 @@ __device__ void task_gemm(const HluTask& t, T2* arena, T2* sm) {
       const int o = tid + k * HX_THREADS;
       if (o < m * n) {
         const int i = o % m, j = o / m;
-        R ar = 0, ai = 0;
-        for (int l = 0; l < q; l++) {
-          const T2 av = sa[i + l * m], bv = sb[l + j * ldb_s];
-          ar += av.x * bv.x - av.y * bv.y;
-          ai += av.x * bv.y + av.y * bv.x;
-        }
-        const T2 v = Cx<T2>::mk(neg ? cv[k].x - ar : cv[k].x + ar, neg ? cv[k].y - ai : cv[k].y + ai);
+        T2 p = cz<T2>();
+#pragma unroll 4
+        for (int l = 0; l < q; l++) cfma(p, sa[i + l * m], sb[l + j * ldb_s]);
+        const T2 v = neg ? csub(cv[k], p) : cadd(cv[k], p);
         stA(C + i + (int64_t)j * t.ldc, v);
       }
     }
@@ -231,11 +240,7 @@ __device__ void task_gemm(const HluTask& t, T2* arena, T2* sm) {
         for (int ll = 0; ll < QC; ll++) {
           const T2 av = sa[ti + ll * TM];
 #pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const T2 bv = sb[ll + (tj0 + k * tjs) * QC];
-            acc[k].x += av.x * bv.x - av.y * bv.y;
-            acc[k].y += av.x * bv.y + av.y * bv.x;
-          }
+          for (int k = 0; k < 4; k++) cfma(acc[k], av, sb[ll + (tj0 + k * tjs) * QC]);
         }
         __syncthreads();
       }
@@ -272,7 +277,8 @@ __device__ void task_lmul(const HluTask& t, T2* arena, T2* sm) {
     for (int e = threadIdx.x; e < m * w; e += HX_THREADS) {
       const int i = e % m, j = e / m;
       T2 acc = cz<T2>();
-      for (int l = 0; l < m; l++) acc = cadd(acc, cmul(sM[i + l * m], sX[l + j * m]));
+#pragma unroll 4
+      for (int l = 0; l < m; l++) cfma(acc, sM[i + l * m], sX[l + j * m]);
       stA(X + i + (int64_t)(j0 + j) * t.ldc, acc);
     }
   }
@@ -297,7 +303,8 @@ __device__ void task_rmul(const HluTask& t, T2* arena, T2* sm) {
     for (int e = threadIdx.x; e < h * n; e += HX_THREADS) {
       const int i = e % h, j = e / h;
       T2 acc = cz<T2>();
-      for (int l = 0; l < n; l++) acc = cadd(acc, cmul(sX[i + l * h], sM[l + j * n]));
+#pragma unroll 4
+      for (int l = 0; l < n; l++) cfma(acc, sX[i + l * h], sM[l + j * n]);
       stA(X + (i0 + i) + (int64_t)j * t.ldc, acc);
     }
   }
@@ -329,27 +336,106 @@ __device__ void task_zero(const HluTask& t, T2* arena) {
 }
 
 // ---------------------------------------------------------------- QR of a diagonal leaf
-// Householder reflectors H_j = I - 2 v v^H (|v| = 1) as in the host H-LU:
-// H_{m-1} .. H_0 A = R, Q = H_0 .. H_{m-1}. W accumulates Q^H = H_{m-1} .. H_0
-// alongside. Outputs: Q, R (column-major), Q^H and R^{-1} (row-major).
+// H_{m-1} .. H_0 [A | I] for m <= 32 into sA and sW: a column in the registers
+// of four lanes (rows sub, sub + 4, ..), so that a step reads only the reflector
+// from shared memory; the lanes of the next column form the next reflector.
+// Bound by the latency of the m steps (FP64: by the FP64 pipe). A leaf's task
+// with 25 rows: 25 us with the columns in shared memory, 17 us so (FP32).
+// FP32 subtracts the rounded product: single fused operations are closer to
+// FP64, but move a solve with the factors of a slender body at low frequency by
+// 3e-5 instead of 8e-6 from what the columns in shared memory give.
 template <typename T2>
-__device__ void task_qr(const HluTask& t, const HluExecArgs& a, T2* arena, T2* sm) {
+__device__ void qr_columns(const HluTask& t, const T2* arena, T2* sA, T2* sW, int ld, T2* sv) {
   using R = typename Cx<T2>::R;
-  const int m = t.m, ld = m + 1;  // odd leading dimension
-  T2* sA = sm;               // m x m
-  T2* sW = sA + m * ld;      // m x m
-  T2* sv = sW + m * ld;      // reflectors of steps j (even / odd), 2 x m
-  T2* sd = sv + 2 * m;       // 1 / R(r, r), m
-  __shared__ R s_r[4];
+  const int m = t.m;
+  const int c = threadIdx.x >> 2, sub = threadIdx.x & 3;
+  T2 y[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int r = sub + 4 * i;
+    y[i] = cz<T2>();
+    if (r < m && c < m) y[i] = ldA(arena + t.a + r + (int64_t)c * t.lda);
+    else if (r < m && r == c - m) y[i].x = 1;
+  }
+  // v = (x + ph |x| e_j) / |.| of column j in rows j .. 31; the column's warp
+  // calls, its lanes store. (FP64 skips the rows above j; in FP32 the branches
+  // cost more than the rows.)
+  constexpr bool SKIP = sizeof(R) == 8;
+  auto reflector = [&](int j) {
+    T2* v = sv + (j & 1) * 32;
+    R xn2 = 0;
+    T2 x0 = cz<T2>();
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int r = sub + 4 * i;
+      if (r >= j && (!SKIP || 4 * i + 3 >= j)) xn2 = fma(y[i].x, y[i].x, fma(y[i].y, y[i].y, xn2));
+      if (r == j) x0 = y[i];
+    }
+    x0.x = __shfl_sync(0xffffffffu, x0.x, j & 3, 4);
+    x0.y = __shfl_sync(0xffffffffu, x0.y, j & 3, 4);
+    xn2 += __shfl_xor_sync(0xffffffffu, xn2, 1);
+    xn2 += __shfl_xor_sync(0xffffffffu, xn2, 2);
+    const R ax2 = cabs2(x0);
+    const R xn = Cx<T2>::sq(xn2);
+    const T2 ph = ax2 > 0 ? cscale(x0, Cx<T2>::rsq(ax2)) : Cx<T2>::mk(1, 0);
+    const T2 v0 = cadd(x0, cscale(ph, xn));
+    const R vn2 = xn2 - ax2 + cabs2(v0);
+    const R inv = vn2 > 0 ? Cx<T2>::rsq(vn2) : R(0);
+    if (c == j) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const int r = sub + 4 * i;
+        v[r] = r < j ? cz<T2>() : cscale(r == j ? v0 : y[i], inv);
+      }
+    }
+  };
+  const int w8 = 8 * (threadIdx.x >> 5);  // the warp's first column
+  if (w8 == 0) reflector(0);
+  __syncthreads();
+  for (int j = 0; j < m; j++) {
+    // H_j = I - 2 v v^H on columns j.. of A and all columns of W
+    if (w8 + 7 >= j && w8 < 2 * m) {
+      const T2* v = sv + (j & 1) * 32;
+      T2 d = cz<T2>();
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (!SKIP || (4 * i + 3 >= j && 4 * i < m)) cfmac(d, v[sub + 4 * i], y[i]);
+#pragma unroll
+      for (int o = 2; o > 0; o >>= 1) {
+        d.x += __shfl_xor_sync(0xffffffffu, d.x, o);
+        d.y += __shfl_xor_sync(0xffffffffu, d.y, o);
+      }
+      d = cscale(d, c >= j ? R(2) : R(0));
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (!SKIP) y[i] = csub(y[i], cmul(v[sub + 4 * i], d));
+        else if (4 * i + 3 >= j && 4 * i < m) cfma(y[i], v[sub + 4 * i], cneg(d));
+      if (j + 1 < m && (unsigned)(j + 1 - w8) < 8u) reflector(j + 1);
+    }
+    __syncthreads();
+  }
+  if (c < 2 * m) {
+    T2* d = c < m ? sA + c * ld : sW + (c - m) * ld;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (sub + 4 * i < m) d[sub + 4 * i] = y[i];
+  }
+  __syncthreads();
+}
+
+// The same with the columns in shared memory, for m > 32: two lanes a column.
+template <typename T2>
+__device__ void qr_columns_smem(const HluTask& t, const T2* arena, T2* sA, T2* sW, int ld, T2* sv) {
+  using R = typename Cx<T2>::R;
+  const int m = t.m;
   for (int e = threadIdx.x; e < m * m; e += HX_THREADS) {
     const int i = e % m, j = e / m;
     sA[i + j * ld] = ldA(arena + t.a + i + (int64_t)j * t.lda);
     sW[i + j * ld] = i == j ? Cx<T2>::mk(1, 0) : cz<T2>();
   }
-  if (threadIdx.x == 0) s_r[0] = 0;
   __syncthreads();
   // tpc threads per column (consecutive lanes): rows i = j + sub, j + sub + tpc, ..
-  const int tpc = m <= 32 ? 4 : 2;
+  constexpr int tpc = 2;
   const int c = threadIdx.x / tpc, sub = threadIdx.x % tpc;
   const unsigned gmask = ((1u << tpc) - 1u) << ((threadIdx.x & 31) & ~(tpc - 1));  // the group's lanes
   // reflector of column j from the group holding it (only its lanes call):
@@ -396,6 +482,23 @@ __device__ void task_qr(const HluTask& t, const HluExecArgs& a, T2* arena, T2* s
     if (c == 1 && j + 1 < m) reflector(j + 1);
     __syncthreads();
   }
+}
+
+// Householder reflectors H_j = I - 2 v v^H (|v| = 1) as in the host H-LU:
+// H_{m-1} .. H_0 A = R, Q = H_0 .. H_{m-1}. W accumulates Q^H = H_{m-1} .. H_0
+// alongside. Outputs: Q, R (column-major), Q^H and R^{-1} (row-major).
+template <typename T2>
+__device__ void task_qr(const HluTask& t, const HluExecArgs& a, T2* arena, T2* sm) {
+  using R = typename Cx<T2>::R;
+  const int m = t.m, ld = m + 1;  // odd leading dimension
+  T2* sA = sm;               // m x m
+  T2* sW = sA + m * ld;      // m x m
+  T2* sv = sW + m * ld;      // reflectors of steps j (even / odd)
+  T2* sd = sv + (m < 32 ? 64 : 2 * m);  // 1 / R(r, r), m
+  __shared__ R s_r[4];
+  if (threadIdx.x == 0) s_r[0] = 0;
+  if (m <= 32) qr_columns<T2>(t, arena, sA, sW, ld, sv);
+  else qr_columns_smem<T2>(t, arena, sA, sW, ld, sv);
   const HluQrOut o = a.qr[t.x0];
   // Q = W^H, Q^H row-major = W column-major read by rows: Qh[r m + c] = W(r, c)
   for (int e = threadIdx.x; e < m * m; e += HX_THREADS) {
@@ -433,8 +536,9 @@ __device__ void task_qr(const HluTask& t, const HluExecArgs& a, T2* arena, T2* s
           if (r < 32) acc0 = yr;
           else acc1 = yr;
         }
-        if (ln < r) acc0 = csub(acc0, cmul(sA[ln + r * ld], yr));
-        if (ln + 32 < r) acc1 = csub(acc1, cmul(sA[ln + 32 + r * ld], yr));
+        yr = cneg(yr);
+        if (ln < r) cfma(acc0, sA[ln + r * ld], yr);
+        if (ln + 32 < r) cfma(acc1, sA[ln + 32 + r * ld], yr);
       }
       if (ln < m) stA(arena + o.rinv + (int64_t)ln * m + tc, ln <= tc ? acc0 : cz<T2>());
       if (ln + 32 < m) stA(arena + o.rinv + (int64_t)(ln + 32) * m + tc, ln + 32 <= tc ? acc1 : cz<T2>());
@@ -589,19 +693,6 @@ __device__ void house_apply(const T2* X, int64_t rows, int p, const T2* head, T2
       __syncthreads();
     }
   }
-}
-
-// element (r, l) of a truncation piece (kinds 0, 2, 3; identity handled by the caller)
-template <typename T2>
-__device__ __forceinline__ T2 piece_get(const HluExecArgs& a, int kind, int64_t off, int64_t soff,
-                                        int rs, int cs, int64_t r, int l) {
-  if (kind == 0) return ldA(reinterpret_cast<const T2*>(a.arena) + off + r * rs + (int64_t)l * cs);
-  if (kind == 2) {
-    const T2 u = __ldg(reinterpret_cast<const T2*>(a.U) + off + r * rs + (int64_t)l * cs);
-    const T2 s = __ldg(reinterpret_cast<const T2*>(a.S) + soff + l);
-    return cmul(u, s);
-  }
-  return __ldg(reinterpret_cast<const T2*>(a.V) + off + r * rs + (int64_t)l * cs);
 }
 
 // One-sided Jacobi on the q columns of X (p x q, column-major): X V = U diag(s),
@@ -772,7 +863,7 @@ __device__ void mm_st(const T2* S, int64_t rows, int kt, const T2* T, int L, T2*
     T2 acc = cz<T2>();
     for (int l = 0; l < kt; l++) {
       const T2 sv = S[i + (int64_t)l * rows];
-      acc = cadd(acc, cmul(conj_s ? cconj(sv) : sv, T[l + (int64_t)c * kt]));
+      cfma(acc, conj_s ? cconj(sv) : sv, T[l + (int64_t)c * kt]);
     }
     Y[e] = acc;
   }
@@ -851,17 +942,10 @@ __device__ void sub_mm_ty(const Side<T2>& S, int rows, int kt, const T2* Y, int 
       const int l = o % kt, c = o / kt;
       const T2* sc = Sc + l * ld;
       const T2* yc = Y + i0 + c * rows;
-      R ar = 0, ai = 0;
+      T2 p = cz<T2>();
 #pragma unroll 4
-      for (int i = 0; i < h; i++) {
-        T2 sv = sc[i];
-        if (conj_s) sv.y = -sv.y;
-        const T2 y = yc[i];
-        ar += sv.x * y.x - sv.y * y.y;
-        ai += sv.x * y.y + sv.y * y.x;
-      }
-      const T2 t0 = T[o];
-      T[o] = Cx<T2>::mk(t0.x + ar, t0.y + ai);
+      for (int i = 0; i < h; i++) cfma(p, conj_s ? cconj(sc[i]) : sc[i], yc[i]);
+      T[o] = cadd(T[o], p);
     }
   }
   if (conj_out) {
@@ -885,30 +969,93 @@ __device__ void sub_mm_st(const Side<T2>& S, int rows, int kt, const T2* T, int 
     for (int o = threadIdx.x; o < h * lq; o += HX_THREADS) {
       const int i = o % h, c = o / h;
       const T2* tc = T + c * kt;
-      R ar = 0, ai = 0;
+      T2 p = cz<T2>();
 #pragma unroll 4
       for (int l = 0; l < kt; l++) {
-        T2 sv = Sc[i + l * ld];
-        if (conj_s) sv.y = -sv.y;
-        const T2 tv = tc[l];
-        ar += sv.x * tv.x - sv.y * tv.y;
-        ai += sv.x * tv.y + sv.y * tv.x;
+        const T2 sv = Sc[i + l * ld];
+        cfma(p, conj_s ? cconj(sv) : sv, tc[l]);
       }
-      Y[i0 + i + c * rows] = Cx<T2>::mk(ar, ai);
+      Y[i0 + i + c * rows] = p;
     }
   }
   __syncthreads();
 }
 
-// Orthonormal columns of Y (rows x lq, shared) in place by modified
-// Gram-Schmidt with a second pass (one warp, lanes over the rows). A column
-// whose remainder falls below drop x its own norm lies in the span of the
-// earlier ones (rank deficiency) and becomes zero: it adds no direction, and
-// a zero column of the basis carries no singular value.
+// K sums over a warp (K = 4, 8 or 16): lanes swap halves of the values that
+// are left until one is, K + log2(32 / K) - 1 exchanges instead of 5 K; sum i
+// goes to out[i] (shared).
+template <int K, typename R>
+__device__ __forceinline__ void warp_sums(R* d, R* out) {
+  const int ln = threadIdx.x & 31;
+#pragma unroll
+  for (int h = K / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = ln & o;
+#pragma unroll
+    for (int i = 0; i < h; i++) {
+      const R send = up ? d[i] : d[i + h], keep = up ? d[i + h] : d[i];
+      d[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+#pragma unroll
+  for (int o = 16 / K; o > 0; o >>= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], o);
+  if ((ln & (32 / K - 1)) == 0) out[ln / (32 / K)] = d[0];
+  __syncwarp();
+}
+
+// One pass of Gram-Schmidt of column j <= KJ of Y against the earlier ones by a
+// warp: d_k = q_k^H y in d[2 k], d[2 k + 1] (shared), y -= sum_k d_k q_k. n0 is a
+// lane's part of |y|^2 before, replaced by the sum when `first`; returns this
+// lane's part of |y|^2 after.
+template <int KJ, typename T2>
+__device__ __forceinline__ typename Cx<T2>::R orth_pass(T2* Y, int rows, int j, bool first,
+                                                        typename Cx<T2>::R& n0,
+                                                        typename Cx<T2>::R* d) {
+  using R = typename Cx<T2>::R;
+  constexpr int K = 2 * KJ + 2;  // the last value: |y|^2
+  const int ln = threadIdx.x;
+  T2* y = Y + j * rows;
+  R s[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) s[k] = 0;
+  for (int i = ln; i < rows; i += 32) {
+    const T2 yi = y[i];
+#pragma unroll
+    for (int k = 0; k < KJ; k++)
+      if (k < j) {
+        const T2 q = Y[i + k * rows];  // conj(q) y
+        s[2 * k] = fma(q.y, yi.y, fma(q.x, yi.x, s[2 * k]));
+        s[2 * k + 1] = fma(-q.y, yi.x, fma(q.x, yi.y, s[2 * k + 1]));
+      }
+  }
+  s[K - 1] = n0;
+  warp_sums<K>(s, d);
+  if (first) n0 = d[K - 1];
+  R part = 0;
+  for (int i = ln; i < rows; i += 32) {
+    T2 yi = y[i];
+#pragma unroll
+    for (int k = 0; k < KJ; k++)
+      if (k < j) {
+        const T2 q = Y[i + k * rows];
+        cfma(yi, q, Cx<T2>::mk(-d[2 * k], -d[2 * k + 1]));
+      }
+    y[i] = yi;
+    part += cabs2(yi);
+  }
+  return part;
+}
+
+// Orthonormal columns of Y (rows x lq, lq <= 8, shared) in place by Gram-Schmidt
+// with a second pass (one warp, lanes over the rows). A column whose remainder
+// falls below drop x its own norm lies in the span of the earlier ones (rank
+// deficiency) and becomes zero: it adds no direction, and a zero column of the
+// basis carries no singular value. The chain of the passes bounds it: each
+// reduces only the sums its column has.
 template <typename T2>
 __device__ void sub_orth(T2* Y, int rows, int lq, T2* Rz = nullptr) {
   using R = typename Cx<T2>::R;
   const R drop = sizeof(R) == 4 ? R(1e-10) : R(1e-26);
+  __shared__ R d[2][16];
   if (threadIdx.x < 32) {
     const int ln = threadIdx.x;
     if (Rz) {
@@ -920,56 +1067,18 @@ __device__ void sub_orth(T2* Y, int rows, int lq, T2* Rz = nullptr) {
     for (int j = 0; j < lq; j++) {
       T2* y = Y + j * rows;
       R nn = 0;
-      for (int pass = 0; pass < 2; pass++) {
-        // d_k = q_k^H y (k < j) and, in the first pass, |y|^2: one butterfly
-        // over all the sums at once
-        R d[2 * HS_L + 1];
-#pragma unroll
-        for (int k = 0; k < 2 * HS_L + 1; k++) d[k] = 0;
-        if (j > 0) {
-          for (int i = ln; i < rows; i += 32) {
-            const T2 yi = y[i];
-#pragma unroll
-            for (int k = 0; k < HS_L; k++)
-              if (k < j) {
-                const T2 q = Y[i + k * rows];  // conj(q) y
-                d[2 * k] += q.x * yi.x + q.y * yi.y;
-                d[2 * k + 1] += q.x * yi.y - q.y * yi.x;
-              }
-          }
+      if (j == 0) {
+        nn = n0 = warp_sum(n0);
+      } else {
+        for (int pass = 0; pass < 2; pass++) {
+          if (j == 1) nn = orth_pass<1>(Y, rows, j, pass == 0, n0, d[pass]);
+          else if (j <= 3) nn = orth_pass<3>(Y, rows, j, pass == 0, n0, d[pass]);
+          else nn = orth_pass<7>(Y, rows, j, pass == 0, n0, d[pass]);
         }
-        if (pass == 0) d[2 * HS_L] = n0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-          for (int k = 0; k < 2 * HS_L + 1; k++) d[k] += __shfl_xor_sync(0xffffffffu, d[k], o);
-        }
-        if (pass == 0) n0 = d[2 * HS_L];
-        if (Rz && ln < j) {  // R(k, j) = the two passes' coefficients
-#pragma unroll
-          for (int k = 0; k < HS_L; k++)
-            if (k == ln) {
-              const T2 o = Rz[k + j * HS_L];
-              Rz[k + j * HS_L] = Cx<T2>::mk(o.x + d[2 * k], o.y + d[2 * k + 1]);
-            }
-        }
-        // y -= sum_k d_k q_k, and the new |y|^2
-        R part = 0;
-        for (int i = ln; i < rows; i += 32) {
-          T2 yi = y[i];
-#pragma unroll
-          for (int k = 0; k < HS_L; k++)
-            if (k < j) {
-              const T2 q = Y[i + k * rows];
-              yi.x -= q.x * d[2 * k] - q.y * d[2 * k + 1];
-              yi.y -= q.x * d[2 * k + 1] + q.y * d[2 * k];
-            }
-          y[i] = yi;
-          part += cabs2(yi);
-        }
-        nn = warp_sum(part);
-        __syncwarp();
-        if (j == 0) break;  // nothing to project on
+        nn = warp_sum(nn);
+        if (Rz && ln < j)  // R(k, j) = the two passes' coefficients
+          Rz[ln + j * HS_L] = Cx<T2>::mk(d[0][2 * ln] + d[1][2 * ln],
+                                         d[0][2 * ln + 1] + d[1][2 * ln + 1]);
       }
       const R s = (nn > 0 && nn > drop * n0) ? Cx<T2>::rsq(nn) : R(0);
       if (Rz && ln == 0) Rz[j + j * HS_L] = Cx<T2>::mk(s > 0 ? nn * s : R(0), 0);
@@ -1145,7 +1254,7 @@ __device__ void trunc_subspace(const Side<T2>& SA, const Side<T2>& SB, int m, in
       if (ident) {
         v = cconj(V[i + j * HS_L]);
       } else {
-        for (int c = 0; c < lq; c++) v = cadd(v, cmul(Q[i + c * m], cconj(V[c + j * HS_L])));
+        for (int c = 0; c < lq; c++) cfma(v, Q[i + c * m], cconj(V[c + j * HS_L]));
       }
       v = cscale(v, sig[j]);
     }
@@ -1156,7 +1265,7 @@ __device__ void trunc_subspace(const Side<T2>& SA, const Side<T2>& SB, int m, in
     T2 v = cz<T2>();
     if (l < r) {
       const int j = s_idx[l];
-      for (int c = 0; c < lq; c++) v = cadd(v, cmul(Z[i + c * n], Rz[c + j * HS_L]));
+      for (int c = 0; c < lq; c++) cfma(v, Z[i + c * n], Rz[c + j * HS_L]);
       v = cscale(v, Cx<T2>::div(R(1), sig[j]));
     }
     stA(Bo + e, v);
@@ -1173,15 +1282,33 @@ __device__ void task_trunc(const HluTask& t, const HluExecArgs& a, T2* arena, T2
   const int kc = a.kc;
   const HluTruncPair* P = a.pairs + t.x0;
   const int np = t.x1;
-  if (threadIdx.x == 0) {
+  // the pairs (short lists in shared memory) and the first column of each
+  __shared__ int4 s_pairs[HX_PAIRS_SMEM * sizeof(HluTruncPair) / sizeof(int4)];
+  if (np <= HX_PAIRS_SMEM) {
+    for (int e = threadIdx.x; e < np * (int)(sizeof(HluTruncPair) / sizeof(int4)); e += HX_THREADS)
+      s_pairs[e] = __ldg(reinterpret_cast<const int4*>(P) + e);
+    P = reinterpret_cast<const HluTruncPair*>(s_pairs);
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) {
     int c = 0;
-    for (int p = 0; p < np; p++) {
-      s_cb[p] = c;
-      int w = P[p].cols;
-      if (P[p].rank_idx >= 0) w = min(w, max(0, __ldg(a.rank + P[p].rank_idx)));
-      c += w;
+    for (int p0 = 0; p0 < np; p0 += 32) {
+      const int p = p0 + threadIdx.x;
+      int w = 0;
+      if (p < np) {
+        w = P[p].cols;
+        if (P[p].rank_idx >= 0) w = min(w, max(0, __ldg(a.rank + P[p].rank_idx)));
+      }
+      int x = w;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if ((int)threadIdx.x >= o) x += y;
+      }
+      if (p < np) s_cb[p] = c + x - w;
+      c += __shfl_sync(0xffffffffu, x, 31);
     }
-    s_cb[np] = c;
+    if (threadIdx.x == 0) s_cb[np] = c;
   }
   __syncthreads();
   const int kt = s_cb[np];
@@ -1220,40 +1347,65 @@ __device__ void task_trunc(const HluTask& t, const HluExecArgs& a, T2* arena, T2
   T2* SA = S;
   T2* SB = S + (int64_t)lda * kt;
   T2* W = SB + (int64_t)ldb * kt;  // work area of the chosen path
-  // gather both sides (placements, zeros elsewhere), four loads in flight
-  // per thread
-  for (int p = 0; p < np; p++) {
-    const HluTruncPair pp = P[p];
-    const int c0 = s_cb[p], w = s_cb[p + 1] - c0;
-    const bool na = pp.neg & 1, nb = pp.neg & 2;
-    for (int side = 0; side < 2; side++) {
-      const int rows = (int)(side ? n : m), ld = side ? ldb : lda;
-      const int64_t r0 = side ? pp.rb : pp.ra, mr = side ? pp.mb : pp.ma;
-      const int kind = side ? pp.bkind : pp.akind;
-      const int64_t off = side ? pp.boff : pp.aoff, soff = side ? 0 : pp.soff;
-      const int rs = side ? pp.brs : pp.ars, cs = side ? pp.bcs : pp.acs;
-      const bool ng = side ? nb : na;
-      T2* D = side ? SB : SA;
-      for (int e0 = threadIdx.x; e0 < rows * w; e0 += 4 * HX_THREADS) {
-        T2 v[4];
+  // gather both sides (placements, zeros elsewhere): a warp per column, over
+  // the columns of all pairs, four columns in flight
+  {
+    constexpr int GU = 4;
+    const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
+    for (int cb = w; cb < 2 * kt; cb += GU * HX_WARPS) {
+      const T2* src[GU];  // row 0 of the target in the piece's column
+      int pq[GU], rs[GU], lo[GU], hi[GU];
+      int rmax = 0;
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int e = e0 + u * HX_THREADS;
-          v[u] = cz<T2>();
-          if (e < rows * w) {
-            const int r = e % rows, l = e / rows;
-            const int64_t rr = r - r0;
-            if (rr >= 0 && rr < mr) {
-              if (kind == 1) v[u] = rr == l ? Cx<T2>::mk(1, 0) : cz<T2>();
-              else v[u] = piece_get<T2>(a, kind, off, soff, rs, cs, rr, l);
-              if (ng) v[u] = cneg(v[u]);
-            }
+      for (int u = 0; u < GU; u++) {
+        const int c = cb + u * HX_WARPS;
+        pq[u] = -1;
+        lo[u] = hi[u] = rs[u] = 0;
+        src[u] = nullptr;
+        if (c < 2 * kt) {
+          const bool side = c >= kt;
+          const int l = side ? c - kt : c;
+          for (int p0 = 0; p0 < np && pq[u] < 0; p0 += 32) {
+            const int p = p0 + ln;
+            const unsigned in =
+                __ballot_sync(0xffffffffu, p < np && s_cb[p] <= l && l < s_cb[p + 1]);
+            if (in) pq[u] = p0 + __ffs(in) - 1;
           }
+          const HluTruncPair& pp = P[pq[u]];
+          const int kind = side ? pp.bkind : pp.akind;
+          lo[u] = side ? pp.rb : pp.ra;
+          hi[u] = lo[u] + (side ? pp.mb : pp.ma);
+          rs[u] = side ? pp.brs : pp.ars;
+          const T2* base = reinterpret_cast<const T2*>(kind == 0 ? a.arena : kind == 2 ? a.U : a.V);
+          if (kind != 1)
+            src[u] = base + (side ? pp.boff : pp.aoff) +
+                     (int64_t)(l - s_cb[pq[u]]) * (side ? pp.bcs : pp.acs) - (int64_t)lo[u] * rs[u];
+          rmax = max(rmax, (int)(side ? n : m));
+        }
+      }
+      for (int r = ln; r < rmax; r += 32) {
+        T2 v[GU];
+#pragma unroll
+        for (int u = 0; u < GU; u++) {
+          v[u] = cz<T2>();
+          if (r >= lo[u] && r < hi[u] && src[u]) v[u] = ldA(src[u] + (int64_t)r * rs[u]);
         }
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int e = e0 + u * HX_THREADS;
-          if (e < rows * w) D[e % rows + (int64_t)(c0 + e / rows) * ld] = v[u];
+        for (int u = 0; u < GU; u++) {
+          const int c = cb + u * HX_WARPS;
+          if (c >= 2 * kt) continue;
+          const bool side = c >= kt;
+          if (r >= (int)(side ? n : m)) continue;
+          const int col = side ? c - kt : c, l = col - s_cb[pq[u]];
+          const HluTruncPair& pp = P[pq[u]];
+          const int kind = side ? pp.bkind : pp.akind;
+          if (r >= lo[u] && r < hi[u]) {
+            if (kind == 1) v[u] = r - lo[u] == l ? Cx<T2>::mk(1, 0) : cz<T2>();
+            else if (kind == 2)
+              v[u] = cmul(v[u], __ldg(reinterpret_cast<const T2*>(a.S) + (side ? 0 : pp.soff) + l));
+            if (pp.neg & (side ? 2 : 1)) v[u] = cneg(v[u]);
+          }
+          (side ? SB : SA)[r + (int64_t)col * (side ? ldb : lda)] = v[u];
         }
       }
     }
@@ -1302,7 +1454,7 @@ __device__ void task_trunc(const HluTask& t, const HluExecArgs& a, T2* arena, T2
       T2 v = cz<T2>();
       if (l < r) {
         const int j = s_idx[l];
-        for (int c = 0; c < L; c++) v = cadd(v, cmul(Q[i + (int64_t)c * m], cconj(V[c + j * L])));
+        for (int c = 0; c < L; c++) cfma(v, Q[i + (int64_t)c * m], cconj(V[c + j * L]));
         v = cscale(v, sig[j]);
       }
       stA(Ao + e, v);
@@ -1341,7 +1493,7 @@ __device__ void task_trunc(const HluTask& t, const HluExecArgs& a, T2* arena, T2
     const int r = e % pa, c = e / pa;
     T2 acc = cz<T2>();
     for (int l = small ? 0 : max(r, c); l < kt; l++)
-      acc = cadd(acc, cmul(SA[r + (int64_t)l * m], SB[c + (int64_t)l * n]));
+      cfma(acc, SA[r + (int64_t)l * m], SB[c + (int64_t)l * n]);
     if (tr) X[c + r * p] = acc;  // X = core^T
     else X[r + c * p] = acc;
   }
@@ -1397,22 +1549,33 @@ __device__ __forceinline__ unsigned long long globaltimer() {
   return t;
 }
 
-// the ready task in queue slot q (-1 until pushed); -1 when the error word is
-// set or the wait ran out (a bounded wait)
-__device__ int wait_slot(const int* q, int* ctrl, int64_t limit) {
+constexpr int HX_DONE = 32;  // ctrl word of the tasks done, on a line of its own
+
+// the ready task in queue slot q (-1 until pushed); -1 when every task is done,
+// the error word is set or no task finished for `limit` cycles (a bounded wait)
+__device__ int wait_slot(const int* q, int* ctrl, int ntasks, int64_t limit) {
   int v = ld_acquire(q);
   if (v >= 0) return v;
-  const long long t0 = clock64();
+  long long t0 = clock64();
+  int seen = -1;
   unsigned ns = 32;
-  for (;;) {
+  for (int n = 0;; n++) {
     __nanosleep(ns);
     if (ns < 512) ns <<= 1;
     v = ld_acquire(q);
     if (v >= 0) return v;
-    if (ld_relaxed(ctrl + 1)) return -1;
-    if (clock64() - t0 > limit) {
-      atomicCAS(ctrl + 1, 0, 1);  // 1: a wait ran out of time
-      return -1;
+    const bool late = clock64() - t0 > limit;
+    if ((n & 3) == 3 || late) {
+      const int done = ld_relaxed(ctrl + HX_DONE);
+      if (done >= ntasks || ld_relaxed(ctrl + 1)) return -1;
+      if (late) {
+        if (done == seen) {
+          atomicCAS(ctrl + 1, 0, 1);  // 1: a wait ran out of time
+          return -1;
+        }
+        t0 = clock64();
+        seen = done;
+      }
     }
   }
 }
@@ -1425,31 +1588,34 @@ __device__ __forceinline__ int dec_acq_rel(int* p) {
   return old;
 }
 
-// The executor pops ready tasks in the order they became ready: thread 0
-// takes the next queue slot and waits (bounded) until a task is pushed into
-// it; the CTA runs the task; then its threads release the successors, each
-// decrementing a successor's pending count, and the one that reaches zero
-// pushes it. Every task is pushed once, so the queue has one slot per task.
+// A CTA takes the next queue slot, waits (bounded) until a ready task is pushed
+// into it and runs it; then its threads release the successors, each decrementing
+// a successor's pending count. Of those that reach zero the CTA keeps one as its
+// next task and pushes the others, so at most one slot per task is used and the
+// slots left over end with the last task. The factorization is a chain of some
+// 12,000 tasks (82,000 elements) of mostly 2 to 5 us: the successor list is read
+// before the task runs, and a task kept needs no push, slot or poll (median
+// hand-over on the chain 3.3 us through the queue, 1.3 us so).
 template <typename T2>
 __global__ void __launch_bounds__(HX_THREADS, sizeof(T2) == 8 ? 4 : 2) hlu_exec_kernel(HluExecArgs a) {
   extern __shared__ __align__(16) unsigned char hx_smem[];
   T2* sm = reinterpret_cast<T2*>(hx_smem);
-  __shared__ int s_task;
+  __shared__ int s_task, s_next;
   T2* arena = reinterpret_cast<T2*>(a.arena);
   T2* slot = reinterpret_cast<T2*>(a.scratch) + (int64_t)blockIdx.x * a.scratch_per_cta;
+  if (threadIdx.x == 0) s_next = -1;
   for (;;) {
     if (threadIdx.x == 0) {
-      int t = -1;
-      if (ld_relaxed(a.ctrl + 1) == 0) {
+      int t = s_next;
+      s_next = -1;
+      unsigned long long tc = a.trace ? globaltimer() : 0ull;
+      if (t < 0 && ld_relaxed(a.ctrl + 1) == 0) {
         const int h = atomicAdd(a.ctrl, 1);
-        if (h < a.ntasks) {
-          const unsigned long long tc = a.trace ? globaltimer() : 0ull;
-          t = wait_slot(a.queue + h, a.ctrl, a.wait_cycles);
-          if (t >= 0 && a.trace) {
-            a.trace[3 * (int64_t)t] = tc;
-            a.trace[3 * (int64_t)t + 1] = globaltimer();
-          }
-        }
+        if (h < a.ntasks) t = wait_slot(a.queue + h, a.ctrl, a.ntasks, a.wait_cycles);
+      }
+      if (t >= 0 && a.trace) {
+        a.trace[3 * (int64_t)t] = tc;
+        a.trace[3 * (int64_t)t + 1] = globaltimer();
       }
       s_task = t;
     }
@@ -1457,6 +1623,9 @@ __global__ void __launch_bounds__(HX_THREADS, sizeof(T2) == 8 ? 4 : 2) hlu_exec_
     const int ti = s_task;
     if (ti < 0) break;
     const HluTask t = a.tasks[ti];
+    const int s0 = __ldg(a.succ_off + ti) + threadIdx.x, s1 = __ldg(a.succ_off + ti + 1);
+    int sc = s0 < s1 ? __ldg(a.succ + s0) : -1;
+    if (sc >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.tasks + sc));
     switch (t.type) {
       case HT_GEMM: task_gemm<T2>(t, arena, sm); break;
       case HT_LMUL: task_lmul<T2>(t, arena, sm); break;
@@ -1467,17 +1636,19 @@ __global__ void __launch_bounds__(HX_THREADS, sizeof(T2) == 8 ? 4 : 2) hlu_exec_
       case HT_ZERO: task_zero<T2>(t, arena); break;
       default: break;
     }
-    __syncthreads();  // the task's writes are done (and ordered before the releases below)
-    if (threadIdx.x == 0 && a.trace) a.trace[3 * (int64_t)ti + 2] = globaltimer();
-    const int s1 = __ldg(a.succ_off + ti + 1);
-    for (int k = __ldg(a.succ_off + ti) + threadIdx.x; k < s1; k += HX_THREADS) {
-      const int sc = __ldg(a.succ + k);
-      __threadfence();
-      if (dec_acq_rel(a.pending + sc) == 1) {
+    __syncthreads();  // the task's writes are done; the releases below carry them
+    if (threadIdx.x == 0) {
+      if (a.trace) a.trace[3 * (int64_t)ti + 2] = globaltimer();
+      asm volatile("red.relaxed.gpu.global.add.s32 [%0], 1;" ::"l"(a.ctrl + HX_DONE) : "memory");
+    }
+    for (int k = s0; k < s1; k += HX_THREADS) {
+      if (k != s0) sc = __ldg(a.succ + k);
+      if (dec_acq_rel(a.pending + sc) == 1 && atomicCAS(&s_next, -1, sc) != -1) {
         const int pos = atomicAdd(a.ctrl + 4, 1);
         st_release(a.queue + pos, sc);
       }
     }
+    __syncthreads();
   }
 }
 

@@ -154,6 +154,8 @@ bool hlu_gpu_plan(const HTree& tree, const Layout& L, int64_t kc, HluProgram& P,
 bool hlu_df_plan_structure(const FlatFactor& f, int64_t N, const std::vector<int64_t>& cuts,
                            HluDfPlan& p, std::string* why);
 
+constexpr int HLU_CTRL = 64;  // control words of the executor (two lines and their neighbours)
+
 struct HluExecArgs {
   int precision;                 // 0 complex FP64, 1 complex FP32 (FP32 arithmetic)
   void* arena;
@@ -169,14 +171,15 @@ struct HluExecArgs {
   int* queue;                    // ntasks slots of ready tasks: the tasks without
                                  // dependencies first, -1 in the others at launch
   int* ctrl;                     // [0] pop counter, [1] error word, [2] bad pivots,
-                                 // [3] non-finite flag, [4] push counter (initial ready count)
+                                 // [3] non-finite flag, [4] push counter (initial ready
+                                 // count), [32] tasks done (HLU_CTRL words)
   void* scratch;                 // grid x scratch_per_cta complex elements
   int64_t scratch_per_cta;
   void* big_scratch;             // regions of the large truncations (HluTask.a)
   int32_t kc;
   double tol;                    // truncation tolerance (0: rank kc)
   int32_t range_power;           // power iterations of the randomized range finder (0 or 1)
-  int64_t wait_cycles;           // bound of one dependency wait (clock64 cycles)
+  int64_t wait_cycles;           // bound of a wait in which no task finishes (clock64 cycles)
   unsigned long long* trace;     // optional: per task claim, start, end (ns)
 };
 

@@ -196,3 +196,21 @@ def test_fp64_entries_in_each_phase_range(bem, meshes, orc, freq, wall):
                 assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
         assert far[0] < 1e-8 * far[1]
     s.close()
+
+
+@pytest.mark.parametrize("n", [1, 3, 31, 32, 33, 64])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_leaf_factorization_sizes(bem, meshes, n, precision):
+    """One diagonal leaf: its factors are exact, below and above the 32 rows that
+    fit in registers. Rounding times a condition number of at most 1e3: 1e-11
+    with FP64 factors, 1e-4 with FP32 ones."""
+    tri = meshes.box(n_target=200, seed=5)[:n]
+    s = bem.Solver(precision=precision, precond_rank=2, leaf_size=64)
+    s.set_mesh(tri)
+    s.set_bc(np.zeros(n), np.ones(n))
+    s.assemble(300.0)
+    s.hlu_build()
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    assert rel(s.hlu_solve(s.hmatvec(1, x)).ravel(), x) < (1e-11, 1e-4)[precision]
+    s.close()
