@@ -246,7 +246,9 @@ __device__ __forceinline__ T aca_entry_part(const AcaArgs& a, const AcaTables& t
     if (row != col && !near_pair32(a.EF, row, col, a.near_r2f)) {
       const ElemF& P = a.EF[row];
       const ElemF& Qe = a.EF[col];
-      OpsF o;
+      // one call for both kinds of rules, for the size of the code (see ops_pts32)
+      const float *x1 = tab.x1, *x2 = tab.x2, *wt = tab.w;
+      int i0 = q, i1 = 16;
       if (a.rule_tab) {
         float dx, dy, dz;
         centroid_diff(P, Qe, dx, dy, dz);
@@ -256,13 +258,13 @@ __device__ __forceinline__ T aca_entry_part(const AcaArgs& a, const AcaTables& t
         const int ix = min(max((int)floorf((x - a.tab_x0) / a.tab_dx), 0), ACA_TAB_N - 1);
         const int iy = min(max((int)floorf((y - a.tab_y0) / a.tab_dy), 0), ACA_TAB_N - 1);
         const int c = min((int)a.rule_tab[ix * ACA_TAB_N + iy], SEL_C - 1);
-        o = ops_pts32<X, Y>(P, Qe, a.kf, tab.cx1, tab.cx2, tab.cw, c_cls.off[c] + q,
-                            c_cls.off[c + 1], Q);
-      } else if (Q == 1) {
-        o = ops_pts32<X, Y>(P, Qe, a.kf, c_rules.freg_x1, c_rules.freg_x2, c_rules.freg_w, 0, 16, 1);
-      } else {
-        o = ops_pts32<X, Y>(P, Qe, a.kf, tab.x1, tab.x2, tab.w, q, 16, Q);
+        x1 = tab.cx1;
+        x2 = tab.cx2;
+        wt = tab.cw;
+        i0 = c_cls.off[c] + q;
+        i1 = c_cls.off[c + 1];
       }
+      OpsF o = ops_pts32<X, Y>(P, Qe, a.kf, x1, x2, wt, i0, i1, Q);
       if constexpr (MODE == 2)
         ops_add(o, ops_pts32<X, Y>(P, a.EFr[col], a.kf, tab.x1, tab.x2, tab.w, q, 16, Q));
       float2 p, d;
