@@ -25,8 +25,8 @@
 // Each task lists the tasks whose results it reads or whose inputs it
 // overwrites (read-after-write, write-after-write and write-after-read on the
 // row segments of every buffer, one segment per leaf cluster). Tasks are
-// numbered in a topological order; the kernel's CTAs claim them in that order
-// and wait (bounded) on the done flags of their dependencies.
+// numbered in a topological order; the kernel's CTAs run them as their last
+// dependency completes (hlu_exec.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -77,14 +77,14 @@ PENCIL_DESC = ("pencil r=4 mm L=0.2 m + 10 mm conical tip, 81,920 triangles, imp
                "Z in [0.5, 50] rho c, 8 RHS, 64 log-spaced f 200 Hz-8 kHz, H-LU preconditioner "
                "rank 2")
 # DRAM bytes per algorithmic byte of the 8-RHS FP32 H-matvec, measured with
-# ncu (dram__bytes_read.sum + dram__bytes_write.sum of hmv32_vpass<8> and
-# hmv32_upass<8,256,6>) on the 20,480-triangle pencil: 592 MB for 521 MB; the
+# ncu (dram__bytes_read.sum + dram__bytes_write.sum of hmv_vpass<ArF32, 8> and
+# hmv_upass<ArF32, 8>) on the 20,480-triangle pencil: 422 MB for 384 MB; the
 # traffic grows with the stored entries, so it scales to the headline size
-HMV32_R8_TRAFFIC_PER_BYTE = 592.2 / 521.4
-# ncu --set full of aca_kernel<0,float2,128> (the 128-thread ACA launch of the
-# phi matrix) on the 20,480-triangle sphere at 1.5 kHz: FMA pipe active 40.6 %
-# of its peak, issue slots 64 %, warps active 50 %, L2 hit rate 66 %
-ACA_FMA_PIPE_NCU = 0.406
+HMV32_R8_TRAFFIC_PER_BYTE = 422.4 / 384.0
+# ncu of aca_kernel<0,float2,128,1> (the 128-thread ACA launch of the phi
+# matrix) on the 20,480-triangle sphere at 1.5 kHz: FMA pipe active 37.9 % of
+# its peak, issue slots 67 %, warps active 50 %, L2 hit rate 66 %
+ACA_FMA_PIPE_NCU = 0.379
 METRIC = "freq-solves/sec (H-matrix Helmholtz BEM solve, <=1e-5 rel. surface-pressure error)"
 UNIT = "freq-solves/s"
 
@@ -641,7 +641,7 @@ def run_ours(args):
                    "l2": "working set (H-matrices and factors, GBs) >> 129 MB L2; no flush"},
         "e2e": {"value": round(e2e, 4), "unit": UNIT, "h2d_bytes_per_step": n * R * 16,
                 "d2h_bytes_per_step": n * R * 16},
-        "roofline": {"kernel": "hmatvec FP32 (hmv32_vpass + hmv32_upass), c64 storage, 8 RHS",
+        "roofline": {"kernel": "hmatvec FP32 (hmv_vpass + hmv_upass), c64 storage, 8 RHS",
                      "bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                      "frac": round(achieved / hbm, 4),
                      "traffic": int(B * HMV32_R8_TRAFFIC_PER_BYTE),
@@ -724,7 +724,7 @@ def run_hmatvec_only(args):
     """The inner-GMRES H-matvec of the pencil (complex-FP32 storage, FP32
     arithmetic, 8 right-hand sides) after one assembly at 1 kHz, args.pencil_n
     triangles: its algorithmic bytes and event-timed duration (for profiling
-    the hmv32 kernels)."""
+    the hmv_vpass and hmv_upass kernels)."""
     import torch
     pkg = importlib.import_module("3d_bem_gb300")
     meshes = importlib.import_module("3d_bem_gb300.meshes")
