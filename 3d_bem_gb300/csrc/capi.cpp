@@ -936,9 +936,9 @@ void upload_df_plan(bem_handle* h, const HluDfPlan& p, int prec, bem_handle::DfD
 }
 
 // The sweeps' vectors and flags, and the inverses of the supers' diagonal blocks
-// (views of both plans set; leaf data of both factors on the device).
-const void* hlu_data(const bem_handle* h, int which);
-void finish_df(bem_handle* h) {
+// (views of both plans set; data: the leaf values of both factors on the device).
+// dfErr[1] is set when a value of the inverses is not finite.
+void finish_df(bem_handle* h, const void* const (&data)[2]) {
   cudaStream_t s = h->stream;
   const size_t cs = h->hlu_prec == 0 ? sizeof(double2) : sizeof(float2);
   bem_handle::DfDev* d[2] = {&h->dfL, &h->dfU};
@@ -946,15 +946,29 @@ void finish_df(bem_handle* h) {
   h->dfS.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
   h->dfT.ensure((size_t)HLU_DF_MAX_R * std::max<int64_t>({d[0]->view.nt, d[1]->view.nt, 1}) * cs);
   h->dfCtrl.ensure((size_t)(1 + 3 * std::max(d[0]->view.D, d[1]->view.D)));
-  h->dfErr.ensure(1);
-  CK(cudaMemsetAsync(h->dfErr.p, 0, sizeof(int), s));
+  h->dfErr.ensure(2);
+  CK(cudaMemsetAsync(h->dfErr.p, 0, 2 * sizeof(int), s));
   h->dfDense.ensure((size_t)std::max(d[0]->view.msize, d[1]->view.msize) * cs);
   for (int q = 0; q < 2; q++) {
     d[q]->minv.ensure((size_t)d[q]->view.msize * cs);
     d[q]->view.minv = d[q]->minv.p;
-    h->launches += launch_hlu_df_invert(d[q]->view, hlu_data(h, q), h->hlu_prec, h->dfDense.p, s);
+    // blocks without a leaf (rank 0) are zero, whatever the buffer held before
+    CK(cudaMemsetAsync(h->dfDense.p, 0, (size_t)d[q]->view.msize * cs, s));
+    h->launches += launch_hlu_df_invert(d[q]->view, data[q], h->hlu_prec, h->dfDense.p, s);
+    launch_hlu_finite_check(d[q]->minv.p, d[q]->view.msize, h->hlu_prec, h->dfErr.p + 1, h->nsm, s);
+    h->launches++;
   }
   CK(cudaGetLastError());
+}
+
+// After finish_df: the dataflow sweeps run when the inverses are finite, else the
+// leaf-by-leaf ones, which need no inverse.
+void accept_df(bem_handle* h) {
+  int bad = 0;
+  CK(cudaMemcpyAsync(&bad, h->dfErr.p + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  h->df_ok = !bad;
+  if (bad) h->df_why = "the inverse of a diagonal block is not finite";
 }
 
 // Plans of the dataflow sweeps for both host factors; when either factor lacks
@@ -984,8 +998,8 @@ void upload_df_plans(bem_handle* h) {
     }
     d.view.diag = d.diag.p;
   }
-  finish_df(h);
-  h->df_ok = true;
+  finish_df(h, {h->dLd.p, h->dUd.p});
+  accept_df(h);
 }
 
 // Bound of one dependency wait of the H-LU executor, in SM clock cycles:
@@ -1293,14 +1307,9 @@ bool build_hlu_device(bem_handle* h) {
   CK(cudaGetLastError());
   launch_hlu_finite_check(h->dArena.p, P.arena, m.prec, h->dHCtrl.p + 3, h->nsm, s);
   h->launches++;
-  if (P.df_ok) {  // the sweeps' inverses, and their own check
+  if (P.df_ok) {
     h->hlu_prec = m.prec;
-    h->hlu_dev = true;
-    finish_df(h);
-    h->hlu_dev = false;
-    for (bem_handle::DfDev* d : {&h->dfL, &h->dfU})
-      launch_hlu_finite_check(d->minv.p, d->view.msize, m.prec, h->dHCtrl.p + 3, h->nsm, s);
-    h->launches += 2;
+    finish_df(h, {h->dArena.p, h->dArena.p});
   }
   int ctrl[4] = {0, 0, 0, 0};
   CK(cudaMemcpyAsync(ctrl, h->dHCtrl.p, sizeof(ctrl), cudaMemcpyDeviceToHost, s));
@@ -1316,8 +1325,9 @@ bool build_hlu_device(bem_handle* h) {
   h->dLl.upload(P.L.leaves, s);
   h->dUs.upload(P.U.schedule, s);
   h->dUl.upload(P.U.leaves, s);
-  h->df_ok = P.df_ok;
+  h->df_ok = false;
   h->df_why = P.df_why;
+  if (P.df_ok) accept_df(h);
   CK(cudaStreamSynchronize(s));
   h->hlu_dev = true;
   h->have_hlu = true;

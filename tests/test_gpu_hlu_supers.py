@@ -1,0 +1,70 @@
+"""The dense inverses of the H-LU sweeps' diagonal blocks: what they hold where
+the factors hold nothing, and how they are built beside other handles."""
+import numpy as np
+import pytest
+
+from conftest import rel
+
+pytestmark = pytest.mark.gpu
+
+
+def _plate(n, axis):
+    """2 n^2 triangles of the unit square through the origin normal to `axis`,
+    with exact coordinates: no element sees another one of its own plate."""
+    u, v = [a for a in range(3) if a != axis]
+    g = np.arange(n + 1) / n
+    tri = []
+    for i in range(n):
+        for j in range(n):
+            c = np.zeros((4, 3))
+            c[:, u] = g[[i, i + 1, i + 1, i]]
+            c[:, v] = g[[j, j, j + 1, j + 1]]
+            tri += [c[[0, 1, 2]].ravel(), c[[0, 2, 3]].ravel()]
+    return np.array(tri)
+
+
+def _factors(s):
+    return [s.hlu_export(which)[:2] for which in (0, 1)]
+
+
+def _leafwise(orc, factors, n, B):
+    (Ll, Ld), (Ul, Ud) = factors
+    return np.stack([orc.upper_solve(n, Ul, Ud, orc.lower_solve(n, Ll, Ld, B[:, q]))
+                     for q in range(B.shape[1])], axis=1)
+
+
+def _absent(factors, info, n, span):
+    """Far blocks within `span` rows and columns of each other that no leaf of
+    either factor covers."""
+    held = np.zeros((n, n), bool)
+    for leaves, _ in factors:
+        for r0, m, c0, nn, *_ in leaves:
+            held[r0:r0 + m, c0:c0 + nn] = True
+    return sum(1 for r0, m, c0, nn, adm in info
+               if adm and max(r0 + m, c0 + nn) - min(r0, c0) <= span
+               and not held[r0:r0 + m, c0:c0 + nn].any())
+
+
+@pytest.mark.parametrize("precision,rank", [(0, 8), (0, 2), (1, 2)])
+def test_blocks_without_a_leaf_are_zero(bem, orc, precision, rank):
+    """Rigid plates at a right angle, coupling 0: far blocks inside a plate are
+    exactly zero, so the host factorization drops their leaves. One handle
+    factorizes a full matrix (soft walls) first, then the rigid one at two
+    frequencies: the sweeps are those of the factors (FP64 1e-11, FP32 1e-4, as
+    for the other tests of the sweeps against the leaf-by-leaf solves)."""
+    tri = np.vstack([_plate(24, 0), _plate(24, 2) + np.tile([0.25, 0.0, 0.0], 3)])
+    n = tri.shape[0]
+    s = bem.Solver(precision=precision, aca_tol=1e-6, leaf_size=32, coupling=0, hlu_device=0,
+                   precond_rank=rank, precond_tol=1e-8)
+    s.set_mesh(tri)
+    rng = np.random.default_rng(4)
+    B = rng.standard_normal((n, 3)) + 1j * rng.standard_normal((n, 3))
+    for k, (a, b, freq) in enumerate([(1.0, 0.0, 300.0), (0.0, 1.0, 300.0), (0.0, 1.0, 500.0)]):
+        s.set_bc(np.full(n, a), np.full(n, b))
+        s.assemble(freq)
+        s.hlu_build()
+        assert s.hlu_sweep_kind() == 1
+        factors = _factors(s)
+        assert (_absent(factors, s.partition(), n, 128) > 0) == (k > 0)
+        assert rel(s.hlu_solve(B), _leafwise(orc, factors, n, B)) < (1e-11, 1e-4)[precision], k
+    s.close()
