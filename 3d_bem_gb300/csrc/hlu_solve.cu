@@ -743,18 +743,24 @@ __global__ void __launch_bounds__(IT) df_invert_kernel(HluDfDev p, const T2* __r
   }
 }
 
-template <typename T2, int RT>
-void df_launch(const DfArgs& a, int grid, cudaStream_t s) {
-  // above 48 KiB a kernel's shared memory has to be asked for, once per device
-  static std::atomic<uint64_t> ready{0};
+// Above 48 KiB a kernel's shared memory has to be asked for, once per device. The
+// limit is the kernel's, not a handle's or a stream's, so `most` is what any launch
+// of it can need: a smaller value would fail another thread's launch.
+template <typename K>
+void allow_smem(K* kernel, size_t most, std::atomic<uint64_t>& ready) {
   int dev = 0;
   CUDA_OK(cudaGetDevice(&dev));
   const uint64_t bit = 1ull << (dev & 63);
   if (dev >= 64 || !(ready.load() & bit)) {
-    CUDA_OK(cudaFuncSetAttribute(hlu_df_kernel<T2, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)df_smem<T2, RT>()));
+    CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     ready |= bit;
   }
+}
+
+template <typename T2, int RT>
+void df_launch(const DfArgs& a, int grid, cudaStream_t s) {
+  static std::atomic<uint64_t> ready{0};
+  allow_smem(hlu_df_kernel<T2, RT>, df_smem<T2, RT>(), ready);
   hlu_df_kernel<T2, RT><<<grid, DT, df_smem<T2, RT>(), s>>>(a);
 }
 
@@ -766,11 +772,17 @@ void df_launch_r(const DfArgs& a, int grid, cudaStream_t s) {
   else df_launch<T2, 8>(a, grid, s);
 }
 
+// shared memory of the inversion of blocks of up to m rows
+template <typename T2, int PW>
+constexpr size_t df_invert_smem(int m) {
+  return (size_t)(m + HLU_DF_MAX_M) * (PW + 1) * sizeof(T2);
+}
+
 template <typename T2, int PW>
 void df_invert(const HluDfDev& p, const void* data, void* dense, cudaStream_t s) {
-  const size_t smem = (size_t)(p.maxm + HLU_DF_MAX_M) * (PW + 1) * sizeof(T2);
-  CUDA_OK(cudaFuncSetAttribute(df_invert_kernel<T2, PW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
+  static std::atomic<uint64_t> ready{0};
+  allow_smem(df_invert_kernel<T2, PW>, df_invert_smem<T2, PW>(HLU_DF_SUPER), ready);
+  const size_t smem = df_invert_smem<T2, PW>(p.maxm);
   if (p.ninner > 0)
     df_expand_kernel<T2><<<(unsigned)p.ninner, 128, 0, s>>>(p.inner, (const T2*)data, (T2*)dense);
   df_invert_kernel<T2, PW><<<(unsigned)p.npanels, IT, smem, s>>>(p, (const T2*)dense);

@@ -1,5 +1,7 @@
 """The dense inverses of the H-LU sweeps' diagonal blocks: what they hold where
 the factors hold nothing, and how they are built beside other handles."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -68,3 +70,41 @@ def test_blocks_without_a_leaf_are_zero(bem, orc, precision, rank):
         assert (_absent(factors, s.partition(), n, 128) > 0) == (k > 0)
         assert rel(s.hlu_solve(B), _leafwise(orc, factors, n, B)) < (1e-11, 1e-4)[precision], k
     s.close()
+
+
+def test_factorizations_in_threads(bem, meshes):
+    """Factors of a body with diagonal blocks of hundreds of rows while other
+    threads factorize a tiny one: a launch's shared memory does not depend on
+    what other handles launched last."""
+    def handle(tri):
+        s = bem.Solver(precision=1, precond_rank=2, leaf_size=32, aca_tol=1e-5)
+        s.set_mesh(tri)
+        s.set_bc(np.zeros(len(tri)), np.ones(len(tri)))
+        s.assemble(300.0)
+        return s
+
+    large = handle(meshes.icosphere(3, 1.0))
+    small = [handle(meshes.box(n_target=12, seed=3)[:12]) for _ in range(3)]
+    done, errors = threading.Event(), []
+
+    def rebuild(s):
+        try:
+            while not done.is_set():
+                s.hlu_build()
+        except Exception as e:  # noqa: BLE001 -- reported below
+            errors.append(e)
+
+    threads = [threading.Thread(target=rebuild, args=(s,)) for s in small]
+    for t in threads:
+        t.start()
+    try:
+        for _ in range(200):
+            large.hlu_build()
+    except Exception as e:  # noqa: BLE001
+        errors.append(e)
+    done.set()
+    for t in threads:
+        t.join()
+    assert not errors
+    for s in (large, *small):
+        s.close()
