@@ -214,9 +214,10 @@ struct bem_handle {
     DBuf<HluDfPanel> panels;
     DBuf<int32_t> need;
     DBuf<unsigned char> diag, minv;
+    std::vector<HluDfBatch> batches;
     HluDfDev view;
   } dfL, dfU;
-  DBuf<unsigned char> dfDense;  // dense diagonal blocks while they are inverted
+  DBuf<unsigned char> dfDense;  // dense diagonal blocks of a batch while they are inverted
   bool df_ok = false;
   int df_helpers = 32;  // helper CTAs per dataflow sweep (12 while concurrent sweep workers run)
   int hlu_ctas_per_sm = 0;  // > 0: the executor's grid, per SM, below hp_grid (sweep workers)
@@ -927,46 +928,56 @@ void upload_df_plan(bem_handle* h, const HluDfPlan& p, int prec, bem_handle::DfD
   v.nt = p.nt;
   v.msize = p.msize;
   v.nitems = (int)p.items.size();
-  v.ninner = (int)p.inner.size();
-  v.npanels = (int)panels.size();
   v.D = p.D();
   v.lower = p.lower ? 1 : 0;
   for (const HluDfSuper& u : p.supers) v.maxm = std::max(v.maxm, u.m);
   d.view = v;
+  d.batches = p.batches(panels, HLU_DF_BATCH);
 }
 
 // The sweeps' vectors and flags, and the inverses of the supers' diagonal blocks
 // (views of both plans set; data: the leaf values of both factors on the device).
-// dfErr[1] is set when a value of the inverses is not finite.
+// df_ok and df_why: the leaf-by-leaf sweeps, which take next to no memory, run
+// instead where these buffers do not fit on the device or an inverse is not finite.
 void finish_df(bem_handle* h, const void* const (&data)[2]) {
   cudaStream_t s = h->stream;
   const size_t cs = h->hlu_prec == 0 ? sizeof(double2) : sizeof(float2);
   bem_handle::DfDev* d[2] = {&h->dfL, &h->dfU};
-  h->dfXi.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
-  h->dfS.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
-  h->dfT.ensure((size_t)HLU_DF_MAX_R * std::max<int64_t>({d[0]->view.nt, d[1]->view.nt, 1}) * cs);
-  h->dfCtrl.ensure((size_t)(1 + 3 * std::max(d[0]->view.D, d[1]->view.D)));
-  h->dfErr.ensure(2);
-  CK(cudaMemsetAsync(h->dfErr.p, 0, 2 * sizeof(int), s));
-  h->dfDense.ensure((size_t)std::max(d[0]->view.msize, d[1]->view.msize) * cs);
+  h->df_ok = false;
+  h->df_why.clear();
+  int64_t most = 0;
+  for (const bem_handle::DfDev* f : d)
+    for (const HluDfBatch& b : f->batches) most = std::max(most, b.size);
+  try {
+    h->dfXi.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
+    h->dfS.ensure((size_t)HLU_DF_MAX_R * h->N * cs);
+    h->dfT.ensure((size_t)HLU_DF_MAX_R * std::max<int64_t>({d[0]->view.nt, d[1]->view.nt, 1}) * cs);
+    h->dfCtrl.ensure((size_t)(1 + 3 * std::max(d[0]->view.D, d[1]->view.D)));
+    h->dfErr.ensure(2);
+    h->dfDense.ensure((size_t)most * cs);
+    for (bem_handle::DfDev* f : d) {
+      f->minv.ensure((size_t)f->view.msize * cs);
+      f->view.minv = f->minv.p;
+    }
+  } catch (const BemError& e) {
+    if (e.st != BEM_ENOMEM) throw;
+    cudaGetLastError();
+    h->dfDense.release();
+    for (bem_handle::DfDev* f : d) f->minv.release();
+    h->df_why = "no device memory for the inverses of the diagonal blocks";
+    return;
+  }
+  CK(cudaMemsetAsync(h->dfErr.p, 0, 2 * sizeof(int), s));  // sticky error, not finite
   for (int q = 0; q < 2; q++) {
-    d[q]->minv.ensure((size_t)d[q]->view.msize * cs);
-    d[q]->view.minv = d[q]->minv.p;
-    // blocks without a leaf (rank 0) are zero, whatever the buffer held before
-    CK(cudaMemsetAsync(h->dfDense.p, 0, (size_t)d[q]->view.msize * cs, s));
-    h->launches += launch_hlu_df_invert(d[q]->view, data[q], h->hlu_prec, h->dfDense.p, s);
+    for (const HluDfBatch& b : d[q]->batches)
+      h->launches += launch_hlu_df_invert(d[q]->view, b, data[q], h->hlu_prec, h->dfDense.p, s);
     launch_hlu_finite_check(d[q]->minv.p, d[q]->view.msize, h->hlu_prec, h->dfErr.p + 1, h->nsm, s);
     h->launches++;
   }
   CK(cudaGetLastError());
-}
-
-// After finish_df: the dataflow sweeps run when the inverses are finite, else the
-// leaf-by-leaf ones, which need no inverse.
-void accept_df(bem_handle* h) {
   int bad = 0;
-  CK(cudaMemcpyAsync(&bad, h->dfErr.p + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  CK(cudaMemcpyAsync(&bad, h->dfErr.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
   h->df_ok = !bad;
   if (bad) h->df_why = "the inverse of a diagonal block is not finite";
 }
@@ -999,7 +1010,6 @@ void upload_df_plans(bem_handle* h) {
     d.view.diag = d.diag.p;
   }
   finish_df(h, {h->dLd.p, h->dUd.p});
-  accept_df(h);
 }
 
 // Bound of one dependency wait of the H-LU executor, in SM clock cycles:
@@ -1307,10 +1317,6 @@ bool build_hlu_device(bem_handle* h) {
   CK(cudaGetLastError());
   launch_hlu_finite_check(h->dArena.p, P.arena, m.prec, h->dHCtrl.p + 3, h->nsm, s);
   h->launches++;
-  if (P.df_ok) {
-    h->hlu_prec = m.prec;
-    finish_df(h, {h->dArena.p, h->dArena.p});
-  }
   int ctrl[4] = {0, 0, 0, 0};
   CK(cudaMemcpyAsync(ctrl, h->dHCtrl.p, sizeof(ctrl), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
@@ -1325,9 +1331,12 @@ bool build_hlu_device(bem_handle* h) {
   h->dLl.upload(P.L.leaves, s);
   h->dUs.upload(P.U.schedule, s);
   h->dUl.upload(P.U.leaves, s);
-  h->df_ok = false;
-  h->df_why = P.df_why;
-  if (P.df_ok) accept_df(h);
+  if (P.df_ok) {
+    finish_df(h, {h->dArena.p, h->dArena.p});
+  } else {
+    h->df_ok = false;
+    h->df_why = P.df_why;
+  }
   CK(cudaStreamSynchronize(s));
   h->hlu_dev = true;
   h->have_hlu = true;

@@ -833,6 +833,29 @@ std::vector<HluDfPanel> HluDfPlan::panels(int precision) const {
   return v;
 }
 
+std::vector<HluDfBatch> HluDfPlan::batches(const std::vector<HluDfPanel>& panels,
+                                           int64_t most) const {
+  std::vector<HluDfBatch> v;
+  size_t in = 0, pn = 0;
+  for (int i = 0; i < D(); i++) {
+    const int64_t beg = supers[i].moff, end = i + 1 < D() ? supers[i + 1].moff : msize;
+    if (v.empty() || end - v.back().moff > most) {
+      HluDfBatch b;
+      b.inner_beg = (int32_t)in;
+      b.panel_beg = (int32_t)pn;
+      b.moff = beg;
+      v.push_back(b);
+    }
+    HluDfBatch& b = v.back();
+    while (in < inner.size() && inner[in].dst < end) in++;
+    while (pn < panels.size() && panels[pn].super == i) pn++;
+    b.ninner = (int32_t)in - b.inner_beg;
+    b.npanels = (int32_t)pn - b.panel_beg;
+    b.size = end - b.moff;
+  }
+  return v;
+}
+
 namespace {
 bool df_plan_impl(const FlatFactor& f, int64_t N, const std::vector<int64_t>& cuts, HluDfPlan& p,
                   std::string* why, bool with_diag) {
@@ -951,6 +974,9 @@ bool df_plan_impl(const FlatFactor& f, int64_t N, const std::vector<int64_t>& cu
     }
   }
   if (p.nt > INT32_MAX / 2) return fail("too many low-rank leaves");
+  std::stable_sort(p.inner.begin(), p.inner.end(), [](const HluDfInner& x, const HluDfInner& y) {
+    return x.dst < y.dst;
+  });
   // items in claim order: ROW(I), DIAG(I), DOT(I) (an empty DOT item keeps the
   // chain DOT(I) after DOT(I - 1))
   p.need.assign(3 * (size_t)D, 0);

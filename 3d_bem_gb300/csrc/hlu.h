@@ -61,7 +61,7 @@ struct HluDfPlan {
   std::vector<HluDfItem> items;
   std::vector<HluDfColumn> columns;
   std::vector<HluDfDot> dots;
-  std::vector<HluDfInner> inner;
+  std::vector<HluDfInner> inner;  // by super
   std::vector<HluDfChunk> chunks;
   std::vector<HluDfSuper> supers;
   std::vector<int32_t> need;  // 3 per super
@@ -70,6 +70,9 @@ struct HluDfPlan {
   bool lower = false;
   int D() const { return (int)supers.size(); }
   std::vector<HluDfPanel> panels(int precision) const;
+  // the inversion in runs of supers with at most `most` values of dense blocks each
+  // (one super at least)
+  std::vector<HluDfBatch> batches(const std::vector<HluDfPanel>& panels, int64_t most) const;
 };
 
 // Row boundaries of the supers: the cluster-tree nodes of at most

@@ -653,11 +653,12 @@ __global__ void __launch_bounds__(DT, 1) hlu_df_kernel(DfArgs a) {
 
 // ---- inverses of the supers' diagonal blocks ----
 
-// one CTA per leaf inside a diagonal block: its entries into the dense copy
+// one CTA per leaf inside a diagonal block: its entries into the dense copy, which
+// starts at value d0 of all the dense blocks
 template <typename T2>
 __global__ void __launch_bounds__(128) df_expand_kernel(const HluDfInner* __restrict__ inner,
                                                         const T2* __restrict__ data,
-                                                        T2* __restrict__ dense) {
+                                                        T2* __restrict__ dense, int64_t d0) {
   const HluDfInner in = inner[blockIdx.x];
   const T2* D = data + in.off;
   for (int e = threadIdx.x; e < in.m * in.n; e += 128) {
@@ -670,7 +671,7 @@ __global__ void __launch_bounds__(128) df_expand_kernel(const HluDfInner* __rest
     } else {
       v = D[(int64_t)c * in.m + r];
     }
-    dense[in.dst + (int64_t)r * in.ld + c] = v;
+    dense[in.dst - d0 + (int64_t)r * in.ld + c] = v;
   }
 }
 
@@ -679,16 +680,17 @@ __global__ void __launch_bounds__(128) df_expand_kernel(const HluDfInner* __rest
 // rows of a chunk; the dense block's entries are read as broadcasts.
 constexpr int IT = 256;
 template <typename T2, int PW>
-__global__ void __launch_bounds__(IT) df_invert_kernel(HluDfDev p, const T2* __restrict__ dense) {
+__global__ void __launch_bounds__(IT) df_invert_kernel(HluDfDev p, int panel_beg,
+                                                       const T2* __restrict__ dense, int64_t d0) {
   extern __shared__ __align__(16) unsigned char raw[];
   constexpr int LD = PW + 1, SUB = 32 / PW, RSTEP = (IT / 32) * SUB;
   constexpr int RT = (HLU_DF_MAX_M + RSTEP - 1) / RSTEP;
-  const HluDfPanel pn = p.panels[blockIdx.x];
+  const HluDfPanel pn = p.panels[panel_beg + blockIdx.x];
   const HluDfSuper su = p.supers[pn.super];
   const int m = su.m, w = min(PW, m - pn.p0);
   T2* X = (T2*)raw;  // [row][column]
   T2* tmp = X + (int64_t)m * LD;
-  const T2* D = dense + su.moff;
+  const T2* D = dense + (su.moff - d0);
   const int tid = threadIdx.x, lane = tid & 31, c = lane % PW;
   const int rs = (tid >> 5) * SUB + lane / PW;  // the thread's first row of a chunk
   for (int e = tid; e < m * LD; e += IT) X[e] = mk<T2>(0, 0);
@@ -779,23 +781,27 @@ constexpr size_t df_invert_smem(int m) {
 }
 
 template <typename T2, int PW>
-void df_invert(const HluDfDev& p, const void* data, void* dense, cudaStream_t s) {
+int df_invert(const HluDfDev& p, const HluDfBatch& b, const void* data, void* dense,
+              cudaStream_t s) {
   static std::atomic<uint64_t> ready{0};
   allow_smem(df_invert_kernel<T2, PW>, df_invert_smem<T2, PW>(HLU_DF_SUPER), ready);
-  const size_t smem = df_invert_smem<T2, PW>(p.maxm);
-  if (p.ninner > 0)
-    df_expand_kernel<T2><<<(unsigned)p.ninner, 128, 0, s>>>(p.inner, (const T2*)data, (T2*)dense);
-  df_invert_kernel<T2, PW><<<(unsigned)p.npanels, IT, smem, s>>>(p, (const T2*)dense);
+  // blocks without a leaf (rank 0) are zero, whatever the buffer held before
+  CUDA_OK(cudaMemsetAsync(dense, 0, (size_t)b.size * sizeof(T2), s));
+  if (b.ninner > 0)
+    df_expand_kernel<T2><<<(unsigned)b.ninner, 128, 0, s>>>(p.inner + b.inner_beg, (const T2*)data,
+                                                            (T2*)dense, b.moff);
+  df_invert_kernel<T2, PW><<<(unsigned)b.npanels, IT, df_invert_smem<T2, PW>(p.maxm), s>>>(
+      p, b.panel_beg, (const T2*)dense, b.moff);
+  return 1 + (b.ninner > 0);
 }
 
 }  // namespace
 
-int launch_hlu_df_invert(const HluDfDev& p, const void* data, int precision, void* dense,
-                         cudaStream_t s) {
-  if (p.D <= 0) return 0;
-  if (precision == 0) df_invert<double2, hlu_df_panel_cols(0)>(p, data, dense, s);
-  else df_invert<float2, hlu_df_panel_cols(1)>(p, data, dense, s);
-  return 1 + (p.ninner > 0);
+int launch_hlu_df_invert(const HluDfDev& p, const HluDfBatch& b, const void* data, int precision,
+                         void* dense, cudaStream_t s) {
+  if (b.npanels <= 0) return 0;
+  return precision == 0 ? df_invert<double2, hlu_df_panel_cols(0)>(p, b, data, dense, s)
+                        : df_invert<float2, hlu_df_panel_cols(1)>(p, b, data, dense, s);
 }
 
 int launch_hlu_df(const HluDfDev& p, const void* data, int precision, const double2* w, double2* x,

@@ -98,7 +98,7 @@ struct HluDfDev {
   void* minv = nullptr;           // inverses of the supers' diagonal blocks
   int64_t nt = 0;                 // values of t
   int64_t msize = 0;              // values of minv
-  int nitems = 0, ninner = 0, npanels = 0, D = 0, lower = 0;
+  int nitems = 0, D = 0, lower = 0;
   int maxm = 0;                   // rows of the largest super
 };
 
@@ -117,10 +117,22 @@ struct HluDfWork {
   unsigned long long wait_ns = 10000000000ull;
 };
 
-// Inverses of the supers' diagonal blocks from the factor's leaves (data) and
-// apply matrices; dense: msize values of scratch. Returns the kernels launched.
-int launch_hlu_df_invert(const HluDfDev& p, const void* data, int precision, void* dense,
-                         cudaStream_t s);
+// A run of consecutive supers that are inverted together: their leaves and panels,
+// and the range of their dense blocks (and inverses) among all of them.
+struct HluDfBatch {
+  int32_t inner_beg = 0, ninner = 0, panel_beg = 0, npanels = 0;
+  int64_t moff = 0, size = 0;
+};
+// Values of the dense copies that are inverted at a time: the copies are scratch of
+// every handle, so they are not all made at once (64 MiB in complex FP32; at 81,920
+// pencil elements all of them would take 210 MB).
+constexpr int64_t HLU_DF_BATCH = 8 << 20;
+
+// Inverses of the diagonal blocks of a batch of supers from the factor's leaves
+// (data) and apply matrices; dense: b.size values of scratch, cleared here. Returns
+// the kernels launched.
+int launch_hlu_df_invert(const HluDfDev& p, const HluDfBatch& b, const void* data, int precision,
+                         void* dense, cudaStream_t s);
 
 // w (R x N) -> x (R x N) with one launch of 1 + `helpers` CTAs (R <=
 // HLU_DF_MAX_R; w is only read). Returns the kernels launched.

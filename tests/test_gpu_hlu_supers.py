@@ -1,11 +1,14 @@
 """The dense inverses of the H-LU sweeps' diagonal blocks: what they hold where
 the factors hold nothing, and how they are built beside other handles."""
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
 import pytest
 
-from conftest import rel
+from conftest import ROOT, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -108,3 +111,72 @@ def test_factorizations_in_threads(bem, meshes):
     assert not errors
     for s in (large, *small):
         s.close()
+
+
+def test_sweeps_without_room_for_inverses(tmp_path):
+    """With less device memory than the inverses take (a cap on the library's
+    allocations, in child processes) the factors are built all the same and the
+    leaf-by-leaf sweeps solve with them. The least cap that is enough is found
+    by bisection; there the inverses have no room."""
+    code = r"""
+import importlib, sys, numpy as np
+sys.path.insert(0, sys.argv[1])
+bem = importlib.import_module("3d_bem_gb300")
+meshes = importlib.import_module("3d_bem_gb300.meshes")
+tri = meshes.icosphere(3, 1.0); n = tri.shape[0]
+s = bem.Solver(precision=0, aca_tol=1e-5, precond_rank=2, leaf_size=32)
+s.set_mesh(tri); s.set_bc(np.zeros(n), np.ones(n))
+try:
+    s.assemble(300.0); s.hlu_build()
+    b = np.random.default_rng(1).standard_normal(n) + 0j
+    x = s.hlu_solve(b)
+except bem.BemError as e:
+    print("STATUS", e.status)
+else:
+    np.save(sys.argv[2], x)
+    print("KIND", s.hlu_sweep_kind())
+"""
+    def run(mib):
+        out = str(tmp_path / f"x{mib}.npy")
+        env = dict(os.environ)
+        env.pop("BEM_DEVICE_MEM_CAP", None)
+        if mib:
+            env["BEM_DEVICE_MEM_CAP"] = str(mib << 20)
+        r = subprocess.run([sys.executable, "-c", code, ROOT, out], env=env, capture_output=True,
+                           text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        word, value = r.stdout.split()
+        if word == "STATUS":
+            assert int(value) == 2  # BEM_ENOMEM
+            return None, None
+        return int(value), np.load(out)
+
+    kind, x = run(0)
+    assert kind == 1
+    lo, hi = 0, 512
+    while hi - lo > 2:
+        mid = (lo + hi) // 2
+        if run(mid)[0] is None:
+            lo = mid
+        else:
+            hi = mid
+    kind, y = run(hi)
+    assert kind == 0
+    assert rel(y, x) < 1e-11
+
+
+def test_inverses_in_batches(bem, meshes, orc):
+    """40,960 elements: the dense blocks of all supers (about 13 million values)
+    are inverted in two batches. FP32 factors: 1e-4, as for the other tests."""
+    tri = meshes.pencil(n_target=40960)
+    n = tri.shape[0]
+    s = bem.Solver(precision=1, aca_tol=1e-4, precond_rank=2, leaf_size=32, wave_speed=343.0)
+    s.set_mesh(tri)
+    s.set_bc_impedance(meshes.wall_admittance(n))
+    s.assemble(1000.0)
+    s.hlu_build()
+    assert s.hlu_sweep_kind() == 1
+    rng = np.random.default_rng(2)
+    B = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    assert rel(s.hlu_solve(B), _leafwise(orc, _factors(s), n, B)) < 1e-4
+    s.close()
