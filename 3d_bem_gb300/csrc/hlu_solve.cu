@@ -430,16 +430,85 @@ __device__ bool df_row_item(const DfArgs& a, const HluDfItem& it, T2* sm) {
   __syncthreads();
   if (orr < RT && orow < it.m) {
     T2 v = mk<T2>((typename HC<T2>::R)wv.x, (typename HC<T2>::R)wv.y);
-    T2 sum = mk<T2>(0, 0);
+    T2 sum[NW];  // pairwise
 #pragma unroll
-    for (int q = 0; q < NW; q++) cacc(sum, part[(q * RT + orr) * 32 + orow]);
-    v.x -= sum.x;
-    v.y -= sum.y;
+    for (int q = 0; q < NW; q++) sum[q] = part[(q * RT + orr) * 32 + orow];
+#pragma unroll
+    for (int n = NW / 2; n >= 1; n /= 2)
+#pragma unroll
+      for (int q = 0; q < n; q++) cacc(sum[q], sum[q + n]);
+    v.x -= sum[0].x;
+    v.y -= sum[0].y;
     ((T2*)a.s)[(int64_t)(it.r0 + orow) * RT + orr] = v;
   }
   df_publish(a, it);
   return true;
 }
+
+// hi + lo += v, the rounding error of hi + v kept in lo (Knuth's TwoSum)
+template <typename R>
+__device__ __forceinline__ void two_sum(R& hi, R& lo, R v) {
+  const R s = hi + v, b = s - hi;
+  lo += (hi - (s - b)) + (v - b);
+  hi = s;
+}
+
+// The sum of the 32 partial sums of a row of M s: compensated in FP32, pairwise in
+// FP64, whose pipe has no room for the compensation. A row of an inverse has
+// hundreds of columns where a leaf has some 22, and with these sums in order the
+// sweeps were further from the exact solve than leaf by leaf: 8 FP32 vectors,
+// sphere of 1,280 elements 1.47e-7 (leaf by leaf 1.33e-7, now 1.14e-7), pencil of
+// 20,480 1.35e-7 (1.28e-7, 1.09e-7). FP64, sphere of 1,280: 2.54e-16 (2.39e-16,
+// 2.33e-16). Cost at 20,480 elements and 8 vectors: 2.01 -> 2.05 ms.
+template <typename T2>
+struct Joined {  // FP64
+  T2 hi;
+  __device__ __forceinline__ void join(const T2 (&p)[8]) {
+    T2 a = p[0], b = p[2], c = p[4], d = p[6];
+    cacc(a, p[1]);
+    cacc(b, p[3]);
+    cacc(c, p[5]);
+    cacc(d, p[7]);
+    cacc(a, b);
+    cacc(c, d);
+    cacc(a, c);
+    hi = a;
+  }
+  __device__ __forceinline__ void store(T2* s, int i, int) const { s[i] = hi; }
+  // this thread's sum and those of i + n, i + 2 n, i + 3 n
+  __device__ __forceinline__ T2 join_stored(const T2* s, int i, int n) const {
+    T2 a = hi, b = s[2 * n + i];
+    cacc(a, s[n + i]);
+    cacc(b, s[3 * n + i]);
+    cacc(a, b);
+    return a;
+  }
+};
+template <>
+struct Joined<float2> {
+  float2 hi, lo;
+  __device__ __forceinline__ void add(float2 v) {
+    two_sum(hi.x, lo.x, v.x);
+    two_sum(hi.y, lo.y, v.y);
+  }
+  __device__ __forceinline__ void join(const float2 (&p)[8]) {
+    hi = p[0];
+    lo = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int q = 1; q < 8; q++) add(p[q]);
+  }
+  __device__ __forceinline__ void store(float2* s, int i, int n) const {
+    s[i] = hi;
+    s[n + i] = lo;
+  }
+  __device__ __forceinline__ float2 join_stored(const float2* s, int i, int n) {
+#pragma unroll
+    for (int q = 1; q < 4; q++) add(s[q * n + i]);
+#pragma unroll
+    for (int q = 1; q < 4; q++) cacc(lo, s[(4 + q) * n + i]);
+    return make_float2(hi.x + lo.x, hi.y + lo.y);
+  }
+};
 
 // DIAG: 16 rows of x = M s. Lanes are 16 rows x 2 columns, warp w takes the
 // columns c0 + 2 w + (0, 1), then every 32nd; the entries of M are held in
@@ -481,24 +550,24 @@ __device__ bool df_diag_item(const DfArgs& a, const HluDfItem& it, T2* sm) {
     for (int r = 0; r < RT; r++) cmac(acc[r], v, sv[c * RT + r]);
   }
   // partial sums [2 warp + half][r][row]; four threads per output add 8 of the
-  // 32 each in order, then one the four
+  // 32 each, then one the four
   T2* pw = part + (2 * warp + (lane >> 4)) * 16 * RT + (lane & 15);
 #pragma unroll
   for (int r = 0; r < RT; r++) pw[r * 16] = acc[r];
   __syncthreads();
   constexpr int NO = 16 * RT;
-  T2 v = mk<T2>(0, 0);
+  Joined<T2> j;
   if (tid < 4 * NO) {
     const T2* pp = part + (tid / NO) * (2 * NW / 4) * NO + tid % NO;
+    T2 p[2 * NW / 4];
 #pragma unroll
-    for (int q = 0; q < 2 * NW / 4; q++) cacc(v, pp[q * NO]);
-    sv[tid] = v;  // s is no longer read
+    for (int q = 0; q < 2 * NW / 4; q++) p[q] = pp[q * NO];
+    j.join(p);
+    j.store(sv, tid, 4 * NO);  // s is no longer read
   }
   __syncthreads();
   if (tid < NO) {
-    cacc(v, sv[NO + tid]);
-    cacc(v, sv[2 * NO + tid]);
-    cacc(v, sv[3 * NO + tid]);
+    const T2 v = j.join_stored(sv, tid, NO);
     const int orow = tid & 15, r = tid >> 4;
     if (orow < nrow) {
       const int64_t g = (int64_t)it.r0 + it.t0 + orow;
@@ -679,6 +748,9 @@ __global__ void __launch_bounds__(128) df_expand_kernel(const HluDfInner* __rest
 // vectors, the panel in shared memory, lanes over its columns, warps over the
 // rows of a chunk; the dense block's entries are read as broadcasts.
 constexpr int IT = 256;
+// Columns of a plain sum; sums of sums are compensated. A thread's one sum over all
+// columns before (up to 480) made the inverse a little worse than its storage.
+constexpr int KB = 8;
 template <typename T2, int PW>
 __global__ void __launch_bounds__(IT) df_invert_kernel(HluDfDev p, int panel_beg,
                                                        const T2* __restrict__ dense, int64_t d0) {
@@ -707,23 +779,35 @@ __global__ void __launch_bounds__(IT) df_invert_kernel(HluDfDev p, int panel_beg
     }
     // rows already solved: [f0, a) going down, [b, f1) going up
     const int k0 = p.lower ? f0 : b, k1 = p.lower ? a : f1;
-    T2 acc[RT];
+    T2 acc[RT], low[RT];
 #pragma unroll
-    for (int t = 0; t < RT; t++) acc[t] = mk<T2>(0, 0);
+    for (int t = 0; t < RT; t++) acc[t] = low[t] = mk<T2>(0, 0);
     const T2* row[RT];
 #pragma unroll
     for (int t = 0; t < RT; t++) row[t] = D + (int64_t)min(a + rs + t * RSTEP, b - 1) * m;
-#pragma unroll 4
-    for (int k = k0; k < k1; k++) {
-      const T2 xv = X[k * LD + c];
+    for (int k = k0; k < k1; k += KB) {
+      T2 part[RT];
 #pragma unroll
-      for (int t = 0; t < RT; t++) cmac(acc[t], HC<T2>::ld(row[t] + k), xv);
+      for (int t = 0; t < RT; t++) part[t] = mk<T2>(0, 0);
+      const int ke = min(k + KB, k1);
+#pragma unroll 4
+      for (int q = k; q < ke; q++) {
+        const T2 xv = X[q * LD + c];
+#pragma unroll
+        for (int t = 0; t < RT; t++) cmac(part[t], HC<T2>::ld(row[t] + q), xv);
+      }
+#pragma unroll
+      for (int t = 0; t < RT; t++) {
+        two_sum(acc[t].x, low[t].x, part[t].x);
+        two_sum(acc[t].y, low[t].y, part[t].y);
+      }
     }
 #pragma unroll
     for (int t = 0; t < RT; t++) {
       const int r = rs + t * RSTEP;
       if (r < ch.m)
-        tmp[r * LD + c] = mk<T2>((a + r == pn.p0 + c ? 1 : 0) - acc[t].x, -acc[t].y);
+        tmp[r * LD + c] = mk<T2>(((a + r == pn.p0 + c ? 1 : 0) - acc[t].x) - low[t].x,
+                                 -(acc[t].y + low[t].y));
     }
     __syncthreads();
     const T2* A = (const T2*)p.diag + ch.aoff;
@@ -731,9 +815,17 @@ __global__ void __launch_bounds__(IT) df_invert_kernel(HluDfDev p, int panel_beg
     for (int t = 0; t < RT; t++) {
       const int r = rs + t * RSTEP;
       if (r < ch.m) {
-        T2 v = mk<T2>(0, 0);
-        for (int k = 0; k < ch.m; k++) cmac(v, HC<T2>::ld(A + r * ch.m + k), tmp[k * LD + c]);
-        X[(a + r) * LD + c] = v;
+        T2 v[4];  // by quarters of the terms
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = mk<T2>(0, 0);
+        for (int k = 0; k < ch.m; k += 4)
+#pragma unroll
+          for (int e = 0; e < 4; e++)
+            if (k + e < ch.m) cmac(v[e], HC<T2>::ld(A + r * ch.m + k + e), tmp[(k + e) * LD + c]);
+        cacc(v[0], v[1]);
+        cacc(v[2], v[3]);
+        cacc(v[0], v[2]);
+        X[(a + r) * LD + c] = v[0];
       }
     }
     __syncthreads();
