@@ -284,8 +284,7 @@ __device__ __forceinline__ void field_points64(const FieldElem& e, double px, do
     const double rx = px - e.q[3 * i], ry = py - e.q[3 * i + 1], rz = pz - e.q[3 * i + 2];
     const double rr = fma(rx, rx, fma(ry, ry, rz * rz));
     const double ir = rsqrt(rr);
-    double r = rr * ir;
-    r = fma(0.5 * ir, fma(-r, r, rr), r);  // one correction: r to half an ulp
+    const double r = newton_sqrt(rr, ir);
     double sn, cs;
     if constexpr (FULL) sincos(k * r, &sn, &cs);
     else sincos_taylor<NS, NC>(fma(k, r, -krc), sn, cs);

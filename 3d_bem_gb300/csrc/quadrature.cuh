@@ -165,8 +165,7 @@ __device__ __forceinline__ void accumulate_fast(Ops& o, double w, const Elem& P,
   const double rx = P.c[0] - qx, ry = P.c[1] - qy, rz = P.c[2] - qz;
   const double rr = fma(rx, rx, fma(ry, ry, rz * rz));
   const double ir = rsqrt(rr);
-  double r = rr * ir;
-  r = fma(0.5 * ir, fma(-r, r, rr), r);  // one correction: r to half an ulp
+  const double r = newton_sqrt(rr, ir);
   const double kr = k * r;
   double sn, cs;
   if constexpr (FULL) sincos(kr, &sn, &cs);
