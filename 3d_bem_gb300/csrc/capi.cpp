@@ -1454,6 +1454,23 @@ const void* hlu_data(const bem_handle* h, int which) {
   return which ? h->dUd.p : h->dLd.p;
 }
 
+// mean phases of a traced lower sweep per level (appended to path): from the end of
+// the level before to the end of its ROW items, from there to that of the DIAG and
+// to that of the DOT items
+void df_trace_summary(bem_handle* h, const DBuf<unsigned long long>& tr, int R, const char* path) {
+  const int D = h->dfL.view.D;
+  std::vector<unsigned long long> t(1 + 3 * (size_t)D);
+  CK(cudaStreamSynchronize(h->stream));
+  CK(cudaMemcpy(t.data(), tr.p, t.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
+  double ph[3] = {};
+  for (size_t i = 0; i + 1 < t.size(); i++) ph[i % 3] += 1e-3 * (double)(t[i + 1] - t[i]) / D;
+  FILE* f = std::fopen(path, "a");
+  if (!f) return;
+  std::fprintf(f, "df L sweep: levels %d R %d total_us %.1f per level us: row %.3f diag %.3f dot %.3f\n",
+               D, R, 1e-3 * (double)(t.back() - t[0]), ph[0], ph[1], ph[2]);
+  std::fclose(f);
+}
+
 // w := U^{-1} L^{-1} w for R device vectors (LUPrecondidionedHMatrixWrapper's
 // two substitutions, gmres.h:134-147)
 void apply_precond(bem_handle* h, double2* w, int R, const int* gate_flags = nullptr) {
@@ -1465,13 +1482,23 @@ void apply_precond(bem_handle* h, double2* w, int R, const int* gate_flags = nul
     if (const char* e = std::getenv("BEM_DF_WAIT_US"))  // tests of the timeout path
       if (std::atof(e) > 0) ws.wait_ns = (unsigned long long)(std::atof(e) * 1000.0);
     const int hp = df_helpers(h);
+    // BEM_DF_TRACE=<file>: the lower sweep's phases, summarised into the file
+    const char* trace_path = std::getenv("BEM_DF_TRACE");
+    DBuf<unsigned long long> trace;
+    if (trace_path && *trace_path && !gate_flags) trace.ensure(1 + 3 * (size_t)h->dfL.view.D);
     for (int r0 = 0; r0 < R; r0 += HLU_DF_MAX_R) {
       const int rc = std::min(HLU_DF_MAX_R, R - r0);
       double2* wr = w + (size_t)r0 * N;
       const HmvGate gate = gate_flags ? HmvGate{gate_flags + r0 * GATE_STRIDE, GATE_STRIDE, rc}
                                       : HmvGate{nullptr, 0, 0};
+      if (trace.p) {
+        CK(cudaMemsetAsync(trace.p, 0, trace.n * sizeof(unsigned long long), s));
+        ws.trace = trace.p;
+      }
       h->launches += launch_hlu_df(h->dfL.view, hlu_data(h, 0), h->hlu_prec, wr, h->dP2.p, N, rc, ws,
                                    hp, s, gate);
+      ws.trace = nullptr;
+      if (trace.p) df_trace_summary(h, trace, rc, trace_path);
       h->launches += launch_hlu_df(h->dfU.view, hlu_data(h, 1), h->hlu_prec, h->dP2.p, wr, N, rc, ws,
                                    hp, s, gate);
     }

@@ -321,6 +321,7 @@ struct DfArgs {
   int* ctrl;  // [0] item counter, then per level the ROW, DIAG and DOT items done
   int* err;
   unsigned long long wait_ns;
+  unsigned long long* trace;  // HluDfWork::trace
   int64_t N;
   int R;
   HmvGate gate;
@@ -335,7 +336,10 @@ struct DfArgs {
 // barrier orders them before thread 0's release)
 __device__ __forceinline__ void df_publish(const DfArgs& a, const HluDfItem& it) {
   __syncthreads();
-  if (threadIdx.x == 0) add_release(a.done(it.level, it.type), 1);
+  if (threadIdx.x == 0) {
+    if (a.trace) atomicMax(a.trace + 1 + 3 * it.level + it.type, gtimer());
+    add_release(a.done(it.level, it.type), 1);
+  }
 }
 
 // shared memory: the warps' staged vectors (ROW) or the super's x / s, and the
@@ -707,7 +711,10 @@ __global__ void __launch_bounds__(DT, 1) hlu_df_kernel(DfArgs a) {
   if (gate_closed(a.gate)) return;  // every CTA reads the same flags
   while (true) {
     __syncthreads();
-    if (threadIdx.x == 0) sq = atomicAdd(a.ctrl, 1);
+    if (threadIdx.x == 0) {
+      sq = atomicAdd(a.ctrl, 1);
+      if (a.trace && sq == 0) a.trace[0] = gtimer();
+    }
     __syncthreads();
     const int q = sq;
     if (q >= a.p.nitems) return;
@@ -916,6 +923,7 @@ int launch_hlu_df(const HluDfDev& p, const void* data, int precision, const doub
   a.R = R;
   a.gate = gate;
   a.wait_ns = ws.wait_ns;
+  a.trace = ws.trace;
   const int grid = std::min(1 + std::max(1, helpers), p.nitems);
   if (precision == 0) df_launch_r<double2>(a, grid, s);
   else df_launch_r<float2>(a, grid, s);

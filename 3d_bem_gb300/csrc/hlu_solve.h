@@ -115,6 +115,9 @@ struct HluDfWork {
   // bound of one wait (ns): an item may wait for others whose CTAs share their
   // SMs with other streams' kernels
   unsigned long long wait_ns = 10000000000ull;
+  // optional (profiling), 1 + 3 D values cleared by the caller: start of the sweep and
+  // end of the last ROW, DIAG and DOT item of every level (ns)
+  unsigned long long* trace = nullptr;
 };
 
 // A run of consecutive supers that are inverted together: their leaves and panels,

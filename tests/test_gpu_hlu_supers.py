@@ -206,3 +206,32 @@ def test_fp32_sweeps_as_accurate_as_leaf_by_leaf(bem, meshes, orc, body):
     X, ref = s.hlu_solve(B), _leafwise(orc, _factors(s), n, B)
     assert np.linalg.norm(X - ref) < 1.33e-7 * np.linalg.norm(ref)
     s.close()
+
+
+def test_sweep_trace(bem, meshes, tmp_path, monkeypatch):
+    """BEM_DF_TRACE: one line per lower sweep of up to 8 vectors, and the same
+    solution."""
+    tri = meshes.icosphere(3, 1.0)
+    n = tri.shape[0]
+    s = bem.Solver(precision=1, aca_tol=1e-5, precond_rank=2)
+    s.set_mesh(tri)
+    s.set_bc(np.zeros(n), np.ones(n))
+    s.assemble(300.0)
+    s.hlu_build()
+    rng = np.random.default_rng(6)
+    B = rng.standard_normal((n, 9)) + 1j * rng.standard_normal((n, 9))
+    X = s.hlu_solve(B)
+    path = tmp_path / "sweeps.txt"
+    monkeypatch.setenv("BEM_DF_TRACE", str(path))
+    assert np.array_equal(s.hlu_solve(B), X)
+    monkeypatch.delenv("BEM_DF_TRACE")
+    lines = path.read_text().split("\n")[:-1]
+    assert len(lines) == 2
+    for line, R in zip(lines, (8, 1)):
+        assert line.startswith("df L sweep: levels ") and f" R {R} " in line
+        words = line.split()
+        levels, total = int(words[words.index("levels") + 1]), float(words[words.index("total_us") + 1])
+        per = [float(words[words.index(w) + 1]) for w in ("row", "diag", "dot")]
+        assert levels > 1 and all(0 < v < 1e4 for v in per)
+        assert total == pytest.approx(levels * sum(per), rel=0.01)
+    s.close()
