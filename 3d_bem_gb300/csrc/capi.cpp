@@ -905,7 +905,7 @@ void upload_bytes(DBuf<unsigned char>& d, const std::vector<T>& v, cudaStream_t 
 }
 
 // Device copy of a sweep plan (all but the apply matrices and inverses).
-void upload_df_plan(bem_handle* h, const HluDfPlan& p, int prec, bem_handle::DfDev& d) {
+void upload_df_plan(bem_handle* h, const HluDfPlan& p, bem_handle::DfDev& d) {
   cudaStream_t s = h->stream;
   d.items.upload(p.items, s);
   d.columns.upload(p.columns, s);
@@ -913,7 +913,7 @@ void upload_df_plan(bem_handle* h, const HluDfPlan& p, int prec, bem_handle::DfD
   d.inner.upload(p.inner, s);
   d.chunks.upload(p.chunks, s);
   d.supers.upload(p.supers, s);
-  const std::vector<HluDfPanel> panels = p.panels(prec);
+  const std::vector<HluDfPanel> panels = p.panels();
   d.panels.upload(panels, s);
   d.need.upload(p.need, s);
   HluDfDev v;
@@ -996,7 +996,7 @@ void upload_df_plans(bem_handle* h) {
   for (int q = 0; q < 2; q++) {
     const HluDfPlan& p = q ? pu : pl;
     bem_handle::DfDev& d = q ? h->dfU : h->dfL;
-    upload_df_plan(h, p, h->hlu_prec, d);
+    upload_df_plan(h, p, d);
     if (h->hlu_prec == 0) {
       upload_bytes(d.diag, p.diag, s);
     } else {
@@ -1108,8 +1108,7 @@ void prepare_hlu_arena(bem_handle* h, int prec) {
   CK(cudaMemsetAsync(h->dArena.p, 0, (size_t)P.arena * es, h->stream));
   h->dHScr.ensure((size_t)h->hp_grid * P.scratch * es);
   h->dHBig.ensure((size_t)std::max<int64_t>(P.big_scratch, 1) * es);
-  // sweep plans of the program's factors (the inversion's panels depend on the
-  // element type)
+  // sweep plans of the program's factors (the supers depend on the element type)
   if (P.df_ok) {
     std::string w;
     HluDfPlan pl, pu;
@@ -1117,8 +1116,8 @@ void prepare_hlu_arena(bem_handle* h, int prec) {
     const bool ok = hlu_df_plan_structure(P.L, h->N, cuts, pl, &w) &&
                     hlu_df_plan_structure(P.U, h->N, cuts, pu, &w);
     require(ok, BEM_EINVAL, "H-LU program: sweep plan");
-    upload_df_plan(h, pl, prec, h->dfL);
-    upload_df_plan(h, pu, prec, h->dfU);
+    upload_df_plan(h, pl, h->dfL);
+    upload_df_plan(h, pu, h->dfU);
     h->dfL.view.diag = h->dArena.p + (size_t)P.qh_base * es;
     h->dfU.view.diag = h->dArena.p + (size_t)P.rinv_base * es;
     CK(cudaStreamSynchronize(h->stream));  // the plans go out of scope

@@ -825,11 +825,10 @@ std::vector<int64_t> hlu_df_cuts(const HTree& tree, int precision) {
   return cuts;
 }
 
-std::vector<HluDfPanel> HluDfPlan::panels(int precision) const {
+std::vector<HluDfPanel> HluDfPlan::panels() const {
   std::vector<HluDfPanel> v;
-  const int w = hlu_df_panel_cols(precision);
   for (int i = 0; i < D(); i++)
-    for (int p0 = 0; p0 < supers[i].m; p0 += w) v.push_back(HluDfPanel{i, p0});
+    for (int p0 = 0; p0 < supers[i].m; p0 += HLU_DF_PANEL) v.push_back(HluDfPanel{i, p0});
   return v;
 }
 

@@ -69,7 +69,7 @@ struct HluDfPlan {
   int64_t nt = 0, msize = 0;
   bool lower = false;
   int D() const { return (int)supers.size(); }
-  std::vector<HluDfPanel> panels(int precision) const;
+  std::vector<HluDfPanel> panels() const;
   // the inversion in runs of supers with at most `most` values of dense blocks each
   // (one super at least)
   std::vector<HluDfBatch> batches(const std::vector<HluDfPanel>& panels, int64_t most) const;

@@ -211,11 +211,13 @@ int launch_hlu_sweep(const int32_t* sched, int nops, const int64_t* leaves, cons
 // sticky error word and returns.
 //
 // Bound by the latency of a level -- three hand-overs through flags in L2 (x ->
-// t -> s -> x, 0.7 us each) and ~2.4 us of work after each -- times the number
-// of levels. With the diagonal leaves (~22 rows) as steps of the chain a sweep
-// of 8 vectors took 14.2 ms at 81,920 pencil elements (3,627 steps); supers of
-// ~320 rows make it 256 steps and 2.36 ms, for one more pass over the inverses
-// (N x ~320 entries). 32, 64 and 120 helper CTAs measured the same.
+// t -> s -> x, 0.7 us each) and 1.5 to 6 us of work after each (row 4.3, diag 4.5,
+// dot 6.8 us with 8 vectors, 2.2, 3.4 and 3.3 us with one) -- times the number of
+// levels. At 81,920 pencil elements the chain has 248 levels of ~330 rows instead of
+// 3,627 of ~22 (the diagonal leaves), for one more pass over the inverses (N x ~330
+// entries): a sweep of 8 vectors takes 3.8 ms, of one 2.1 ms; in a solve of 8, whose
+// vectors end one by one, 2.4 ms on average against 14.2 ms over the leaves. 32, 64
+// and 120 helper CTAs measured the same.
 //
 // All arithmetic and every vector inside the sweep is in the factor's type T2:
 // complex FP32 for the mixed method, whose FP64 rate on GB300 would otherwise
@@ -899,8 +901,8 @@ int df_invert(const HluDfDev& p, const HluDfBatch& b, const void* data, void* de
 int launch_hlu_df_invert(const HluDfDev& p, const HluDfBatch& b, const void* data, int precision,
                          void* dense, cudaStream_t s) {
   if (b.npanels <= 0) return 0;
-  return precision == 0 ? df_invert<double2, hlu_df_panel_cols(0)>(p, b, data, dense, s)
-                        : df_invert<float2, hlu_df_panel_cols(1)>(p, b, data, dense, s);
+  return precision == 0 ? df_invert<double2, HLU_DF_PANEL>(p, b, data, dense, s)
+                        : df_invert<float2, HLU_DF_PANEL>(p, b, data, dense, s);
 }
 
 int launch_hlu_df(const HluDfDev& p, const void* data, int precision, const double2* w, double2* x,

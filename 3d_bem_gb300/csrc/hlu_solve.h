@@ -33,8 +33,13 @@ int launch_hlu_sweep(const int32_t* sched, int nops, const int64_t* leaves, cons
 // Items of a level wait for those of the previous kind, and DOT(I) for
 // DOT(I - 1), so t is summed in column order.
 constexpr int HLU_DF_SUPER = 512;    // most rows of a super
-// in complex FP64 shorter supers: the inversion (cubic in their rows) and the
-// products with the inverses are bound by the FP64 pipe
+// Most rows of a super in each precision: longer ones make the chain shorter, but the
+// inversion is cubic in their rows. FP32, 81,920 pencil elements: a sweep of 8 (1)
+// vectors 3.8 (2.1) ms with 512 rows, 5.9 (3.5) with 256, 8.0 (4.9) with 128, the
+// inversions 4.3 / 1.8 / 0.7 ms, against 38 sweeps of a solve; beyond 512 a panel
+// and the x of a super no longer fit. In complex FP64 the FP64 pipe bounds the
+// inversion: 1,280 sphere elements, 1.2 ms and 0.19 ms a sweep with 256 rows, 3.1 and
+// 0.11 with 512, 0.4 and 0.34 with 128, against 6 sweeps of a solve.
 constexpr int hlu_df_super(int precision) { return precision == 0 ? 256 : HLU_DF_SUPER; }
 constexpr int HLU_DF_MAX_M = 32;     // rows of a diagonal leaf
 constexpr int HLU_DF_MAX_RANK = 32;  // rank of a low-rank leaf
@@ -81,8 +86,10 @@ struct HluDfSuper {
 struct HluDfPanel {  // columns p0 .. of super's inverse (one CTA of the inversion)
   int32_t super, p0;
 };
-// columns per inversion CTA (their panel stays in shared memory)
-constexpr int hlu_df_panel_cols(int precision) { return precision == 0 ? 8 : 32; }
+// Columns per inversion CTA (their panel stays in shared memory). Both factors of
+// 81,920 pencil elements in FP32: 4.3 ms, 16 columns 5.0, 32 columns 10.3 (one CTA
+// per SM); of 5,120 in FP64 2.8 ms, 4 columns 3.9, 16 columns 5.1.
+constexpr int HLU_DF_PANEL = 8;
 
 // device copy of one factor's plan
 struct HluDfDev {
