@@ -498,7 +498,7 @@ class Solver:
         return x
 
     def hlu_sweep_kind(self) -> int:
-        """1: dataflow sweeps (driver + helper CTAs), 0: sequential sweeps."""
+        """1: dataflow sweeps over inverted diagonal blocks, 0: sequential sweeps."""
         k = ct.c_int32()
         self._check(lib().bem_hlu_sweep_kind(self._h, ct.byref(k)), "bem_hlu_sweep_kind")
         return k.value

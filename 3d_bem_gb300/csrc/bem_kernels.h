@@ -147,11 +147,10 @@ struct HmvArgs {
   const double2* x;
   int64_t ldx;
   double2* t;
-  int64_t ldt;
   double2* y;
   int64_t ldy;
   int accumulate;
-  float2* xf;  // FP32 scratch copies of x (ldx x nrhs) and t (ldt x nrhs)
+  float2* xf;  // FP32 scratch copies of x (ldx x nrhs) and t (as long as the complex FP64 t)
   float2* tf;  // for the FP32-arithmetic variant
   // pass-V records, longest rows first; the first nlong are those of HMV_VLROWS
   // rows of the blocks with more than HMV_VLONG columns (launch_vrec)
@@ -183,7 +182,7 @@ int launch_hmatvec(const HmvArgs& a, cudaStream_t s);  // returns kernels launch
 void launch_vrec(const HmvArgs& a, HmvVRec* rec, cudaStream_t s);
 
 // Fixed device scratch of the allocation-free H-matvec (complex FP64 entries,
-// 32 MiB): holds ldt x nrhs projections of one pass.
+// 32 MiB): holds the projections t of one pass.
 constexpr int64_t HMV_NOALLOC_SCRATCH = int64_t(1) << 21;
 int64_t hmatvec_noalloc_capacity();
 cudaError_t hmatvec_noalloc_scratch(double2** out);

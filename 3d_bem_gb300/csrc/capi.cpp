@@ -219,7 +219,7 @@ struct bem_handle {
   } dfL, dfU;
   DBuf<unsigned char> dfDense;  // dense diagonal blocks of a batch while they are inverted
   bool df_ok = false;
-  int df_helpers = 32;  // helper CTAs per dataflow sweep (12 while concurrent sweep workers run)
+  int df_helpers = 32;  // CTAs of a dataflow sweep beyond the first (12 while concurrent sweep workers run)
   int hlu_ctas_per_sm = 0;  // > 0: the executor's grid, per SM, below hp_grid (sweep workers)
   std::string df_why;
   DBuf<unsigned char> dfXi, dfS, dfT;  // factor-type vectors
@@ -796,7 +796,6 @@ void hmatvec_dev(bem_handle* h, int which, const double2* x, double2* y, int64_t
     a.x = x + r0 * ncols;
     a.ldx = ncols;
     a.t = h->dT.p;
-    a.ldt = std::max<int64_t>(h->L.s_size, 1);
     a.y = y + r0 * nrows;
     a.ldy = nrows;
     a.accumulate = acc;
@@ -2748,7 +2747,6 @@ bem_status bem_hmatvec_noalloc(bem_handle* h, int32_t which, const void* x, void
       a.x = xd + r0 * ncols;
       a.ldx = ncols;
       a.t = t;
-      a.ldt = ldt;
       a.y = yd + r0 * nrows;
       a.ldy = nrows;
       a.accumulate = accumulate;

@@ -42,8 +42,11 @@ static_assert(sizeof(FieldElem) == 224, "FieldElem is fourteen 16-byte pieces");
 
 // Observation points (threads) per CTA, and elements per shared-memory tile:
 // below 4,096 points CTAs of 64, so that a ragged last CTA idles at most 63
-// threads and there are enough CTAs to even out the SMs; above, 256 points
-// share one staging of the elements.
+// threads and there are enough CTAs to even out the SMs (5,120 elements, FP64: 250
+// points 0.95 ms, CTAs of 256 1.21; 500 points 1.73, 2.00); above, 256 points
+// share one staging of the elements (FP32, 4,096 points 148 us, CTAs of 64 152;
+// 8,192 points 267, 274; but where 256 does not divide them the idle threads cost
+// up to 8 %: FP64, 5,000 points 18.5 ms, 17.0).
 constexpr int FIELD_PTS_SMALL = 64, FIELD_PTS_LARGE = 256;
 constexpr int64_t FIELD_SMALL_POINTS = 4096;
 inline int field_points(int64_t M) {

@@ -394,15 +394,19 @@ int krylov_num_ctas(int64_t N) {
 // basis is short (up to one chunk per 128 elements), one per 1,024 elements when
 // it is long -- every CTA of the update kernel adds up the partials of all
 // chunks, which took a third of it at 41 chunks and 70 vectors (N = 5,123).
+// Box sweep of 5,123 elements and 4 right-hand sides with 4,864 / 2,432 / 1,216 tasks:
+// 101 / 98 / 100 ms. A fixed number (16 per SM of a GB300): the chunks decide the
+// order of the sums.
+constexpr int64_t DOT_TASKS = 2432;
 int krylov_dot_chunks(int64_t N, int64_t tasks) {
-  const int64_t want = (2432 + tasks - 1) / tasks;
+  const int64_t want = (DOT_TASKS + tasks - 1) / tasks;
   return (int)std::max<int64_t>(
       1, std::min<int64_t>(std::max<int64_t>(want, (N + 1023) / 1024), (N + 127) / 128));
 }
 // complex values the partial dot products of any step take
 int64_t krylov_partials(int64_t N, int R, int m) {
   const int64_t t = (int64_t)R * (m + 1);
-  return (N + 1023) / 1024 * t + 2432 + t;
+  return (N + 1023) / 1024 * t + DOT_TASKS + t;
 }
 
 // CGS2 step j in five launches: dot partials, reduction + update (twice; the

@@ -393,7 +393,9 @@ constexpr int TT = 256;      // threads of a training CTA
 constexpr int TS = 32;       // samples per tile
 constexpr int TLD = SEL_H + 4;   // row stride of the hidden tiles (16-byte rows)
 constexpr int TW2 = SEL_H + 1;   // row stride of W2
-constexpr int TRAIN_MAX_CTAS = 304;  // partial gradients of one step: two per SM
+// Most partial gradients of one step: two per SM of a GB300, a fixed number so that
+// the order of their sums, and with it the result's bits, is the same on any device.
+constexpr int TRAIN_MAX_CTAS = 304;
 
 struct TrainSmem {
   float x[TS * SEL_NF];

@@ -227,11 +227,12 @@ bem_status bem_hlu_build(bem_handle* h);
 /* x = U^{-1} L^{-1} b on the GPU for nrhs vectors (cluster order, host
  * buffers): HArithm::LUSubstitutionSolve (harithm.cpp:1168-1190). */
 bem_status bem_hlu_solve(bem_handle* h, const double* b, double* x, int64_t nrhs);
-/* Form of the sweeps of the built factors: 1 = dataflow (one driver CTA on
- * the chain of diagonal leaves, helper CTAs applying the off-diagonal leaves
- * as their columns are solved; needs diagonal leaves <= 32 rows and ranks
- * <= 32), 0 = one CTA per right-hand side walking the leaf schedule in the
- * reference's order. Both give the same solve to rounding. */
+/* Form of the sweeps of the built factors: 1 = dataflow (a chain over blocks of
+ * up to 512 rows, 256 in complex FP64, whose diagonal parts are kept as dense
+ * inverses; the CTAs of one launch claim its items in order and wait on each
+ * other's flags; needs diagonal leaves <= 32 rows, ranks <= 32 and device
+ * memory for the inverses), 0 = one CTA per right-hand side walking the leaf
+ * schedule in the reference's order. Both give the same solve to rounding. */
 bem_status bem_hlu_sweep_kind(const bem_handle* h, int32_t* kind);
 /* ---- Learned quadrature-order selector (no counterpart in the reference,
  * which integrates every regular pair with one 16-point rule,
