@@ -409,14 +409,14 @@ __global__ void __launch_bounds__(VT) hmv_vpass(const HmvVRec* __restrict__ rec,
 // i-th, loads its values of t or x and leaves both in shared memory, where the
 // loop over the columns reads them as broadcasts. So the loads in flight do not
 // stop at the end of a block (mean rank 17), and blocks of rank 5 and 80 do not
-// unbalance the warps. FP32 sums are plain over 16 columns (the even and the odd
-// ones of 32) and compensated beyond: over 32 a product of 20,480 elements was
-// 1.04e-7 to 1.09e-7 from the exact one, so 0.83e-7 to 0.88e-7 (sums per block, as
-// before the columns were laid end to end: 0.95e-7 to 1.02e-7). The partial sums of
-// the warps and CTAs are added in a fixed order. Bound by the bytes of U and F for
-// one vector (20,480 sphere, 351 MB: 68 us, 5.2 TB/s; one warp per block with 125 us
-// before) and by the shared-memory broadcasts and FMAs for eight (pencil, 20,480:
-// 120 us, 107 with one sum of 32 columns, before 221 us).
+// unbalance the warps. FP32 sums are plain over 16 columns and compensated beyond:
+// over 32 a product of 20,480 elements was 1.04e-7 to 1.09e-7 from the exact one, so
+// 0.79e-7 to 0.86e-7 (sums per block, as before the columns were laid end to end:
+// 0.95e-7 to 1.02e-7). The partial sums of the warps and CTAs are added in a fixed
+// order. Bound by the bytes of U and F for one vector (20,480 sphere, 351 MB: 68 us,
+// 5.2 TB/s; one warp per block with 125 us before) and by the shared-memory
+// broadcasts and FMAs for eight (pencil, 20,480: 117 us, 107 with sums of 32 columns,
+// before 221 us).
 // ---------------------------------------------------------------------------
 
 // FP32 sums across blocks, compensated
@@ -447,7 +447,7 @@ __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
   return d;
 }
 
-// Row sums of a warp over its columns: column() per column, flush() after 32 of
+// Row sums of a warp over its columns: column() per column, flush() after 16 of
 // them; total[r][lane] (shared memory, zero at first) holds what is summed over
 // the warps in the end.
 template <class A, int R>
@@ -459,7 +459,7 @@ struct RowSum {  // FP64, two-float
 #pragma unroll
     for (int r = 0; r < R; r++) acc[r] = A::zero();
   }
-  __device__ __forceinline__ void column(typename A::S u, const typename A::X* v, int) {
+  __device__ __forceinline__ void column(typename A::S u, const typename A::X* v) {
 #pragma unroll
     for (int r = 0; r < R; r++) A::fma(acc[r], u, v[r]);
   }
@@ -474,55 +474,45 @@ template <int R>
 struct RowSum<ArF32, R> {
   using Out = float4;  // compensated sums (re.hi, re.lo, im.hi, im.lo)
   static __device__ __forceinline__ Out none() { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
-  // partial sums of up to 16 columns each, column q in sum q % C; with 4 or more
-  // vectors as packed pairs: pa sums u.x (t.x, t.y) and pb sums u.y (t.x, t.y),
-  // re = pa.x - pb.y, im = pa.y + pb.x
+  // partial sums of up to 16 columns; with 4 or more vectors as packed pairs: pa
+  // sums u.x (t.x, t.y) and pb sums u.y (t.x, t.y), re = pa.x - pb.y,
+  // im = pa.y + pb.x
   static constexpr bool kPacked = R >= 4;
-  static constexpr int C = 2;
-  uint64_t pa[C][kPacked ? R : 1], pb[C][kPacked ? R : 1];
-  float2 acc[C][kPacked ? 1 : R];
+  uint64_t pa[kPacked ? R : 1], pb[kPacked ? R : 1];
+  float2 acc[kPacked ? 1 : R];
   __device__ __forceinline__ RowSum() { clear(); }
   __device__ __forceinline__ void clear() {
+    if constexpr (kPacked) {
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-      if constexpr (kPacked) {
+      for (int r = 0; r < R; r++) pa[r] = pb[r] = 0;
+    } else {
 #pragma unroll
-        for (int r = 0; r < R; r++) pa[c][r] = pb[c][r] = 0;
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) acc[c][r] = make_float2(0.0f, 0.0f);
-      }
+      for (int r = 0; r < R; r++) acc[r] = make_float2(0.0f, 0.0f);
     }
   }
-  __device__ __forceinline__ void column(float2 u, const float2* v, int q) {
-    const int c = q % C;
+  __device__ __forceinline__ void column(float2 u, const float2* v) {
     if constexpr (kPacked) {
       const uint64_t ux = pack2(u.x, u.x), uy = pack2(u.y, u.y);
 #pragma unroll
       for (int r = 0; r < R; r++) {
         const uint64_t w = pack2(v[r].x, v[r].y);
-        pa[c][r] = ffma2(ux, w, pa[c][r]);
-        pb[c][r] = ffma2(uy, w, pb[c][r]);
+        pa[r] = ffma2(ux, w, pa[r]);
+        pb[r] = ffma2(uy, w, pb[r]);
       }
     } else {
 #pragma unroll
-      for (int r = 0; r < R; r++) ArF32::fma(acc[c][r], u, v[r]);
+      for (int r = 0; r < R; r++) ArF32::fma(acc[r], u, v[r]);
     }
   }
   __device__ __forceinline__ void flush(Out (*total)[32], int lane) {
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      float2 s = make_float2(0.0f, 0.0f);
-#pragma unroll
-      for (int c = 0; c < C; c++) {
-        if constexpr (kPacked) {
-          const float2 a = unpack2(pa[c][r]), b = unpack2(pb[c][r]);
-          s.x += a.x - b.y;
-          s.y += a.y + b.x;
-        } else {
-          s.x += acc[c][r].x;
-          s.y += acc[c][r].y;
-        }
+      float2 s;
+      if constexpr (kPacked) {
+        const float2 a = unpack2(pa[r]), b = unpack2(pb[r]);
+        s = make_float2(a.x - b.y, a.y + b.x);
+      } else {
+        s = acc[r];
       }
       const Out o = total[r][lane];
       TwoSum sx{o.x, o.y}, sy{o.z, o.w};
@@ -585,6 +575,7 @@ __global__ void __launch_bounds__(UT, MINB) hmv_upass(
   using X = typename A::X;
   using Sum = RowSum<A, R>;
   using Out = typename Sum::Out;
+  static_assert(16 % UN == 0, "flush() after 16 columns");
   constexpr int NW = UT / 32;
   struct __align__(16) Stage {  // the warp's 32 columns
     X v[32][R];
@@ -674,7 +665,7 @@ __global__ void __launch_bounds__(UT, MINB) hmv_upass(
               if (i + q >= nb) u[q].x = u[q].y = 0;
             }
 #pragma unroll
-            for (int q = 0; q < UN; q++) sum.column(u[q], st.v[i + q], q);
+            for (int q = 0; q < UN; q++) sum.column(u[q], st.v[i + q]);
             if constexpr (A::kLo) {
               if (dense && Flo) {  // FP64 entries as hi + lo
 #pragma unroll
@@ -683,9 +674,10 @@ __global__ void __launch_bounds__(UT, MINB) hmv_upass(
                   if (i + q >= nb) u[q].x = u[q].y = 0;
                 }
 #pragma unroll
-                for (int q = 0; q < UN; q++) sum.column(u[q], st.v[i + q], q);
+                for (int q = 0; q < UN; q++) sum.column(u[q], st.v[i + q]);
               }
             }
+            if (i + UN == 16 && nb > 16) sum.flush(part[w], lane);
           }
           sum.flush(part[w], lane);
         }
