@@ -215,9 +215,9 @@ int launch_hlu_sweep(const int32_t* sched, int nops, const int64_t* leaves, cons
 // dot 6.8 us with 8 vectors, 2.2, 3.4 and 3.3 us with one) -- times the number of
 // levels. At 81,920 pencil elements the chain has 248 levels of ~330 rows instead of
 // 3,627 of ~22 (the diagonal leaves), for one more pass over the inverses (N x ~330
-// entries): a sweep of 8 vectors takes 3.8 ms, of one 2.1 ms; in a solve of 8, whose
-// vectors end one by one, 2.4 ms on average against 14.2 ms over the leaves. 32, 64
-// and 120 helper CTAs measured the same.
+// entries): a sweep of 8 vectors takes 3.8 ms, of one 2.1 ms; the 38
+// launches of a solve of 8 (14 of them gated off after convergence) 2.4 ms on average,
+// over the leaves 14.2 ms. 32, 64 and 120 CTAs beyond the first measured the same.
 //
 // All arithmetic and every vector inside the sweep is in the factor's type T2:
 // complex FP32 for the mixed method, whose FP64 rate on GB300 would otherwise

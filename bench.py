@@ -78,13 +78,13 @@ PENCIL_DESC = ("pencil r=4 mm L=0.2 m + 10 mm conical tip, 81,920 triangles, imp
                "rank 2")
 # DRAM bytes per algorithmic byte of the 8-RHS FP32 H-matvec, measured with
 # ncu (dram__bytes_read.sum + dram__bytes_write.sum of hmv_vpass<ArF32, 8> and
-# hmv_upass<ArF32, 8>) on the 20,480-triangle pencil: 422 MB for 384 MB; the
+# hmv_upass<ArF32, 8>) on the 20,480-triangle pencil: 423 MB for 384 MB; the
 # traffic grows with the stored entries, so it scales to the headline size
-HMV32_R8_TRAFFIC_PER_BYTE = 422.4 / 384.0
+HMV32_R8_TRAFFIC_PER_BYTE = 422.9 / 384.0
 # ncu of aca_kernel<0,float2,128,1> (the 128-thread ACA launch of the phi
-# matrix) on the 20,480-triangle sphere at 1.5 kHz: FMA pipe active 37.9 % of
-# its peak, issue slots 67 %, warps active 50 %, L2 hit rate 66 %
-ACA_FMA_PIPE_NCU = 0.379
+# matrix) on the 20,480-triangle sphere at 1.5 kHz: FMA pipe active 37.8 % of
+# its peak, issue slots 66 %, warps active 50 %, L2 hit rate 66 %
+ACA_FMA_PIPE_NCU = 0.378
 METRIC = "freq-solves/sec (H-matrix Helmholtz BEM solve, <=1e-5 rel. surface-pressure error)"
 UNIT = "freq-solves/s"
 
