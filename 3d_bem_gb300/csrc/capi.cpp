@@ -1460,6 +1460,7 @@ void df_trace_summary(bem_handle* h, const DBuf<unsigned long long>& tr, int R, 
   std::vector<unsigned long long> t(1 + 3 * (size_t)D);
   CK(cudaStreamSynchronize(h->stream));
   CK(cudaMemcpy(t.data(), tr.p, t.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
+  if (!t[0]) return;  // gated off: every vector has converged
   double ph[3] = {};
   for (size_t i = 0; i + 1 < t.size(); i++) ph[i % 3] += 1e-3 * (double)(t[i + 1] - t[i]) / D;
   FILE* f = std::fopen(path, "a");
@@ -1483,7 +1484,7 @@ void apply_precond(bem_handle* h, double2* w, int R, const int* gate_flags = nul
     // BEM_DF_TRACE=<file>: the lower sweep's phases, summarised into the file
     const char* trace_path = std::getenv("BEM_DF_TRACE");
     DBuf<unsigned long long> trace;
-    if (trace_path && *trace_path && !gate_flags) trace.ensure(1 + 3 * (size_t)h->dfL.view.D);
+    if (trace_path && *trace_path) trace.ensure(1 + 3 * (size_t)h->dfL.view.D);
     for (int r0 = 0; r0 < R; r0 += HLU_DF_MAX_R) {
       const int rc = std::min(HLU_DF_MAX_R, R - r0);
       double2* wr = w + (size_t)r0 * N;

@@ -235,3 +235,23 @@ def test_sweep_trace(bem, meshes, tmp_path, monkeypatch):
         assert levels > 1 and all(0 < v < 1e4 for v in per)
         assert total == pytest.approx(levels * sum(per), rel=0.01)
     s.close()
+
+
+def test_sweep_trace_of_a_solve(bem, meshes, tmp_path, monkeypatch):
+    """BEM_DF_TRACE in a preconditioned solve: the sweeps of its GMRES steps are
+    traced too, those launched after convergence leave no line."""
+    tri = meshes.icosphere(2, 1.0)
+    n = tri.shape[0]
+    s = bem.Solver(aca_tol=1e-5, gmres_tol=1e-9, use_preconditioner=1, precond_rank=2)
+    s.set_mesh(tri)
+    s.set_bc(np.zeros(n), np.ones(n))
+    p = s.solve(300.0, np.ones(n))[2]
+    path = tmp_path / "sweeps.txt"
+    monkeypatch.setenv("BEM_DF_TRACE", str(path))
+    q, info = s.solve(300.0, np.ones(n))[2:]
+    monkeypatch.delenv("BEM_DF_TRACE")
+    assert np.array_equal(p, q)
+    lines = path.read_text().split("\n")[:-1]
+    assert len(lines) >= info["iterations"] + 1  # the right-hand side and every step
+    assert all(float(x.split("total_us")[1].split()[0]) > 0 for x in lines)
+    s.close()
